@@ -1,5 +1,5 @@
 """Prefill operator on the GPU against the oracle: both kernels (tcgen05 for
-head dims 64/128, mma.sync for the rest), every supported bias, BMK / BMHK /
+head dims up to 128, mma.sync for the rest), every supported bias, BMK / BMHK /
 BMGHK layouts, LSE, sharded keys + merge."""
 
 import pytest
@@ -537,3 +537,31 @@ def test_two_key_ranges_in_one_launch(D, q0, Mq, L0, o0, L1, o1):
         P.FwOp._apply(inp, want_lse=True, kv_offset=0, kv_split=100, kv_offset2=o1)  # not a multiple of 128
     with pytest.raises(NotImplementedError):
         P.FwOp_Tcgen05_M256._apply(inp, want_lse=True, kv_offset=o0 - q0, kv_split=L0, kv_offset2=o1 - q0)
+
+
+@gpu
+@pytest.mark.parametrize("layout", ["dense", "causal_gqa", "varlen"])
+@pytest.mark.parametrize("D", [8, 24, 56, 72, 80, 96, 120])
+def test_padded_head_dims_on_the_tcgen05_kernel(D, layout):
+    """Head dims that are no tile width: zero-filled columns, partial k-steps and a narrower PV product (its width a multiple
+    of 16), outputs in all three types; several row blocks, ragged key tiles.  Tolerance: the suite's, for O and LSE."""
+    require_cuda()
+    op, dtype = P.FwOp_Tcgen05_Persistent, torch.float16 if D % 16 else torch.bfloat16
+    g = torch.Generator().manual_seed(D)
+    mk = lambda *s: torch.randn(*s, generator=g).to(dtype)
+    out_dtype = {8: torch.float32, 80: torch.float16}.get(D)
+    if layout == "dense":
+        q, k, v, bias = mk(2, 300, 3, D), mk(2, 197, 3, D), mk(2, 197, 3, D), None
+    elif layout == "causal_gqa":
+        q, bias = mk(1, 515, 2, 3, D), ab.LowerTriangularMask()
+        k, v = (mk(1, 515, 2, 1, D).expand(-1, -1, -1, 3, -1) for _ in range(2))
+    else:
+        lens = [1, 130, 257]
+        q, k, v = (mk(1, sum(lens), 2, D) for _ in range(3))
+        bias = ab.BlockDiagonalCausalMask.from_seqlens(lens)
+    dev_bias = bias.to("cuda") if layout == "varlen" else bias
+    out, lse = fmha.memory_efficient_attention_forward_requires_grad(q.cuda(), k.cuda(), v.cuda(), dev_bias, op=op, output_dtype=out_dtype)
+    assert out.dtype == (out_dtype or dtype)
+    ro, rl = oracle.ref_attention_with_lse(q.float(), k.float(), v.float(), bias)
+    assert_o_lse(out, lse, ro, rl, dtype, f"head dim {D}, {layout}")
+    _status_ok()

@@ -58,6 +58,6 @@ extern "C" int xfb200_prefill_forward(const xfb200_prefill_params* p, void* stre
                       (p->bias == nullptr || p->kernel_path != XFB200_PREFILL_TCGEN05_CTA) && prefill_sm100_supported(p);
   if (p->kernel_path >= XFB200_PREFILL_TCGEN05 && !can100) return set_error(XFB200_E_UNSUPPORTED, "prefill: the tcgen05 kernel does not cover this input");
   if (can100) return prefill_sm100_launch(p, st);
-  if (p->kv_split != 0) return set_error(XFB200_E_UNSUPPORTED, "prefill: two key ranges in one call need the tcgen05 kernel (head dim 64 or 128)");
+  if (p->kv_split != 0) return set_error(XFB200_E_UNSUPPORTED, "prefill: two key ranges in one call need the tcgen05 kernel (head dim up to 128)");
   return prefill_generic_launch(p, st);
 }

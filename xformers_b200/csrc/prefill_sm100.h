@@ -16,7 +16,7 @@ struct Sm100Args {
   const int32_t* seqlen_k;
   int32_t* status;    // [0] first code a launch gave up with, [1] epoch of that launch
   int32_t* counters;  // persistent kernel: [0] next work item, [1] CTAs that have finished; zero between launches
-  int32_t batch, mq, mkv, groups, heads_per_group;
+  int32_t batch, mq, mkv, groups, heads_per_group, head_dim;
   int32_t kv_h_is_broadcast;  // K/V head stride 0: KV head index is g only
   xfb200_strides os;
   int64_t lse_b, lse_g, lse_h;

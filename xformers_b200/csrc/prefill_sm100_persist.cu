@@ -268,7 +268,9 @@ __device__ __forceinline__ bool decode_item(const Sm100Args& a, int idx, Item& i
   return true;
 }
 
-template <int D, bool kBf16>
+// D: columns of the tiles (64 or 128).  kPad: the head dim a.head_dim is smaller than D; the copies fill the columns
+// behind it with zeros, the products leave out what lies wholly behind it, the output is written up to it.
+template <int D, bool kBf16, bool kPad>
 __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(const __grid_constant__ Sm100Args a) {
   using L = Smem<D>;
   constexpr int kHalves = D / 64;
@@ -280,6 +282,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_items = a.q_tiles * a.groups * a.heads_per_group * a.batch;
   const long long budget = a.wait_budget;
+  const int head_dim = kPad ? a.head_dim : D;
 
   // a CTA of this launch already gave up: take no work (the counters are still settled below)
   const bool drained = reinterpret_cast<volatile int32_t*>(a.status)[1] == int32_t(a.epoch);
@@ -365,7 +368,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
             if (it.j_end > it.j_begin) return;
             const int nrows = min(kBM * kTiles, it.qlen - it.m0);
             const int osz = a.out_dtype == XFB200_F32 ? 4 : 2;
-            const int chunks = D * osz / 16;
+            const int chunks = head_dim * osz / 16;
             uint8_t* ob = reinterpret_cast<uint8_t*>(a.out);
             const int64_t base = int64_t(it.tb) * a.os.b + int64_t(it.q_row0 + it.m0) * a.os.m + int64_t(it.g) * a.os.g + int64_t(it.h) * a.os.h;
             for (int i = lane; i < nrows * chunks; i += 32) {
@@ -475,7 +478,9 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
 #endif
         const int t = warp - kMmaWarp0;
         constexpr uint32_t idesc_qk = umma_idesc(kBM, kBN, kBf16, false, false);
-        constexpr uint32_t idesc_pv = umma_idesc(kBM, D, kBf16, false, true);
+        // (a padded head dim: QK^T in steps of 16 columns, PV in a width that is a multiple of 16)
+        const uint32_t idesc_pv = umma_idesc(kBM, kPad ? (head_dim + 15) / 16 * 16 : D, kBf16, false, true);
+        const int qk_steps = kPad ? (head_dim + 15) / 16 : D / 16;
         // Shared-memory descriptors: the upper word is constant (stride between
         // 8-row groups = 1024 B, version 1, 128B swizzle); the lower word holds
         // (address >> 4) and the leading-dimension offset, so stepping through a
@@ -494,7 +499,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           const uint32_t kl = k_lo0 + k_stage * (L::kKV >> 4);
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
-            if (kk < kk_lo || kk >= kk_hi) continue;
+            if (kk < kk_lo || kk >= kk_hi || (kPad && kk >= qk_steps)) continue;
             const uint32_t off = ((kk / 4) * kHalfBytes + (kk % 4) * 32) >> 4;
             umma_ss(tmem_s, desc(q_lo + off), desc(kl + off), idesc_qk, kk > 0);
           }
@@ -755,8 +760,9 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
                 float* dst = reinterpret_cast<float*>(a.out) + o_off + cblk * 32;
 #pragma unroll
                 for (int i = 0; i < 32; i += 4)
-                  *reinterpret_cast<float4*>(dst + i) = make_float4(__uint_as_float(orr[i]) * inv, __uint_as_float(orr[i + 1]) * inv,
-                                                                    __uint_as_float(orr[i + 2]) * inv, __uint_as_float(orr[i + 3]) * inv);
+                  if (!kPad || cblk * 32 + i < head_dim)
+                    *reinterpret_cast<float4*>(dst + i) = make_float4(__uint_as_float(orr[i]) * inv, __uint_as_float(orr[i + 1]) * inv,
+                                                                      __uint_as_float(orr[i + 2]) * inv, __uint_as_float(orr[i + 3]) * inv);
               } else {
                 uint16_t* dst = reinterpret_cast<uint16_t*>(a.out) + o_off + cblk * 32;
 #pragma unroll
@@ -767,7 +773,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
                     const float x0 = __uint_as_float(orr[i + 2 * e]) * inv, x1 = __uint_as_float(orr[i + 2 * e + 1]) * inv;
                     w[e] = a.out_dtype == XFB200_BF16 ? pack_pair<true>(x0, x1) : pack_pair<false>(x0, x1);
                   }
-                  *reinterpret_cast<uint4*>(dst + i) = make_uint4(w[0], w[1], w[2], w[3]);
+                  if (!kPad || cblk * 32 + i < head_dim) *reinterpret_cast<uint4*>(dst + i) = make_uint4(w[0], w[1], w[2], w[3]);
                 }
               }
             }
@@ -1056,9 +1062,9 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
   }
 }
 
-template <int D, bool kBf16>
+template <int D, bool kBf16, bool kPad>
 static int launch_t(const Sm100Args& a, cudaStream_t stream) {
-  auto kern = prefill_sm100_persist_kernel<D, kBf16>;
+  auto kern = prefill_sm100_persist_kernel<D, kBf16, kPad>;
   constexpr int smem = Smem<D>::kTotal;
   static bool configured[kMaxDevices] = {false};  // the attribute belongs to the device's context
   if (first_use_on_device(configured)) {
@@ -1088,9 +1094,15 @@ extern "C" __attribute__((visibility("default"))) int xfb200_debug_read_prefill_
 }
 #endif
 
+template <int D, bool kPad>
+static int persist_launch_d(const Sm100Args& a, bool bf16, cudaStream_t stream) {
+  return bf16 ? pst::launch_t<D, true, kPad>(a, stream) : pst::launch_t<D, false, kPad>(a, stream);
+}
+
 int prefill_sm100_persist_launch(Sm100Args a, int head_dim, bool bf16, cudaStream_t stream) {
-  if (head_dim == 128) return bf16 ? pst::launch_t<128, true>(a, stream) : pst::launch_t<128, false>(a, stream);
-  return bf16 ? pst::launch_t<64, true>(a, stream) : pst::launch_t<64, false>(a, stream);
+  if (head_dim == 128) return persist_launch_d<128, false>(a, bf16, stream);
+  if (head_dim == 64) return persist_launch_d<64, false>(a, bf16, stream);
+  return head_dim > 64 ? persist_launch_d<128, true>(a, bf16, stream) : persist_launch_d<64, true>(a, bf16, stream);
 }
 
 }  // namespace xfb

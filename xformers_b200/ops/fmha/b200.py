@@ -4,8 +4,8 @@ Slots into the dispatcher next to the reference's forward operators
 (``fmha.cutlass_blackwell.FwOp``, ``fmha.flash.FwOp``; registration record as
 tests/test_mem_eff_attention.py:104-111 reads it).  The arithmetic is done by
 ``xfb200_prefill_forward`` of libxfb200.so: a persistent TMA + tcgen05/TMEM
-kernel for head dims 64 and 128 (every mask, additive tensor biases included),
-an mma.sync kernel for the other head dims.
+kernel for head dims up to 128 (every mask, additive tensor biases included),
+an mma.sync kernel for the head dims above.
 """
 
 from __future__ import annotations
