@@ -565,3 +565,28 @@ def test_padded_head_dims_on_the_tcgen05_kernel(D, layout):
     ro, rl = oracle.ref_attention_with_lse(q.float(), k.float(), v.float(), bias)
     assert_o_lse(out, lse, ro, rl, dtype, f"head dim {D}, {layout}")
     _status_ok()
+
+
+@gpu
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("bias_dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("Mkv,wide,D", [(520, 520, 128), (517, 520, 64), (517, 517, 80), (3, 8, 128), (131, 136, 40)])
+def test_additive_bias_units_of_the_tcgen05_kernel(Mkv, wide, D, bias_dtype, causal):
+    """The bias comes in units of 64 bytes per row: rows on 16-byte boundaries (vector loads, the last vector of a row cut) and
+    rows that are not, one and several key steps, two row blocks, a bias shared by the heads (stride 0)."""
+    require_cuda()
+    B, Mq, H, dtype = 2, 300, 3, torch.float16
+    g = torch.Generator().manual_seed(Mkv + D)
+    q = torch.randn(B, Mq, H, D, generator=g).to(dtype).cuda()
+    k, v = (torch.randn(B, Mkv, H, D, generator=g).to(dtype).cuda() for _ in range(2))
+    t = torch.randn(B, 1, Mq, wide, generator=g).to(bias_dtype).cuda()
+    t[..., Mkv:] = float("nan")  # what lies behind a row is never used
+    t = t[..., :Mkv].expand(B, H, Mq, Mkv)
+    bias = ab.LowerTriangularMaskWithTensorBias(t) if causal else t
+    out, lse = fmha.memory_efficient_attention_forward_requires_grad(q, k, v, bias, op=P.FwOp_Tcgen05_Persistent)
+    add = t.float().cpu()
+    if causal:
+        add = add + ab.LowerTriangularMask().materialize((Mq, Mkv))
+    ro, rl = oracle.ref_attention_with_lse(q.float().cpu(), k.float().cpu(), v.float().cpu(), add)
+    assert_o_lse(out, lse, ro, rl, dtype, f"bias {bias_dtype} of {Mkv} columns")
+    _status_ok()

@@ -38,6 +38,7 @@ struct Sm100Args {
   // the kernel adds bias / scale to q k^T, so that the softmax sees q k^T * scale + bias
   const void* bias;
   int32_t bias_dtype;
+  int32_t bias_vec;  // every row of the bias starts on a 16-byte boundary
   float inv_scale;
   int64_t bias_b, bias_g, bias_h, bias_m;
 };

@@ -120,6 +120,11 @@ int prefill_sm100_launch(const xfb200_prefill_params* p, cudaStream_t stream) {
   a.wait_budget = p->wait_budget_kcycles > 0 ? 1000LL * p->wait_budget_kcycles : kDefaultWaitBudgetCycles;
   a.bias = p->bias, a.bias_dtype = p->bias_dtype, a.inv_scale = 1.f / p->scale;
   a.bias_b = p->bias_stride_b, a.bias_g = p->bias_stride_g, a.bias_h = p->bias_stride_h, a.bias_m = p->bias_stride_m;
+  {
+    const int64_t per16 = p->bias_dtype == XFB200_F32 ? 4 : 8;
+    a.bias_vec = (reinterpret_cast<uintptr_t>(p->bias) & 15) == 0 && p->bias_stride_b % per16 == 0 && p->bias_stride_g % per16 == 0 &&
+                 p->bias_stride_h % per16 == 0 && p->bias_stride_m % per16 == 0;
+  }
   const bool bf16 = p->dtype == XFB200_BF16;
   if (p->kernel_path == XFB200_PREFILL_TCGEN05_CTA) {
     if (p->kv_split > 0) return set_error(XFB200_E_UNSUPPORTED, "prefill: two key ranges in one call need the persistent kernel");

@@ -49,8 +49,8 @@
 // the step has no loop and no per-chunk test.  On diagonal and ragged tiles a
 // small loop first writes -inf over the hidden scores in tensor memory; the step
 // itself is one piece of code for every tile, which the instruction cache likes.
-// An additive bias is folded into the scores the same way (bias / scale added in
-// tensor memory).  When the first half of P (keys 64-127) is stored the softmax
+// An additive bias is added in the first pass (bias / scale; a kernel variant of its
+// own).  When the first half of P (keys 64-127) is stored the softmax
 // arrives on a barrier of its own and the MMA warp issues that half of PV while
 // the other half is still being computed.  Measured
 // alternatives on the causal 4k case: one pass with a stale reference, a vote per
@@ -132,7 +132,10 @@ struct Smem {
   static constexpr int kV = kK + kStages * kKV;
   static constexpr int kStats = kV + kStages * kKV;          // float2 [kTiles][kBM]: running maximum (log2 units), row sum
   static constexpr int kBar = kStats + kTiles * kBM * 8;
+  static constexpr int kBias = kBar + 1024;  // kBiased only: one unit of 32 rows x 64 bytes for each softmax warp
+  static constexpr int kBiasUnit = 32 * 64;
   static constexpr int kTotal = kBar + 1024 + 1024;
+  static constexpr int kTotalBiased = kTotal + 8 * kBiasUnit;
 };
 static_assert(sizeof(Barriers) <= 1024, "barrier block");
 
@@ -268,11 +271,16 @@ __device__ __forceinline__ bool decode_item(const Sm100Args& a, int idx, Item& i
   return true;
 }
 
-// D: columns of the tiles (64 or 128).  kPad: the head dim a.head_dim is smaller than D; the copies fill the columns
-// behind it with zeros, the products leave out what lies wholly behind it, the output is written up to it.
-template <int D, bool kBf16, bool kPad>
+// D: columns of the tiles (64 or 128).  kVariant:
+//   kExact   the head dim is D
+//   kPadded  the head dim a.head_dim is smaller than D; the copies fill the columns behind it with zeros, the products
+//            leave out what lies wholly behind it, the output is written up to it
+//   kBiased  an additive bias; the head dim may be D or smaller
+constexpr int kExact = 0, kPadded = 1, kBiased = 2;
+template <int D, bool kBf16, int kVariant>
 __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(const __grid_constant__ Sm100Args a) {
   using L = Smem<D>;
+  constexpr bool kPad = kVariant != kExact, kBias = kVariant == kBiased;
   constexpr int kHalves = D / 64;
   extern __shared__ uint8_t smem_dyn[];
   uint8_t* smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);  // an offset, so that the compiler keeps seeing shared memory
@@ -864,6 +872,89 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
         tc_wait_st();
       };
 
+      // ---- additive bias (kBiased).  Bound by how its bytes reach the registers: a row per thread is the layout of the
+      // scores, and reading memory that way costs one sector request per element (2048 x 2048 x 16 heads, bf16: 600 us).
+      // A warp therefore reads its 32 rows in units of 64 bytes per row, four lanes to a row and 16 bytes to a lane, holds
+      // the units of a step in registers from before the wait for the scores on, and turns one after the other into
+      // rows through 2 KB of shared memory (16-byte chunks XOR-ed with row / 2, no bank conflict either way): 99 us for the
+      // same call (34 GFLOP, 134 MB of bias).  A unit is
+      // 32 columns of a 16-bit bias (four units: a step) or 16 of an f32 one (four: half a step).
+      uint8_t* const bias_smem = smem + L::kBias + warp * L::kBiasUnit;
+      auto bias_load = [&](uint4* w, int64_t off, int mt0, int qlen, int col_first, int n_keys) {
+        const int esz = a.bias_dtype == XFB200_F32 ? 4 : 2, per16 = 16 / esz;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int r = mt0 + (warp & 3) * 32 + i * 8 + (lane >> 2);
+          const uint8_t* src = reinterpret_cast<const uint8_t*>(a.bias) + (off + int64_t(r) * a.bias_m) * esz;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int col = col_first + (u * 4 + (lane & 3)) * per16;
+            uint4 x = make_uint4(0, 0, 0, 0);
+            if (r < qlen && col < n_keys) {
+              if (a.bias_vec && col + per16 <= n_keys) {
+                x = __ldg(reinterpret_cast<const uint4*>(src + col * esz));
+              } else if (esz == 4) {
+                const uint32_t* e = reinterpret_cast<const uint32_t*>(src) + col;
+                x.x = e[0];
+                if (col + 1 < n_keys) x.y = e[1];
+                if (col + 2 < n_keys) x.z = e[2];
+                if (col + 3 < n_keys) x.w = e[3];
+              } else {
+                const uint16_t* e = reinterpret_cast<const uint16_t*>(src) + col;
+                auto el = [&](int k) -> uint32_t { return col + k < n_keys ? e[k] : 0; };
+                x = make_uint4(el(0) | el(1) << 16, el(2) | el(3) << 16, el(4) | el(5) << 16, el(6) | el(7) << 16);
+              }
+            }
+            w[u * 4 + i] = x;
+          }
+        }
+      };
+      auto bias_prefetch = [&](int64_t off, int mt0, int qlen, int col_first, int n_keys) {
+        const int esz = a.bias_dtype == XFB200_F32 ? 4 : 2;
+        const int r = mt0 + row;
+        const uint8_t* src = reinterpret_cast<const uint8_t*>(a.bias) + (off + int64_t(r) * a.bias_m) * esz;
+        for (int col = col_first; col < col_first + kBN; col += 128 / esz)
+          if (r < qlen && col < n_keys) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + int64_t(col) * esz));
+      };
+      // the scores of columns [32 chunk, 32 chunk + 32) of this thread's row += bias / scale (so that the step's scale *
+      // log2 e applies to the sum)
+      auto bias_add = [&](uint32_t* sc, const uint4* w, int chunk) {
+        auto to_rows = [&](int u, uint4 (&mine)[4]) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<uint4*>(bias_smem + (i * 8 + (lane >> 2)) * 64 + (((lane & 3) ^ ((lane >> 3) & 3)) << 4)) = w[u * 4 + i];
+          __syncwarp();
+#pragma unroll
+          for (int k = 0; k < 4; ++k) mine[k] = *reinterpret_cast<const uint4*>(bias_smem + lane * 64 + ((k ^ ((lane >> 1) & 3)) << 4));
+          __syncwarp();
+        };
+        auto add = [&](int c, float x) { sc[c] = __float_as_uint(fmaf(x, a.inv_scale, __uint_as_float(sc[c]))); };
+        if (a.bias_dtype == XFB200_F32) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint4 mine[4];
+            to_rows((chunk & 1) * 2 + h, mine);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              add(h * 16 + k * 4, __uint_as_float(mine[k].x)), add(h * 16 + k * 4 + 1, __uint_as_float(mine[k].y));
+              add(h * 16 + k * 4 + 2, __uint_as_float(mine[k].z)), add(h * 16 + k * 4 + 3, __uint_as_float(mine[k].w));
+            }
+          }
+          return;
+        }
+        uint4 mine[4];
+        to_rows(chunk, mine);
+        auto add2 = [&](int c, uint32_t x) {
+          float lo, hi;
+          if (a.bias_dtype == XFB200_BF16) unpack_pair<true>(x, lo, hi);
+          else unpack_pair<false>(x, lo, hi);
+          add(c, lo), add(c + 1, hi);
+        };
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          add2(k * 8, mine[k].x), add2(k * 8 + 2, mine[k].y), add2(k * 8 + 4, mine[k].z), add2(k * 8 + 6, mine[k].w);
+      };
+
       while (ok) {
         struct {
           int jlo, jhi, m0, shift, shift2, n_base, klen, qlen;
@@ -873,7 +964,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           it.jlo = t == 0 ? d.jlo[0] : d.jlo[1];
           it.jhi = t == 0 ? d.jhi[0] : d.jhi[1];
           it.m0 = d.m0, it.shift = d.shift, it.shift2 = d.shift2, it.n_base = d.n_base, it.klen = d.klen, it.qlen = d.qlen;
-          it.bias_off = a.bias != nullptr ? int64_t(d.b) * a.bias_b + int64_t(d.g) * a.bias_g + int64_t(d.h) * a.bias_h : 0;
+          it.bias_off = kBias ? int64_t(d.b) * a.bias_b + int64_t(d.g) * a.bias_g + int64_t(d.h) * a.bias_h : 0;
         });
         if (idx < 0) {
           if (idx == -2) {
@@ -889,10 +980,6 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
         const bool causal = a.window_right >= 0;
         col_hi = causal ? min(it.klen, i_loc + it.shift + a.window_right + 1) : it.klen;
         col_lo = a.window_left >= 0 ? i_loc + it.shift - a.window_left : 0;
-        // this thread's row of the additive bias (dense batches only), or null
-        const uint8_t* bias_row = nullptr;
-        if (a.bias != nullptr && i_loc < it.qlen)
-          bias_row = reinterpret_cast<const uint8_t*>(a.bias) + (it.bias_off + int64_t(i_loc) * a.bias_m) * (a.bias_dtype == XFB200_F32 ? 4 : 2);
         // m_run: the reference maximum the probabilities and O_t are taken against (log2 units; at most 2^8 below
         // the true running maximum); l_run: the row sum against m_run
         float m_run = -INFINITY, l_run = 0.f;
@@ -911,6 +998,13 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           }
           const bool need_mask = (n0 + kBN > klen) || (causal && n0 + kBN - 1 > mt0 + shift + a.window_right) ||
                                  (a.window_left >= 0 && n0 < mt0 + kBM - 1 + shift - a.window_left);
+          uint4 bw[kBias ? 16 : 1];
+          if constexpr (kBias) {
+            // asked for before the wait for the scores, which hides most of their latency; the next step's are asked
+            // into the L2 at the same time
+            bias_load(bw, it.bias_off, mt0, it.qlen, n0, klen);
+            bias_prefetch(it.bias_off, mt0, it.qlen, n0 + kBN, j + 1 < jhi ? klen : 0);
+          }
           ok = mbar_wait(&bar->s_full[t], cnt & 1, abort_flag, budget);
           XFB_PROF_LAP(1)  // wait for the scores
           if (!ok) {
@@ -918,30 +1012,6 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
             break;
           }
           tc_fence_after();
-          if (a.bias != nullptr) {  // (warp-uniform: the tensor-memory accesses below are warp-wide)
-            // An additive bias is folded into the scores where they lie (as bias / scale, so that the step's
-            // scale * log2 e applies to the sum); rows past the end of the queries and keys past the end of the
-            // keys are left alone (the former are never written, the latter are masked below).
-            uint32_t sm[32];
-#pragma unroll 1
-            for (int c = 0; c < kBN / 32; ++c) {
-              const int col0 = n0 + c * 32;
-              XFB_TMEM_LD_32(tmem_s + c * 32, sm);
-              XFB_TMEM_WAIT_LD_32(sm);
-#pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                float bv = 0.f;
-                if (bias_row != nullptr && col0 + i < klen) {
-                  if (a.bias_dtype == XFB200_F32) bv = reinterpret_cast<const float*>(bias_row)[col0 + i];
-                  else if (a.bias_dtype == XFB200_BF16) bv = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(bias_row)[col0 + i]);
-                  else bv = __half2float(reinterpret_cast<const __half*>(bias_row)[col0 + i]);
-                }
-                sm[i] = __float_as_uint(fmaf(bv, a.inv_scale, __uint_as_float(sm[i])));
-              }
-              XFB_TMEM_ST_32(tmem_s + c * 32, sm);
-              tc_wait_st();  // (the registers are written again in the next round)
-            }
-          }
           if (need_mask) {
             // Diagonal and ragged tiles: hidden scores are turned into -inf where they lie, in tensor memory, by this
             // small loop; the step itself then is the same code for every tile (one copy of it in the instruction
@@ -980,11 +1050,24 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
             XFB_TMEM_LD_32(tmem_s + 32, sb);
             XFB_TMEM_WAIT_LD_32(sa);
             XFB_TMEM_WAIT_LD_32(sb);
+            if constexpr (kBias) {
+              // the biased scores of keys 0-63 are read again in the second pass: they go back to where they came from
+              bias_add(sa, bw, 0);
+              XFB_TMEM_ST_32(tmem_s, sa);
+              bias_add(sb, bw, 1);
+              XFB_TMEM_ST_32(tmem_s + 32, sb);
+              if (a.bias_dtype == XFB200_F32) bias_load(bw, it.bias_off, mt0, it.qlen, n0 + 64, klen);
+            }
             float mx = fmaxf(chunk_max(reinterpret_cast<float*>(sa)), chunk_max(reinterpret_cast<float*>(sb)));
+            if constexpr (kBias) tc_wait_st();
             XFB_TMEM_LD_32(tmem_s + 64, sa);
             XFB_TMEM_LD_32(tmem_s + 96, sb);
             XFB_TMEM_WAIT_LD_32(sa);
             XFB_TMEM_WAIT_LD_32(sb);
+            if constexpr (kBias) {
+              bias_add(sa, bw, 2);
+              bias_add(sb, bw, 3);
+            }
             mx = fmaxf(mx, fmaxf(chunk_max(reinterpret_cast<float*>(sa)), chunk_max(reinterpret_cast<float*>(sb))));
             const float ms = mx * sl2;  // scale > 0 (host guarantees)
             // ---- the reference follows the maximum only when it has to (a fresh row: from -inf).  QK(t,j) completing
@@ -1062,10 +1145,11 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
   }
 }
 
-template <int D, bool kBf16, bool kPad>
+template <int D, bool kBf16, int kVariant>
 static int launch_t(const Sm100Args& a, cudaStream_t stream) {
-  auto kern = prefill_sm100_persist_kernel<D, kBf16, kPad>;
-  constexpr int smem = Smem<D>::kTotal;
+  auto kern = prefill_sm100_persist_kernel<D, kBf16, kVariant>;
+  constexpr int smem = kVariant == kBiased ? Smem<D>::kTotalBiased : Smem<D>::kTotal;
+  static_assert(smem <= 227 * 1024, "shared memory of one CTA");
   static bool configured[kMaxDevices] = {false};  // the attribute belongs to the device's context
   if (first_use_on_device(configured)) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -1094,15 +1178,16 @@ extern "C" __attribute__((visibility("default"))) int xfb200_debug_read_prefill_
 }
 #endif
 
-template <int D, bool kPad>
+template <int D, int kVariant>
 static int persist_launch_d(const Sm100Args& a, bool bf16, cudaStream_t stream) {
-  return bf16 ? pst::launch_t<D, true, kPad>(a, stream) : pst::launch_t<D, false, kPad>(a, stream);
+  return bf16 ? pst::launch_t<D, true, kVariant>(a, stream) : pst::launch_t<D, false, kVariant>(a, stream);
 }
 
 int prefill_sm100_persist_launch(Sm100Args a, int head_dim, bool bf16, cudaStream_t stream) {
-  if (head_dim == 128) return persist_launch_d<128, false>(a, bf16, stream);
-  if (head_dim == 64) return persist_launch_d<64, false>(a, bf16, stream);
-  return head_dim > 64 ? persist_launch_d<128, true>(a, bf16, stream) : persist_launch_d<64, true>(a, bf16, stream);
+  if (a.bias != nullptr) return head_dim > 64 ? persist_launch_d<128, pst::kBiased>(a, bf16, stream) : persist_launch_d<64, pst::kBiased>(a, bf16, stream);
+  if (head_dim == 128) return persist_launch_d<128, pst::kExact>(a, bf16, stream);
+  if (head_dim == 64) return persist_launch_d<64, pst::kExact>(a, bf16, stream);
+  return head_dim > 64 ? persist_launch_d<128, pst::kPadded>(a, bf16, stream) : persist_launch_d<64, pst::kPadded>(a, bf16, stream);
 }
 
 }  // namespace xfb
