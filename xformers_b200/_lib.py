@@ -10,7 +10,9 @@ from __future__ import annotations
 import ctypes as C
 import os
 from pathlib import Path
-from typing import Optional
+from typing import Any, Optional
+
+import torch  # noqa: F401  (the extension module is linked against its libraries)
 
 ABI_VERSION = 4
 
@@ -207,6 +209,7 @@ def library_path() -> Path:
 
 
 _LIB: Optional[C.CDLL] = None
+front: Any = None  # the extension module _front (csrc/front.cpp), once load() has bound it to the library
 
 
 def load() -> C.CDLL:
@@ -244,6 +247,15 @@ def load() -> C.CDLL:
     lib.xfb200_rope_padded.restype = C.c_int
     if lib.xfb200_abi_version() != ABI_VERSION:
         raise RuntimeError(f"{path}: ABI version {lib.xfb200_abi_version()} != {ABI_VERSION}")
+    try:
+        from . import _front
+    except ImportError as e:
+        raise RuntimeError(f"the extension module xformers_b200._front cannot be loaded ({e}): build it with `python -m xformers_b200.build`") from e
+    address = lambda f: C.cast(f, C.c_void_p).value
+    _front.bind(address(lib.xfb200_prefill_forward), address(lib.xfb200_decode_forward), address(lib.xfb200_decode_scratch_bytes),
+                address(lib.xfb200_merge_attentions), address(lib.xfb200_rope_padded))
+    global front
+    front = _front
     _LIB = lib
     return lib
 

@@ -14,7 +14,7 @@ from typing import Any, List, Optional, Sequence, Tuple, Type, Union
 
 import torch
 
-from . import attn_bias, b200, b200_splitk, common, dispatch, merge, triton_splitk  # noqa: F401
+from . import attn_bias, b200, b200_splitk, common, dispatch, front, merge, triton_splitk  # noqa: F401
 from .attn_bias import (  # noqa: F401
     VARLEN_BIASES,
     AttentionBias,
@@ -89,6 +89,9 @@ def memory_efficient_attention_forward(
     output_dtype: Optional[torch.dtype] = None,
 ) -> torch.Tensor:
     """``softmax(Q K^T * scale + bias) V`` (xformers/ops/__init__.py:18)."""
+    done = front.forward(query, key, value, attn_bias, p, scale, op, output_dtype, 0)
+    if done is not None:
+        return done[0]
     return _run_forward(Inputs(query, key, value, attn_bias, p, scale, output_dtype), op, needs_lse=False)[0]
 
 
@@ -107,6 +110,9 @@ def memory_efficient_attention_forward_requires_grad(
     (tests/test_mem_eff_attention.py:657-663)."""
     if p != 0.0:
         raise NotImplementedError("dropout is outside the forward hot path")
+    done = front.forward(query, key, value, attn_bias, p, scale, op, output_dtype, front.WANT_LSE)
+    if done is not None:
+        return done
     out, lse = _run_forward(Inputs(query, key, value, attn_bias, p, scale, output_dtype), op, needs_lse=True)
     assert lse is not None
     return out, lse
@@ -115,12 +121,18 @@ def memory_efficient_attention_forward_requires_grad(
 def _memory_efficient_attention_forward(inp: Inputs, op=None) -> torch.Tensor:
     """Forward on a prepared :class:`Inputs` (or :class:`InputsFp8`) object
     (used as ``fmha._memory_efficient_attention_forward`` by the reference's tests)."""
+    done = front.forward_inputs(inp, op, 0)
+    if done is not None:
+        return done[0]
     return _run_forward(inp, op, needs_lse=False)[0]
 
 
 def _memory_efficient_attention_forward_requires_grad(inp: Inputs, op=None) -> Tuple[torch.Tensor, Context]:
     """Same, returning ``(out, Context)`` with the log-sum-exp
     (tests/test_mem_eff_attention.py:2843-2848)."""
+    done = front.forward_inputs(inp, op, front.WANT_LSE)
+    if done is not None:
+        return done[0], Context(out=done[0], lse=done[1])
     out, lse = _run_forward(inp, op, needs_lse=True)
     return out, Context(out=out, lse=lse)
 
@@ -138,6 +150,9 @@ def memory_efficient_attention_partial(
 ) -> Tuple[torch.Tensor, torch.Tensor]:
     """Attention over a part of the keys, to be combined with
     :func:`merge_attentions` (tests/test_fmha_merge_attentions.py:117-122)."""
+    done = front.forward(query, key, value, attn_bias, p, scale, op, output_dtype, front.WANT_LSE | front.PARTIAL)
+    if done is not None:
+        return done
     inp = Inputs(query, key, value, attn_bias, p, scale, output_dtype, is_partial=True)
     out, lse = _run_forward(inp, op, needs_lse=True)
     assert lse is not None
@@ -170,6 +185,9 @@ def memory_efficient_attention(
         raise NotImplementedError("memory_efficient_attention: attn_bias requires grad; the backward pass is outside this library")
     if p != 0.0:
         raise NotImplementedError("dropout is outside the forward hot path")
+    done = front.forward(query, key, value, attn_bias, p, scale, op, output_dtype, 0)
+    if done is not None:
+        return done[0]
     return _run_forward(Inputs(query, key, value, attn_bias, p, scale, output_dtype), op, needs_lse=False)[0]
 
 

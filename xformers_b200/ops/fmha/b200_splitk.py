@@ -34,7 +34,6 @@ from .attn_bias import (
 from .common import AttentionFwOpBase, Context, Inputs, InputsFp8, check_lastdim_alignment_stride1
 
 _DTYPE_CODE = {torch.bfloat16: _lib.BF16, torch.float16: _lib.F16, torch.float32: _lib.F32}
-_SM_COUNT = 148
 _MAX_ROWS_PER_KV_HEAD = 64
 
 
@@ -231,21 +230,12 @@ class FwOp(AttentionFwOpBase):
     # ------------------------------------------------------------------ split
     @classmethod
     def get_split_k(cls, batch: int, kv_bound: int, kv_heads: int, row_bytes: int) -> int:
-        """Static heuristic: chunks of 1280 tokens per CTA (measured optimum
-        for both cache formats at 8 kv heads per CTA: 24-32 chunks of a 32k
-        context), halved while the grid would not fill the machine four times
-        over."""
+        """Number of key chunks per sequence: ``SPLIT_K`` where a subclass fixes
+        it, else the host front's rule (``split_k`` in csrc/front.cpp)."""
         if cls.SPLIT_K is not None:
             return max(1, int(cls.SPLIT_K))
-        hb = 8
-        while kv_heads % hb:
-            hb //= 2
-        head_blocks = kv_heads // hb
-        bound = -(-kv_bound // 128) * 128
-        chunk = max(128, min(bound, 1280))
-        while chunk > 128 and batch * head_blocks * (-(-bound // chunk)) < 4 * _SM_COUNT:
-            chunk = max(128, (chunk // 2) // 128 * 128)
-        return -(-bound // chunk)
+        _lib.load()
+        return _lib.front.split_k(batch, kv_bound, kv_heads)
 
     @classmethod
     def apply(cls, inp: Inputs, needs_gradient: bool) -> Tuple[torch.Tensor, Optional[Context]]:

@@ -34,6 +34,10 @@ def merge_attentions(
         raise ValueError("attn_split and lse_split must both be tensors or both be lists")
     if attn_is_list:
         attn_list, lse_list = list(attn_split), list(lse_split)
+        if _lib.front is not None and all(type(t) is torch.Tensor for t in attn_list) and all(type(t) is torch.Tensor for t in lse_list):
+            done = _lib.front.merge(attn_list, lse_list, write_lse, output_dtype)
+            if done is not None:
+                return done
         if len(attn_list) == 0 or len(attn_list) != len(lse_list):
             raise ValueError("attn_split and lse_split need the same, non-zero number of partials")
         if len(attn_list) > _lib.MERGE_MAX_PTRS:

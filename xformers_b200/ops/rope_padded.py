@@ -81,6 +81,19 @@ def rope_padded(
         raise ValueError("Gradients not supported.")
     n_total_queries = attn_bias.q_seqinfo.seqstart_py[-1]
     paged = isinstance(attn_bias, PagedBlockDiagonalCausalWithOffsetPaddedKeysMask)
+    if (
+        _lib.front is not None and first_seqpos is None and seqpos is None and cache_k_scale_shift is None and cache_v_scale_shift is None
+        and internal_dtype in ("", "f32", "f64") and all(type(t) is torch.Tensor for t in (xq, xk, xv, cache_k, cache_v))
+    ):
+        # the host front takes the call unless something about it is unusual (csrc/front.cpp)
+        qi, ki = attn_bias.q_seqinfo, attn_bias.k_seqinfo
+        done = _lib.front.rope(
+            xq, xk, xv, cache_k, cache_v, out_q, qi.seqstart, ki.seqstart, ki.seqlen, len(qi.seqstart_py) - 1, n_total_queries, ki.seqstart_py[-1],
+            qi.max_seqlen, attn_bias.block_tables if paged else None, attn_bias.page_size if paged else 0, adjacents, use_dynamic_scaling,
+            internal_dtype == "f64", theta, linear_scale, dynamic_old_context_len, dynamic_scale_factor, dynamic_low_freq_factor, dynamic_high_freq_factor,
+        )
+        if done is not None:
+            return done
     if paged:
         if cache_k.ndim < 2 or cache_k.shape[1] % attn_bias.page_size:
             raise ValueError(f"unexpected cache_k shape {tuple(cache_k.shape)}: rows must be a whole number of pages of {attn_bias.page_size}")
