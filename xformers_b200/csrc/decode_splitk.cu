@@ -1730,55 +1730,81 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt>::kCtasPerSm) d
 }
 
 // ---------------------------------------------------------------------------
-// Merge of the per-chunk partials of each sequence.  One warp per output row
-// (b, kv head, query row); chunks are visited in order, so the result is
-// deterministic.  Only the chunks that exist for sequence b are read.
+// Merge of the per-chunk partials of each sequence.  Four warps per output row
+// (b, kv head, query row), which take its chunks in turn with four loads in
+// flight each and meet in shared memory: with one warp per row, walking the
+// chunks one after the other, 64 rows of 128 chunks took 28 us -- latency, not
+// bytes.  Every chunk goes to a fixed warp and the warps are added up in order,
+// whatever the number of chunks, so the result is deterministic and does not
+// depend on a bound.  Only the chunks that exist for sequence b are read.
 // ---------------------------------------------------------------------------
+constexpr int kMergeWarpsPerCta = 8, kMergeWarpsPerRow = 4;
 template <int D>
-__global__ void __launch_bounds__(256) decode_merge_kernel(const __grid_constant__ DecodeArgs a) {
-  const int lane = threadIdx.x & 31;
-  const int64_t gw = int64_t(blockIdx.x) * 8 + (threadIdx.x >> 5);
+__global__ void __launch_bounds__(kMergeWarpsPerCta * 32) decode_merge_kernel(const __grid_constant__ DecodeArgs a) {
+  constexpr int V = D / 32;
+  __shared__ float red[kMergeWarpsPerCta][D + 4];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int step = kMergeWarpsPerRow;
+  const int part = warp % step;
+  const int64_t gw = int64_t(blockIdx.x) * (kMergeWarpsPerCta / step) + warp / step;
   const int R = a.rows;
-  const int64_t total = int64_t(a.batch) * a.kv_heads * R;
-  if (gw >= total) return;
+  const bool live = gw < int64_t(a.batch) * a.kv_heads * R;
   const int row = int(gw % R);
   const int head = int((gw / R) % a.kv_heads);
-  const int b = int(gw / (int64_t(R) * a.kv_heads));
+  const int b = live ? int(gw / (int64_t(R) * a.kv_heads)) : 0;
   int kv_len = a.seqlen_k != nullptr ? min(max(a.seqlen_k[b], 0), a.kv_padding) : a.kv_padding;
   if (a.window_size > 0) kv_len = min(kv_len, a.window_span);
-  const int nsplit = min(a.split_k, (kv_len + a.chunk_tokens - 1) / a.chunk_tokens);
+  const int nsplit = live ? min(a.split_k, (kv_len + a.chunk_tokens - 1) / a.chunk_tokens) : 0;
+  const int64_t prow0 = (int64_t(b) * a.split_k * a.kv_heads + head) * R + row, pstep = int64_t(a.kv_heads) * R;
 
   float mx = -INFINITY;
-  for (int s = lane; s < nsplit; s += 32) {
-    const float l = a.part_lse[((int64_t(b) * a.split_k + s) * a.kv_heads + head) * R + row];
-    mx = fmaxf(mx, l);
-  }
+  for (int s = lane; s < nsplit; s += 32) mx = fmaxf(mx, a.part_lse[prow0 + s * pstep]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  constexpr int V = D / 32;
   float acc[V];
 #pragma unroll
   for (int i = 0; i < V; ++i) acc[i] = 0.f;
   float den = 0.f;
   if (mx > -INFINITY) {
-    for (int s = 0; s < nsplit; ++s) {
-      const int64_t prow = ((int64_t(b) * a.split_k + s) * a.kv_heads + head) * R + row;
-      const float l = a.part_lse[prow];
-      if (!(l > -INFINITY)) continue;
-      const float w = __expf(l - mx);
-      den += w;
-      const float* po = a.part_o + prow * D + lane * V;
-      if constexpr (V == 4) {
-        const float4 x = *reinterpret_cast<const float4*>(po);
-        acc[0] += w * x.x, acc[1] += w * x.y, acc[2] += w * x.z, acc[3] += w * x.w;
-      } else if constexpr (V == 2) {
-        const float2 x = *reinterpret_cast<const float2*>(po);
-        acc[0] += w * x.x, acc[1] += w * x.y;
-      } else {
+    for (int s0 = part; s0 < nsplit; s0 += 4 * step) {
+      float l[4], x[4][V];
 #pragma unroll
-        for (int i = 0; i < V; ++i) acc[i] += w * po[i];
+      for (int u = 0; u < 4; ++u) {
+        const int s = s0 + u * step;
+        l[u] = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < V; ++i) x[u][i] = 0.f;
+        if (s < nsplit) {
+          l[u] = a.part_lse[prow0 + s * pstep];
+          const float* po = a.part_o + (prow0 + s * pstep) * D + lane * V;
+          if constexpr (V == 4) {
+            const float4 y = *reinterpret_cast<const float4*>(po);
+            x[u][0] = y.x, x[u][1] = y.y, x[u][2] = y.z, x[u][3] = y.w;
+          } else {
+            const float2 y = *reinterpret_cast<const float2*>(po);
+            x[u][0] = y.x, x[u][1] = y.y;
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float w = l[u] > -INFINITY ? __expf(l[u] - mx) : 0.f;
+        den += w;
+#pragma unroll
+        for (int i = 0; i < V; ++i) acc[i] += w > 0.f ? w * x[u][i] : 0.f;
       }
     }
+  }
+#pragma unroll
+  for (int i = 0; i < V; ++i) red[warp][lane * V + i] = acc[i];
+  if (lane == 0) red[warp][D] = den;
+  __syncthreads();
+  if (part != 0 || !live) return;
+#pragma unroll
+  for (int w = 1; w < step; ++w) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) acc[i] += red[warp + w][lane * V + i];
+    den += red[warp + w][D];
   }
   const float inv = den > 0.f ? 1.f / den : 0.f;
   const int qi = row / a.q_per_kv, h = row % a.q_per_kv;
@@ -1846,7 +1872,8 @@ static int launch_decode_t(const DecodeArgs& a_in, int head_blocks, cudaStream_t
   if (rc != XFB200_OK) return rc;
   if (a.split_k > 1) {
     const int64_t rows = int64_t(a.batch) * a.kv_heads * a.rows;
-    decode_merge_kernel<D><<<unsigned((rows + 7) / 8), 256, 0, stream>>>(a);
+    constexpr int per_cta = kMergeWarpsPerCta / kMergeWarpsPerRow;
+    decode_merge_kernel<D><<<unsigned((rows + per_cta - 1) / per_cta), kMergeWarpsPerCta * 32, 0, stream>>>(a);
     rc = check_launch("decode_merge_kernel");
   }
   return rc;
@@ -1936,9 +1963,14 @@ extern "C" int xfb200_decode_forward(const xfb200_decode_params* p, void* stream
     a.status = words + kWordDecodeStatus;
   }
 
-  // kv heads per CTA: the largest of 8, 4, 2, 1 that divides kv_heads
+  // kv heads per CTA: the largest of 8, 4, 2, 1 that divides kv_heads -- fewer while the grid would still fit the machine at
+  // once: an SM takes in at most some 110 GB/s, so a short context is read faster by all of them (4 sequences of 1000 keys, 8
+  // heads: 32 CTAs of 512 KB at 8 heads each, 128 of 128 KB at 2).  A 16-bit cache only: the stripes of a quantised one are
+  // short, and copied whole.
   int hb = 8;
   while (p->kv_heads % hb) hb >>= 1;
+  if (!int4 && !fp8)
+    while (hb > 1 && int64_t(p->batch) * (p->kv_heads / hb) * row_blocks * p->split_k * 2 <= sm_count()) hb >>= 1;
   a.hb = hb;
   const int head_blocks = p->kv_heads / hb;
 

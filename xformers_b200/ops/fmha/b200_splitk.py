@@ -229,13 +229,13 @@ class FwOp(AttentionFwOpBase):
 
     # ------------------------------------------------------------------ split
     @classmethod
-    def get_split_k(cls, batch: int, kv_bound: int, kv_heads: int, row_bytes: int) -> int:
+    def get_split_k(cls, batch: int, kv_bound: int, kv_heads: int, row_bytes: int, rows: int = 8, quantised: bool = False) -> int:
         """Number of key chunks per sequence: ``SPLIT_K`` where a subclass fixes
         it, else the host front's rule (``split_k`` in csrc/front.cpp)."""
         if cls.SPLIT_K is not None:
             return max(1, int(cls.SPLIT_K))
         _lib.load()
-        return _lib.front.split_k(batch, kv_bound, kv_heads)
+        return _lib.front.split_k(batch, kv_bound, kv_heads, rows, row_bytes, quantised)
 
     @classmethod
     def apply(cls, inp: Inputs, needs_gradient: bool) -> Tuple[torch.Tensor, Optional[Context]]:
@@ -343,7 +343,8 @@ class FwOp(AttentionFwOpBase):
             if _lib.debug_checks():
                 _debug_check_decode(bias, p, k)
             row_bytes = D if fp8 else (D // 8 + cls.NUM_GROUPS) * 4 if quantized else D * 2
-            p.split_k = cls.get_split_k(p.batch, min(p.kv_padding, p.window_size + p.mq - 1) if p.window_size else p.kv_padding, p.kv_heads, row_bytes)
+            p.split_k = cls.get_split_k(p.batch, min(p.kv_padding, p.window_size + p.mq - 1) if p.window_size else p.kv_padding, p.kv_heads, row_bytes,
+                                        p.mq * p.q_per_kv, quantized)
             lib = _lib.load()
             nbytes = lib.xfb200_decode_scratch_bytes(p.batch, p.mq, p.kv_heads, p.q_per_kv, D, p.split_k)
             scratch = torch.empty((nbytes,), dtype=torch.uint8, device=q.device) if nbytes else None
