@@ -48,6 +48,7 @@ struct DecodeArgs {
   const int32_t* block_tables;
   int32_t batch, mq, kv_heads, q_per_kv;
   int32_t kv_padding, page_size, bt_stride;
+  int32_t page_shift;  // log2(page_size), -1 if that is no power of two
   int32_t split_k, chunk_tokens;
   int32_t hb;          // kv heads per CTA (1, 2, 4 or 8)
   int32_t rows;        // R = mq * q_per_kv
@@ -1519,18 +1520,49 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt>::kCtasPerSm) d
     int64_t cached_base = 0;
     const int64_t kv_base = (a.kv_start != nullptr ? int64_t(a.kv_start[b]) : int64_t(b) * a.kv_padding) + win_skip;  // padded / gappy cache
     const int t_shift = ((a.block_tables != nullptr && a.kv_start != nullptr) ? a.kv_start[b] : 0) + win_skip;       // paged gappy cache
+    auto page_of = [&](int t) { return a.page_shift >= 0 ? t >> a.page_shift : t / a.page_size; };
     auto row_of = [&](int t_rel) -> int64_t {
       if (a.block_tables == nullptr) return kv_base + t_rel;
       const int t = t_rel + t_shift;
-      const int pg = t / a.page_size;
+      const int pg = page_of(t);
       if (pg != cached_page) {
         cached_page = pg;
         cached_base = int64_t(a.block_tables[int64_t(b) * a.bt_stride + pg]) * a.page_size;
       }
       return cached_base + (t - pg * a.page_size);
     };
+    // The same for the rows of the coming copies, a token per lane: the page-table entries of the chunk are kept in two windows of
+    // 32 pages, one entry per lane, the second read a whole window before it is needed.  With a look-up per copy a stage
+    // waited for a load at each new page, and one lane issued all its copies.  64 sequences of up to 32768 keys, one kv head with
+    // 16 query heads, pages of 16 tokens: bf16 cache 217 -> 128 us, fp8 255 -> 200; 8 sequences of up to 1024 keys, 8 kv heads,
+    // pages of 64: 16.8 -> 14.8.  (Divisions by the page size, if not done by a shift, cost the large ones 1 %.)
+    constexpr int kWindowPages = 32;
+    const bool windowed = a.block_tables != nullptr && a.page_size >= (TOK + kWindowPages - 3) / (kWindowPages - 2);
+    const int last_page = windowed ? page_of(chunk_hi - 1 + t_shift) : 0;
+    const int32_t* table = a.block_tables + (windowed ? int64_t(b) * a.bt_stride : 0);
+    int win = windowed ? page_of(chunk_lo + t_shift) : 0;  // first page of the window `cur`
+    int32_t cur = windowed ? table[min(win + lane, last_page)] : 0, nxt = windowed ? table[min(win + kWindowPages + lane, last_page)] : 0;
+    auto row_ahead = [&](int t_rel) -> int64_t {
+      if (!windowed) return row_of(t_rel);
+      const int t = t_rel + t_shift, pg = page_of(t), i = pg - win;
+      const int32_t e0 = __shfl_sync(0xffffffffu, cur, i & 31), e1 = __shfl_sync(0xffffffffu, nxt, i & 31);
+      return int64_t(i < kWindowPages ? e0 : e1) * a.page_size + (t - pg * a.page_size);
+    };
+    // a lane's copies of a stage begin every unit_tok tokens
+    const int grp = (kInt4 && a.copy_mode == 0) ? a.copy_group : 1;
+    const int per_tok_copies = a.copy_mode == 1 ? hb : 1;
+    const int unit_tok = a.copy_mode == 3 ? a.box_tok : grp;
     for (int tile = 0; tile < n_tiles; ++tile) {
       const int st = tile % kDecStages;
+      const int t0 = chunk_lo + tile * TOK;
+      const int nvalid = min(TOK, chunk_hi - t0);
+      if (windowed && page_of(t0 + t_shift) - win >= kWindowPages) {  // (a stage spans less than a window)
+        win += kWindowPages;
+        cur = nxt;
+        nxt = table[min(win + kWindowPages + lane, last_page)];
+      }
+      // (before the wait for the stage, which hides the look-up)
+      const int64_t row = a.copy_mode != 2 ? row_ahead(t0 + min((lane / per_tok_copies) * unit_tok, nvalid - 1)) : 0;
       if (tile >= kDecStages) {
         if (!mbar_wait(&empty_bar[st], ((tile / kDecStages) - 1) & 1)) {
           if (lane == 0) atomicCAS(a.status, 0, 1);
@@ -1542,20 +1574,20 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt>::kCtasPerSm) d
           return;
         }
       }
-      const int t0 = chunk_lo + tile * TOK;
-      const int nvalid = min(TOK, chunk_hi - t0);
       uint8_t* ks = stage_base + st * stage_bytes;
       uint8_t* vs = ks + kv_bytes;
       if (a.copy_mode == 3) {
-        // one tiled copy per run of box_tok tokens: {64 elements} x {box_tok rows} x {hb*D/64 column groups}
-        if (lane == 0) {
-          const int nbox = (nvalid + a.box_tok - 1) / a.box_tok;
+        // one tiled copy per run of box_tok tokens, {64 elements} x {box_tok rows} x {hb*D/64 column groups}: a lane each (a stage
+        // has 16 runs at most)
+        {
+          const int nbox = (nvalid + a.box_tok - 1) / a.box_tok;  // (no lane has two)
           const uint32_t box_bytes = uint32_t(a.box_tok) * hb * kHeadBytes;
           const bool ss_tma = kFp8 && a.ss_tma;
           const uint32_t box_ss = uint32_t(a.box_tok) * hb * (a.ss_tma == 2 ? 4u : 16u);  // per (token, head): the word, or the word and three replicas
-          mbar_expect_tx(&full_bar[st], uint32_t(nbox) * (box_bytes + (ss_tma ? box_ss : 0u)) * 2u);
-          for (int bx = 0; bx < nbox; ++bx) {
-            const int64_t row = row_of(t0 + bx * a.box_tok);
+          if (lane == 0) mbar_expect_tx(&full_bar[st], uint32_t(nbox) * (box_bytes + (ss_tma ? box_ss : 0u)) * 2u);
+          __syncwarp();
+          if (lane < nbox) {
+            const int bx = lane;
             // third coordinate: 128-byte column group (16-bit cache) or kv head (fp8: a head is one 128-byte row)
             const int c2 = kFp8 ? head0 : head0 * (D / 64);
             tma_load_3d(ks + bx * box_bytes, &a.tm_k, &full_bar[st], 0, int(row), c2);
@@ -1611,20 +1643,19 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt>::kCtasPerSm) d
         if (lane == 0) mbar_arrive(&full_bar[st]);
         continue;
       }
-      const int grp = (kInt4 && a.copy_mode == 0) ? a.copy_group : 1;
       const int ngroups = (nvalid + grp - 1) / grp;  // a group is always copied whole
-      const int per_tok_copies = a.copy_mode == 0 ? 1 : hb;
       const uint32_t seg_bytes = a.copy_mode == 0 ? uint32_t(hb * kHeadBytes * grp) : uint32_t(kHeadBytes);
       if (lane == 0) mbar_expect_tx(&full_bar[st], uint32_t(ngroups) * per_tok_copies * seg_bytes * 2u);
       __syncwarp();
-      for (int i = lane; i < ngroups * per_tok_copies; i += 32) {
+      for (int i0 = 0; i0 < ngroups * per_tok_copies; i0 += 32) {
+        const int i = i0 + lane;
         const int gi = i / per_tok_copies;
         const int hh = i % per_tok_copies;
         const int tok = gi * grp;
-        const int t = t0 + tok;
-        const int64_t row = row_of(t);
-        const int64_t ko = (row * a.k_sm + (head0 + hh) * a.k_sg) * kElem;
-        const int64_t vo = (row * a.v_sm + (head0 + hh) * a.v_sg) * kElem;
+        const int64_t rw = i0 == 0 ? row : row_ahead(t0 + min(tok, nvalid - 1));
+        if (i >= ngroups * per_tok_copies) continue;
+        const int64_t ko = (rw * a.k_sm + (head0 + hh) * a.k_sg) * kElem;
+        const int64_t vo = (rw * a.v_sm + (head0 + hh) * a.v_sg) * kElem;
         bulk_g2s(ks + tok * row_bytes + hh * kHeadBytes, kg + ko, seg_bytes, &full_bar[st]);
         bulk_g2s(vs + tok * row_bytes + hh * kHeadBytes, vg + vo, seg_bytes, &full_bar[st]);
       }
@@ -1936,6 +1967,9 @@ extern "C" int xfb200_decode_forward(const xfb200_decode_params* p, void* stream
   a.seqlen_k = p->seqlen_k, a.block_tables = p->block_tables, a.kv_start = p->kv_seqstart;
   a.batch = p->batch, a.mq = p->mq, a.kv_heads = p->kv_heads, a.q_per_kv = p->q_per_kv;
   a.kv_padding = p->kv_padding, a.page_size = p->page_size, a.bt_stride = p->block_table_stride;
+  a.page_shift = -1;
+  if (p->page_size > 0 && (p->page_size & (p->page_size - 1)) == 0)
+    for (a.page_shift = 0; (1 << a.page_shift) < p->page_size;) ++a.page_shift;
   a.split_k = p->split_k;
   // with a window no sequence has more than window_size + mq - 1 keys to read: the chunks divide that
   const int window_span = p->window_size > 0 ? p->window_size + p->mq - 1 : 0;
