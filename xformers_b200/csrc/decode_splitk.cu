@@ -7,10 +7,10 @@
 // 16-B aligned), 8 consumer warps do QK^T and PV with warp-level
 // mma.sync.m16n8k16 (query heads of a GQA group are the M rows, tokens the N
 // columns; K/V are never expanded), the online softmax lives in registers.
-// The int4 row-wise cache is unpacked in registers: nibbles become bf16/f16
-// values 16 + n by one shift+lop3 per element pair, and scale/shift are folded
-// into the scores (K) and into the probabilities (V) so no per-element FMA is
-// spent on dequantisation.
+// The int4 row-wise cache is unpacked in registers, nibbles becoming subnormal
+// f16 values, the fp8 one by conversions; scale/shift are folded into the scores
+// (K) and into the probabilities (V) so no per-element FMA is spent on
+// dequantisation.
 //
 // Each CTA writes a normalised partial (O_s fp32, LSE_s) to caller-provided
 // scratch; the row-merge kernel (merge.cu arithmetic) combines the chunks that
@@ -138,13 +138,7 @@ struct DecStage {
   // sub-tiles of 16 tokens each warp takes from one stage: the int4 cache is 4x
   // denser, so its stages hold more tokens to keep the per-stage overhead
   // (barrier round trip, page-table look-ups of the producer) off the critical path
-#ifndef XFB_FP8_SUBTILES
-#define XFB_FP8_SUBTILES 1
-#endif
-#ifndef XFB_FP8_CTAS
-#define XFB_FP8_CTAS 2
-#endif
-  static constexpr int kSubTiles = kFmt == kFmtInt4 ? 2 : kFmt == kFmtFp8 ? XFB_FP8_SUBTILES : 1;
+  static constexpr int kSubTiles = kFmt == kFmtInt4 ? 2 : 1;
   __host__ __device__ static int tokens(int hb) { return 16 * kSubTiles * (kDecConsumerWarps / hb); }
   __host__ __device__ static int kv_bytes(int hb) {  // K or V part of a stage, rounded to 128 B
     return (row_bytes(hb) * tokens(hb) + 127) & ~127;
@@ -159,9 +153,11 @@ constexpr int kDecMaxStages = 12;
 // arithmetic per byte and each warp's sub-tile is one long dependency chain, so
 // it runs two CTAs per SM (twice the warps to interleave) with half the ring each;
 // so does the fp8 kernel, which shares its structure.
-template <int kFmt>
+// (Two n-tiles of query rows need more registers than two CTAs leave a thread: spilled, 128 query heads on 8 kv heads took
+// 746 us over the int4 cache and 926 us over the fp8 one; one CTA per SM with both sub-tiles in flight: 460 and 718 us.)
+template <int kFmt, int MT>
 struct DecOccupancy {
-  static constexpr int kCtasPerSm = kFmt == kFmtInt4 ? 2 : kFmt == kFmtFp8 ? XFB_FP8_CTAS : 1;
+  static constexpr int kCtasPerSm = (kFmt == kFmtInt4 || kFmt == kFmtFp8) && MT == 1 ? 2 : 1;
   static constexpr int kRingBudget = kCtasPerSm == 2 ? 108 * 1024 : 212 * 1024;
 };
 
@@ -449,22 +445,221 @@ __device__ __forceinline__ void consume_plain(const DecodeArgs& a, const DecWarp
 }
 
 // ---------------------------------------------------------------------------
-// int4 row-wise cache.  The integer pipe that unpacks the nibbles is what
-// bounds this path, so everything is arranged to spend as few logic
-// operations per nibble as possible:
-//  * The products are taken transposed: tokens are the M rows of S^T = K Q^T
-//    and the K dimension of O^T = V^T P^T, the query rows (8 per n-tile) are
-//    the N columns.  One 16-token sub-tile costs D/16 + D/16 MMAs per n-tile
-//    and no MMA row is padding when the GQA group has 8 query heads.
-//  * Both products run in f16 whatever the type of Q.  With 10 mantissa bits a
-//    nibble can be read where it already sits: (w & 0x000F000F) | 0x64006400
-//    is the pair (1024 + n_e, 1024 + n_{e+4}) and (w & 0x00F000F0) | 0x64006400
-//    the pair (1024 + 16 n), so a word costs one shift (w >> 8, for the upper
-//    byte of each half) and four logic operations.  One half2 subtraction or
-//    fused multiply-add per pair, on the otherwise idle FMA pipe, brings the
-//    values back to exactly n, so the accumulators never see the offset.
-//    bf16 queries are converted to f16 after scaling each row by a power of
-//    two that keeps it below 2^15; the factor returns with the softmax scale.
+// What the consumers of the quantised caches (one scale / shift word per row)
+// share.  The products are taken transposed: tokens are the M rows of
+// S^T = K Q^T and the K dimension of O^T = V^T P^T, the query rows (8 per
+// n-tile) are the N columns, so no MMA row is padding when the GQA group has 8
+// query heads.  Both products run in f16 whatever the type of Q.
+//   Issue slots bound these consumers, and a warp's sub-tile is one chain of
+// dependent steps, so the softmax is arranged for few instructions:
+//  * scale and shift of a key are applied to the score, relative to the row's
+//    reference maximum at once: (s * scale + shift * sum(q)) * fac - ref is
+//    three instructions, and its exponential the probability.
+//  * the reference is refreshed (cross-lane reduction, rescaling) only when some
+//    score exceeds it by more than 2^4; otherwise probabilities are taken
+//    against the stale one, which is exact in floating point.  One vote and
+//    one rarely taken branch for all U sub-tiles of 16 tokens of a step.
+//  * V's scale is folded into P, its shift is a per-row term sum_t p_t * shift_t
+//    added at the end.  P^T reaches the B operand of the second product through
+//    movmatrix.
+// ---------------------------------------------------------------------------
+// log2 of the largest probability taken against a stale maximum; P * scale(V) is
+// an f16 value, so 2^kLazy * scale must stay below 65504
+constexpr float kQuantLazy = 4.f;
+
+template <int NTQ>
+struct QuantRows {  // rows 2c and 2c + 1 of each n-tile
+  float fac[NTQ][2];    // softmax scale * log2(e) * 2^-k
+  float sum[NTQ][2];    // sum over d of the scaled q
+  float ref[NTQ][2];    // reference maximum (0 while there is none)
+  float slack[NTQ][2];  // a score above ref + slack refreshes it: kQuantLazy, or -inf while there is none
+  float l[NTQ][2], corr[NTQ][2];
+  int lim[NTQ][2];      // token t is visible iff t < lim
+  int lim_min;          // below it nothing is masked for any row of this warp
+};
+
+// Q^T fragments' source: the row's largest magnitude and the power of two 2^k that brings it to [2^14, 2^15).  The f16 values
+// keep 11 bits down to 2^-28 of the row's maximum.
+template <int D, typename T>
+__device__ __forceinline__ int quant_q_exponent(const T* qrow, int c) {
+  float amax = 0.f;
+  for (int d = c; d < D; d += 4) amax = fmaxf(amax, fabsf(float(qrow[d])));
+  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+  const int e = int(__float_as_uint(amax) >> 23) - 127;
+  return e > 127 ? 0 : 14 - max(e, -100);  // (an infinity stays one)
+}
+__device__ __forceinline__ float exp2_int(int k) { return __uint_as_float(uint32_t(127 + k) << 23); }
+
+// Row sums and factors of n-tile `nt` (thread (r, c) has row r at hand), limits, and the empty state.
+template <int D, int NTQ, typename T>
+__device__ __forceinline__ void quant_rows_init(QuantRows<NTQ>& q, int nt, const T* qrow, int kexp, const DecodeArgs& a, const DecWarp& w) {
+  const int c = w.lane & 3;
+  const float qmul = exp2_int(kexp);
+  float sr = 0.f;  // the quad of row r adds up that row, then rows 2c, 2c+1 are fetched
+  for (int d = c; d < D; d += 4) sr += __half2float(__float2half_rn(float(qrow[d]) * qmul));
+  sr += __shfl_xor_sync(0xffffffffu, sr, 1);
+  sr += __shfl_xor_sync(0xffffffffu, sr, 2);
+  const float fac = exp2_int(-kexp) * a.scale_log2;
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    q.fac[nt][e] = __shfl_sync(0xffffffffu, fac, 8 * c + 4 * e);
+    q.sum[nt][e] = __shfl_sync(0xffffffffu, sr, 8 * c + 4 * e);
+    q.ref[nt][e] = 0.f, q.slack[nt][e] = -INFINITY, q.l[nt][e] = 0.f, q.corr[nt][e] = 0.f;
+    // (a window with several queries per sequence, which also has lower limits, is served by the 16-bit consumer only)
+    const int row = w.row0 + nt * 8 + 2 * c + e;
+    int lim = w.chunk_hi;
+    if (a.causal && row < a.rows) lim = min(lim, w.kv_len - a.mq + row / a.q_per_kv + 1);
+    q.lim[nt][e] = lim;
+  }
+}
+template <int NTQ>
+__device__ __forceinline__ void quant_rows_limit(QuantRows<NTQ>& q, int chunk_hi) {
+  q.lim_min = chunk_hi;
+#pragma unroll
+  for (int nt = 0; nt < NTQ; ++nt) q.lim_min = min(q.lim_min, min(q.lim[nt][0], q.lim[nt][1]));
+  q.lim_min = min(q.lim_min, __shfl_xor_sync(0xffffffffu, q.lim_min, 1));
+  q.lim_min = min(q.lim_min, __shfl_xor_sync(0xffffffffu, q.lim_min, 2));
+}
+
+__device__ __forceinline__ float2 scale_shift(uint32_t word) { return __half22float2(*reinterpret_cast<const __half2*>(&word)); }
+
+// Softmax of U sub-tiles: scores s (S^T fragments, before K's scale) and the scale / shift words of tokens r, r + 8 of each to the
+// B fragments pb of P^T times V's scale.  `kmul` multiplies K's scale; sub-tile u starts at token t_sub + u * t_step.
+template <int NTQ, int U, int MTV>
+__device__ __forceinline__ void quant_softmax(QuantRows<NTQ>& q, const float (&s)[U][NTQ][4], const uint32_t (&kw)[U][2], const uint32_t (&vw)[U][2], float kmul,
+                                              int t_sub, int t_step, int chunk_hi, int r, float (&acc)[MTV][NTQ][4], uint32_t (&pb)[U][NTQ][2]) {
+  float p[U][NTQ][4];  // scores relative to the reference, then probabilities
+  float2 vss[U][2];    // V's scale and shift
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float2 kss = scale_shift(kw[u][h]);
+      const float ksc = kss.x * kmul;
+      vss[u][h] = scale_shift(vw[u][h]);
+#pragma unroll
+      for (int nt = 0; nt < NTQ; ++nt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          p[u][nt][2 * h + e] = fmaf(fmaf(ksc, s[u][nt][2 * h + e], kss.y * q.sum[nt][e]), q.fac[nt][e], -q.ref[nt][e]);
+    }
+  if (t_sub + (U - 1) * t_step + 16 > q.lim_min) {  // (warp-uniform)
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int t = t_sub + u * t_step + r + 8 * h;
+        if (t >= chunk_hi) vss[u][h] = make_float2(0.f, 0.f);  // tokens past the end were not copied: their words are garbage
+#pragma unroll
+        for (int nt = 0; nt < NTQ; ++nt)
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            if (t >= q.lim[nt][e]) p[u][nt][2 * h + e] = -INFINITY;
+      }
+  }
+  bool need = false;
+  float mx[NTQ][2];
+#pragma unroll
+  for (int nt = 0; nt < NTQ; ++nt)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      mx[nt][e] = fmaxf(p[0][nt][e], p[0][nt][2 + e]);
+#pragma unroll
+      for (int u = 1; u < U; ++u) mx[nt][e] = fmaxf(mx[nt][e], fmaxf(p[u][nt][e], p[u][nt][2 + e]));
+      need |= mx[nt][e] > q.slack[nt][e];
+    }
+  if (__any_sync(0xffffffffu, need)) {
+    // some row's maximum grew by more than the slack: refresh all of them
+#pragma unroll
+    for (int nt = 0; nt < NTQ; ++nt) {
+      float alpha[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float m = mx[nt][e];
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+        const bool none = q.slack[nt][e] == -INFINITY;
+        m = fmaxf(m, none ? -INFINITY : 0.f);
+        float up = 0.f;  // by how much the reference moves
+        if (m > -INFINITY) {
+          const float ref = q.ref[nt][e] + m;
+          up = ref - q.ref[nt][e];
+          q.ref[nt][e] = ref, q.slack[nt][e] = kQuantLazy;
+        }
+        alpha[e] = none ? 0.f : fast_exp2(-up);
+        q.l[nt][e] *= alpha[e];
+        q.corr[nt][e] *= alpha[e];
+#pragma unroll
+        for (int u = 0; u < U; ++u) p[u][nt][e] -= up, p[u][nt][2 + e] -= up;
+      }
+#pragma unroll
+      for (int mt = 0; mt < MTV; ++mt) {
+        acc[mt][nt][0] *= alpha[0];
+        acc[mt][nt][1] *= alpha[1];
+        acc[mt][nt][2] *= alpha[0];
+        acc[mt][nt][3] *= alpha[1];
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+#pragma unroll
+    for (int nt = 0; nt < NTQ; ++nt) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) p[u][nt][i] = fast_exp2(p[u][nt][i]);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        q.l[nt][e] += p[u][nt][e] + p[u][nt][2 + e];
+        q.corr[nt][e] = fmaf(p[u][nt][e], vss[u][0].y, fmaf(p[u][nt][2 + e], vss[u][1].y, q.corr[nt][e]));
+      }
+      pb[u][nt][0] = movmatrix_trans(pack2<false>(p[u][nt][0] * vss[u][0].x, p[u][nt][1] * vss[u][0].x));  // tokens 2c, 2c+1   of row r
+      pb[u][nt][1] = movmatrix_trans(pack2<false>(p[u][nt][2] * vss[u][1].x, p[u][nt][3] * vss[u][1].x));  // tokens 2c+8, 2c+9 of row r
+    }
+}
+
+// Full row sums (each thread saw tokens r and r+8 of every sub-tile); the warp's maxima and sums go to its combine slot.
+template <int D, int NTQ>
+__device__ __forceinline__ void quant_rows_finish(QuantRows<NTQ>& q, const DecWarp& w) {
+  const int r = w.lane >> 2, c = w.lane & 3;
+#pragma unroll
+  for (int nt = 0; nt < NTQ; ++nt)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) {
+        q.l[nt][e] += __shfl_xor_sync(0xffffffffu, q.l[nt][e], o);
+        q.corr[nt][e] += __shfl_xor_sync(0xffffffffu, q.corr[nt][e], o);
+      }
+    }
+  // the ring is no longer in use once every consumer warp got here
+  asm volatile("bar.sync 1, %0;" ::"n"(kDecConsumerWarps * 32) : "memory");
+  if (r == 0) {
+#pragma unroll
+    for (int nt = 0; nt < NTQ; ++nt)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float* row = w.mine + (nt * 8 + 2 * c + e) * (D + 2);
+        row[D] = q.slack[nt][e] == -INFINITY ? -INFINITY : q.ref[nt][e];
+        row[D + 1] = q.l[nt][e];
+      }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// int4 row-wise cache.  The integer pipe that unpacks the nibbles (16 lanes per
+// clock and scheduler) and the issue slots bound this path, so everything is
+// arranged to spend as few operations per nibble as possible:
+//  * A nibble is used almost where it sits, as a subnormal f16, which the tensor
+//    cores multiply exactly: (w << 2) & 0x003C003C is the pair (n_e, n_{e+4}) *
+//    2^-22 and (w << 2) & 0x03C003C0 the pair n * 2^-18; w >> 6 has the upper byte
+//    of each half in the same places.  A word costs two shifts and four ANDs for
+//    8 nibbles.  The power of two is taken out of the output rows (V) and of K's
+//    scale; K's even elements are brought to 2^-18 too, because the tensor core
+//    aligns subnormals by their exponent field, so that the sum of the products
+//    keeps all its bits only for those in the upper bits (LSE error up to 4e-6
+//    instead of 1e-6 with the plain w & 0x000F000F).
 //  * K: thread (r, c) reads word 4i + c of tokens r and r + 8; its nibble pairs
 //    (e, e + 4) are the k-slots (2c, 2c+1) / (2c+8, 2c+9) of k-steps 2i and
 //    2i + 1.  Q^T is loaded in the same permuted order of d.
@@ -472,15 +667,17 @@ __device__ __forceinline__ void consume_plain(const DecodeArgs& a, const DecWarp
 //    a byte permute first puts the same half-word of two neighbouring tokens
 //    side by side, so that unpacking yields A-fragment registers directly:
 //    m-tile wi*4 + e holds d = 8*(WPT*r + wi) + e in row r, d + 4 in row r + 8.
-//  * K's scale and shift are applied to the scores (shift times the row sum
-//    of q), V's scale is folded into P and its shift is a per-row term
-//    sum_t p_t * shift_t added at the end.  P^T reaches the B operand of the
-//    second product through movmatrix.
-//  * The running maximum is refreshed (cross-lane reduction, rescaling) only
-//    when some score exceeds it by more than 2^8; otherwise probabilities are
-//    taken against the stale maximum, which is exact in floating point.
+//  * The number of heads per CTA is a template parameter: the row pitch of the
+//    stage is a constant then, and every load an offset from one register.
+//  * The two sub-tiles that a warp has in a stage go through the step together,
+//    so that one's loads and unpacking fill the other's waits and the softmax's
+//    overhead is paid once for 32 tokens.
+// 64 sequences of 1024 to 32768 keys, 8 kv heads, 64 query heads, pages of 256:
+// 388 -> 274 us (2.84 -> 4.02 TB/s); 128 query heads 924 -> 463 us, 32 query heads
+// on 4 kv heads, pages of 64, 221 -> 156 us.  The issue slots are what is left:
+// about 290 instructions per sub-tile were 437.
 // ---------------------------------------------------------------------------
-template <int D, int NTQ, bool kBf16>
+template <int D, int NTQ, bool kBf16, int HB>
 __device__ __forceinline__ void consume_int4(const DecodeArgs& a, const DecWarp& w) {
   using T = typename Half2Type<kBf16>::T;
   constexpr int W = 1 + D / 8;  // words per row (scale/shift word + nibbles)
@@ -489,56 +686,28 @@ __device__ __forceinline__ void consume_int4(const DecodeArgs& a, const DecWarp&
   constexpr int WPT = D / 64;   // V words per thread and token
   constexpr int kQRowBytes = D * 2;
   constexpr int kCmbRow = D + 2;
-  constexpr int kSps = DecStage<D, kFmtInt4>::kSubTiles;
-  // log2 of the largest probability taken against a stale maximum; P * scale(V)
-  // is an f16 value, so 2^kLazy * scale must stay below 65504
-  constexpr float kLazy = 4.f;
+  constexpr int U = DecStage<D, kFmtInt4>::kSubTiles;  // all of a stage in one step
   const int lane = w.lane, r = lane >> 2, c = lane & 3;
-  const int R = a.rows, hw = w.hw, row_bytes = w.row_bytes;
+  const int hw = w.hw;
 
-  // nibble pairs (e, e+4), e = 0..3, of a packed word as two f16 values n
+  // nibble pairs (e, e+4) of a packed word as f16 pairs: n * 2^-22 for even e, n * 2^-18 for odd e
   auto unpack4 = [](uint32_t x, uint32_t (&out)[4]) {
-    constexpr uint32_t kMagic = 0x64006400u;                   // 1024.0 | 1024.0
-    const __half2 k1024 = __half2half2(__ushort_as_half(0x6400));
-    const __half2 k64 = __half2half2(__ushort_as_half(0x5400));   // 64.0
-    const __half2 k16th = __half2half2(__ushort_as_half(0x2C00));  // 1/16
-    const uint32_t hi = x >> 8;
-    uint32_t v0 = (x & 0x000F000Fu) | kMagic, v1 = (x & 0x00F000F0u) | kMagic;
-    uint32_t v2 = (hi & 0x000F000Fu) | kMagic, v3 = (hi & 0x00F000F0u) | kMagic;
-    __half2 h0 = __hsub2(*reinterpret_cast<__half2*>(&v0), k1024);
-    __half2 h1 = __hfma2(*reinterpret_cast<__half2*>(&v1), k16th, __hneg2(k64));
-    __half2 h2 = __hsub2(*reinterpret_cast<__half2*>(&v2), k1024);
-    __half2 h3 = __hfma2(*reinterpret_cast<__half2*>(&v3), k16th, __hneg2(k64));
-    out[0] = *reinterpret_cast<uint32_t*>(&h0);
-    out[1] = *reinterpret_cast<uint32_t*>(&h1);
-    out[2] = *reinterpret_cast<uint32_t*>(&h2);
-    out[3] = *reinterpret_cast<uint32_t*>(&h3);
+    const uint32_t lo = x << 2, hi = x >> 6;
+    out[0] = lo & 0x003C003Cu;
+    out[1] = lo & 0x03C003C0u;
+    out[2] = hi & 0x003C003Cu;
+    out[3] = hi & 0x03C003C0u;
   };
 
-  // B fragments of Q^T (n = query row nt*8 + r) in the permuted order of d, as
-  // f16 of q * 2^-k with k chosen per row so that nothing overflows
+  // B fragments of Q^T (n = query row nt*8 + r) in the permuted order of d, as f16 of q * 2^k
   uint32_t qf[NTQ][KS][2];
-  float qsum[NTQ][2];  // sum over d of the scaled q, for the rows 2c, 2c+1 of each n-tile
-  float qfac[NTQ][2];  // 2^k * softmax scale * log2(e) of those rows
+  QuantRows<NTQ> rows;
 #pragma unroll
   for (int nt = 0; nt < NTQ; ++nt) {
     const T* qrow = reinterpret_cast<const T*>(w.qs + (nt * 8 + r) * kQRowBytes);
-    float amax = 0.f;
-    for (int d = c; d < D; d += 4) amax = fmaxf(amax, fabsf(float(qrow[d])));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    int kexp = 0;
-    if (amax >= 32768.f && amax < INFINITY) kexp = int(__float_as_uint(amax) >> 23) - 127 - 14;
-    const float qmul = __uint_as_float(uint32_t(127 - kexp) << 23);  // 2^-k
-    float sr = 0.f;  // the quad of row r adds up that row, then rows 2c, 2c+1 are fetched
-    for (int d = c; d < D; d += 4) sr += __half2float(__float2half_rn(float(qrow[d]) * qmul));
-    sr += __shfl_xor_sync(0xffffffffu, sr, 1);
-    sr += __shfl_xor_sync(0xffffffffu, sr, 2);
-    const float fac = __uint_as_float(uint32_t(127 + kexp) << 23) * a.scale_log2;
-    qsum[nt][0] = __shfl_sync(0xffffffffu, sr, 8 * c);
-    qsum[nt][1] = __shfl_sync(0xffffffffu, sr, 8 * c + 4);
-    qfac[nt][0] = __shfl_sync(0xffffffffu, fac, 8 * c);
-    qfac[nt][1] = __shfl_sync(0xffffffffu, fac, 8 * c + 4);
+    const int kexp = quant_q_exponent<D>(qrow, c);
+    quant_rows_init<D>(rows, nt, qrow, kexp, a, w);
+    const float qmul = exp2_int(kexp);
 #pragma unroll
     for (int ks = 0; ks < KS; ++ks) {
       const T* q0 = qrow + (4 * (ks >> 1) + c) * 8;
@@ -551,214 +720,105 @@ __device__ __forceinline__ void consume_int4(const DecodeArgs& a, const DecWarp&
       qf[nt][ks][1] = pk(q0, e0 + 1, e0 + 5);
     }
   }
+  quant_rows_limit(rows, w.chunk_hi);
   // Q now lives in registers: release the staging area to the producer
   __syncwarp();
   if (lane == 0) mbar_arrive(w.q_done_bar);
 
-  // per-query-row visibility limit: token t visible iff t < lim
-  // per-query-row visibility limit: token t visible iff t < lim (a window with several queries per sequence, which
-  // also has lower limits, is served by the 16-bit consumer only)
-  int lim[NTQ][2];
-  int lim_min = w.chunk_hi;  // below it nothing is masked for any row of this warp
+  float acc[MTV][NTQ][4];
 #pragma unroll
   for (int nt = 0; nt < NTQ; ++nt)
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int row = w.row0 + nt * 8 + 2 * c + e;
-      int l = w.chunk_hi;
-      if (a.causal && row < R) l = min(l, w.kv_len - a.mq + row / a.q_per_kv + 1);
-      lim[nt][e] = l;
-      lim_min = min(lim_min, l);
-    }
-  lim_min = min(lim_min, __shfl_xor_sync(0xffffffffu, lim_min, 1));
-  lim_min = min(lim_min, __shfl_xor_sync(0xffffffffu, lim_min, 2));
-
-  float acc[MTV][NTQ][4];
-  float m_run[NTQ][2], l_run[NTQ][2], corr[NTQ][2];
-#pragma unroll
-  for (int nt = 0; nt < NTQ; ++nt) {
-#pragma unroll
     for (int mt = 0; mt < MTV; ++mt) acc[mt][nt][0] = acc[mt][nt][1] = acc[mt][nt][2] = acc[mt][nt][3] = 0.f;
-    m_run[nt][0] = m_run[nt][1] = -INFINITY;
-    l_run[nt][0] = l_run[nt][1] = 0.f;
-    corr[nt][0] = corr[nt][1] = 0.f;
-  }
 
-  const int rw = row_bytes / 4;  // words per token row of the stage
+  constexpr int rw = HB * W;                             // words per token row of the stage
+  constexpr int u_step = 16 * (kDecConsumerWarps / HB);  // tokens from one sub-tile of this warp to its next
+  int st = 0;
+  uint32_t phase = 0;
   for (int tile = 0; tile < w.n_tiles; ++tile) {
-    const int st = tile % w.stages;
-    if (!mbar_wait(&w.full_bar[st], (tile / w.stages) & 1)) {
+    if (!mbar_wait(&w.full_bar[st], phase)) {
       if (lane == 0) atomicCAS(a.status, 0, 2);
       break;
     }
-    const uint32_t* kst = reinterpret_cast<const uint32_t*>(w.stage_base + st * w.stage_bytes) + hw * W;
+    const uint32_t* kst = reinterpret_cast<const uint32_t*>(w.stage_base + st * w.stage_bytes) + hw * W + w.sub * 16 * rw;
     const uint32_t* vst = kst + w.kv_bytes / 4;
-#pragma unroll 1
-    for (int sp = 0; sp < kSps; ++sp) {
-      const int usub = w.sub + w.wph * sp;                                // this warp's sub-tile of the stage
-      const int t_sub = w.chunk_lo + tile * w.tok_per_stage + usub * 16;  // its first token
-      if (t_sub >= w.chunk_hi) continue;
-      const uint32_t* k0 = kst + (usub * 16 + r) * rw;  // token r; token r + 8 is 8 rows on
-      const uint32_t* v0 = vst + (usub * 16 + r) * rw;
+    const int t_sub = w.chunk_lo + tile * w.tok_per_stage + w.sub * 16;  // first token of the step (a second sub-tile past the end is masked)
+    if (t_sub < w.chunk_hi) {
+      const uint32_t* k0 = kst + r * rw;  // token r; token r + 8 is 8 rows on
 
-      // ------------------------------------------- S^T = K Q^T (16 tokens x 8*NTQ)
-      float s[NTQ][4], s2[NTQ][4];  // two chains of dependent MMAs instead of one
+      // ------------------------------------------- S^T = K Q^T (16 tokens x 8*NTQ, U times)
+      float s[U][NTQ][4];
+      uint32_t kw[U][2], vw[U][2];
 #pragma unroll
-      for (int nt = 0; nt < NTQ; ++nt) {
-        s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
-        s2[nt][0] = s2[nt][1] = s2[nt][2] = s2[nt][3] = 0.f;
+      for (int u = 0; u < U; ++u) {
+        kw[u][0] = k0[u * u_step * rw], kw[u][1] = k0[(u * u_step + 8) * rw];
+        vw[u][0] = vst[(u * u_step + r) * rw], vw[u][1] = vst[(u * u_step + r + 8) * rw];
+#pragma unroll
+        for (int nt = 0; nt < NTQ; ++nt) s[u][nt][0] = s[u][nt][1] = s[u][nt][2] = s[u][nt][3] = 0.f;
       }
 #pragma unroll
       for (int i = 0; i < KS / 2; ++i) {
-        uint32_t u0[4], u1[4];
-        unpack4(k0[1 + 4 * i + c], u0);
-        unpack4(k0[8 * rw + 1 + 4 * i + c], u1);
-        const uint32_t ka[4] = {u0[0], u1[0], u0[1], u1[1]};
-        const uint32_t kb[4] = {u0[2], u1[2], u0[3], u1[3]};
 #pragma unroll
-        for (int nt = 0; nt < NTQ; ++nt) {
-          mma_16816<false>(s[nt], ka, qf[nt][2 * i][0], qf[nt][2 * i][1]);
-          mma_16816<false>(s2[nt], kb, qf[nt][2 * i + 1][0], qf[nt][2 * i + 1][1]);
+        for (int u = 0; u < U; ++u) {
+          uint32_t u0[4], u1[4];
+          unpack4(k0[u * u_step * rw + 1 + 4 * i + c], u0);
+          unpack4(k0[(u * u_step + 8) * rw + 1 + 4 * i + c], u1);
+#pragma unroll
+          for (int e = 0; e < 4; e += 2) u0[e] *= 16u, u1[e] *= 16u;  // (on the FMA pipe)
+          const uint32_t ka[4] = {u0[0], u1[0], u0[1], u1[1]};
+          const uint32_t kb[4] = {u0[2], u1[2], u0[3], u1[3]};
+#pragma unroll
+          for (int nt = 0; nt < NTQ; ++nt) {
+            mma_16816<false>(s[u][nt], ka, qf[nt][2 * i][0], qf[nt][2 * i][1]);
+            mma_16816<false>(s[u][nt], kb, qf[nt][2 * i + 1][0], qf[nt][2 * i + 1][1]);
+          }
         }
       }
 
-      // ------------------ scale/shift of tokens r, r+8; mask; online softmax
-      const uint32_t kw0 = k0[0], kw1 = k0[8 * rw], vw0 = v0[0], vw1 = v0[8 * rw];
-      const float ksc0 = half_bits_to_float(kw0 & 0xFFFFu), ksh0 = half_bits_to_float(kw0 >> 16);
-      const float ksc1 = half_bits_to_float(kw1 & 0xFFFFu), ksh1 = half_bits_to_float(kw1 >> 16);
-      float vsc0 = half_bits_to_float(vw0 & 0xFFFFu), vsh0 = half_bits_to_float(vw0 >> 16);
-      float vsc1 = half_bits_to_float(vw1 & 0xFFFFu), vsh1 = half_bits_to_float(vw1 >> 16);
-      const bool all_visible = t_sub + 16 <= lim_min;  // warp-uniform
-      float sc0[NTQ][2], sc1[NTQ][2];                  // scores of tokens r / r+8, log2 domain
-      bool need = false;
-#pragma unroll
-      for (int nt = 0; nt < NTQ; ++nt)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          sc0[nt][e] = fmaf(ksc0, s[nt][e] + s2[nt][e], ksh0 * qsum[nt][e]) * qfac[nt][e];
-          sc1[nt][e] = fmaf(ksc1, s[nt][2 + e] + s2[nt][2 + e], ksh1 * qsum[nt][e]) * qfac[nt][e];
-        }
-      if (!all_visible) {
-        const int t0 = t_sub + r, t1 = t_sub + r + 8;
-        // tokens past the end were not copied: their scale words are garbage
-        if (t0 >= w.chunk_hi) vsc0 = 0.f, vsh0 = 0.f;
-        if (t1 >= w.chunk_hi) vsc1 = 0.f, vsh1 = 0.f;
-#pragma unroll
-        for (int nt = 0; nt < NTQ; ++nt)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            if (t0 >= lim[nt][e]) sc0[nt][e] = -INFINITY;
-            if (t1 >= lim[nt][e]) sc1[nt][e] = -INFINITY;
-          }
-      }
-#pragma unroll
-      for (int nt = 0; nt < NTQ; ++nt)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) need |= fmaxf(sc0[nt][e], sc1[nt][e]) > m_run[nt][e] + kLazy;
-      if (__any_sync(0xffffffffu, need)) {
-        // some row's maximum grew by more than the slack: refresh all of them
-#pragma unroll
-        for (int nt = 0; nt < NTQ; ++nt) {
-          float alpha[2];
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            float mx = fmaxf(sc0[nt][e], sc1[nt][e]);
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-            const float m_new = fmaxf(m_run[nt][e], mx);
-            alpha[e] = fast_exp2(m_run[nt][e] - (m_new == -INFINITY ? 0.f : m_new));  // exp2(-inf) = 0 at first
-            m_run[nt][e] = m_new;
-            l_run[nt][e] *= alpha[e];
-            corr[nt][e] *= alpha[e];
-          }
-#pragma unroll
-          for (int mt = 0; mt < MTV; ++mt) {
-            acc[mt][nt][0] *= alpha[0];
-            acc[mt][nt][1] *= alpha[1];
-            acc[mt][nt][2] *= alpha[0];
-            acc[mt][nt][3] *= alpha[1];
-          }
-        }
-      }
-      uint32_t pb[NTQ][2];
-#pragma unroll
-      for (int nt = 0; nt < NTQ; ++nt) {
-        float p0[2], p1[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const float m_use = m_run[nt][e] == -INFINITY ? 0.f : m_run[nt][e];
-          p0[e] = fast_exp2(sc0[nt][e] - m_use);
-          p1[e] = fast_exp2(sc1[nt][e] - m_use);
-          l_run[nt][e] += p0[e] + p1[e];
-          corr[nt][e] = fmaf(p0[e], vsh0, fmaf(p1[e], vsh1, corr[nt][e]));
-        }
-        // V's scale rides on the probabilities
-        pb[nt][0] = movmatrix_trans(pack2<false>(p0[0] * vsc0, p0[1] * vsc0));  // tokens 2c, 2c+1   of row r
-        pb[nt][1] = movmatrix_trans(pack2<false>(p1[0] * vsc1, p1[1] * vsc1));  // tokens 2c+8, 2c+9 of row r
-      }
+      uint32_t pb[U][NTQ][2];
+      quant_softmax(rows, s, kw, vw, 262144.f, t_sub, u_step, w.chunk_hi, r, acc, pb);
 
       // ------------------------------------------------- O^T += V^T P^T
-      const uint32_t* va = vst + (usub * 16 + 2 * c) * rw + 1 + WPT * r;
 #pragma unroll
-      for (int wi = 0; wi < WPT; ++wi) {
-        const uint32_t x0 = va[wi], x1 = va[rw + wi], x2 = va[8 * rw + wi], x3 = va[9 * rw + wi];
-        // low / high half-words of two neighbouring tokens side by side
-        uint32_t ylo[4], yhi[4], zlo[4], zhi[4];
-        unpack4(__byte_perm(x0, x1, 0x5410), ylo);  // nibbles e   of tokens 2c,   2c+1 -> rows r
-        unpack4(__byte_perm(x0, x1, 0x7632), yhi);  // nibbles e+4 of tokens 2c,   2c+1 -> rows r+8
-        unpack4(__byte_perm(x2, x3, 0x5410), zlo);  // nibbles e   of tokens 2c+8, 2c+9
-        unpack4(__byte_perm(x2, x3, 0x7632), zhi);
-        // unpack4 pairs nibble e of the low half with nibble e of the high half
-        // (its "e + 4"), i.e. the same element of the two tokens: out[0..3] are
-        // elements 0, 1, 2, 3 of the half-word
+      for (int u = 0; u < U; ++u) {
+        const uint32_t* va = vst + (u * u_step + 2 * c) * rw + 1 + WPT * r;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const uint32_t vf[4] = {ylo[e], yhi[e], zlo[e], zhi[e]};
+        for (int wi = 0; wi < WPT; ++wi) {
+          const uint32_t x0 = va[wi], x1 = va[rw + wi], x2 = va[8 * rw + wi], x3 = va[9 * rw + wi];
+          // low / high half-words of two neighbouring tokens side by side
+          uint32_t ylo[4], yhi[4], zlo[4], zhi[4];
+          unpack4(__byte_perm(x0, x1, 0x5410), ylo);  // nibbles e   of tokens 2c,   2c+1 -> rows r
+          unpack4(__byte_perm(x0, x1, 0x7632), yhi);  // nibbles e+4 of tokens 2c,   2c+1 -> rows r+8
+          unpack4(__byte_perm(x2, x3, 0x5410), zlo);  // nibbles e   of tokens 2c+8, 2c+9
+          unpack4(__byte_perm(x2, x3, 0x7632), zhi);
+          // unpack4 pairs nibble e of the low half with nibble e of the high half
+          // (its "e + 4"), i.e. the same element of the two tokens: out[0..3] are
+          // elements 0, 1, 2, 3 of the half-word
 #pragma unroll
-          for (int nt = 0; nt < NTQ; ++nt) mma_16816<false>(acc[wi * 4 + e][nt], vf, pb[nt][0], pb[nt][1]);
+          for (int e = 0; e < 4; ++e) {
+            const uint32_t vf[4] = {ylo[e], yhi[e], zlo[e], zhi[e]};
+#pragma unroll
+            for (int nt = 0; nt < NTQ; ++nt) mma_16816<false>(acc[wi * 4 + e][nt], vf, pb[u][nt][0], pb[u][nt][1]);
+          }
         }
       }
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(&w.empty_bar[st]);
+    if (++st == w.stages) st = 0, phase ^= 1;
   }
 
-  // full row sums (each thread saw tokens r and r+8 of every sub-tile)
+  quant_rows_finish<D>(rows, w);
 #pragma unroll
   for (int nt = 0; nt < NTQ; ++nt)
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      float l = l_run[nt][e], cs = corr[nt][e];
-#pragma unroll
-      for (int o = 4; o < 32; o <<= 1) {
-        l += __shfl_xor_sync(0xffffffffu, l, o);
-        cs += __shfl_xor_sync(0xffffffffu, cs, o);
-      }
-      l_run[nt][e] = l;
-      corr[nt][e] = cs;
-    }
-
-  // the ring is no longer in use once every consumer warp got here
-  asm volatile("bar.sync 1, %0;" ::"n"(kDecConsumerWarps * 32) : "memory");
-#pragma unroll
-  for (int nt = 0; nt < NTQ; ++nt) {
 #pragma unroll
     for (int mt = 0; mt < MTV; ++mt)
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int d = 8 * (WPT * r + (mt >> 2)) + (mt & 3) + (q >> 1) * 4;
         const int rr = nt * 8 + 2 * c + (q & 1);
-        w.mine[rr * kCmbRow + d] = acc[mt][nt][q] + corr[nt][q & 1];
+        w.mine[rr * kCmbRow + d] = fmaf(acc[mt][nt][q], (mt & 1) ? 262144.f : 4194304.f, rows.corr[nt][q & 1]);
       }
-    if (r == 0) {
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        w.mine[(nt * 8 + 2 * c + e) * kCmbRow + D] = m_run[nt][e];
-        w.mine[(nt * 8 + 2 * c + e) * kCmbRow + D + 1] = l_run[nt][e];
-      }
-    }
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1164,36 +1224,21 @@ __device__ __forceinline__ void consume_fp8(const DecodeArgs& a, const DecWarp& 
   constexpr int kQRowBytes = D * 2;
   constexpr int kCmbRow = D + 2;
   constexpr int kSps = DecStage<D, kFmtFp8>::kSubTiles;
-  constexpr float kLazy = 4.f;  // as in the int4 consumer
   const int lane = w.lane, r = lane >> 2, c = lane & 3;
-  const int R = a.rows, hw = w.hw, hb = a.hb;
+  const int hw = w.hw, hb = a.hb;
   const int box_shift = __ffs(a.box_tok) - 1;
   const int head_bytes = a.box_tok * 128;      // one head of a box
   const int box_bytes = head_bytes * hb;
 
-  // B fragments of Q^T (n = query row nt*8 + r): f16 of q * 2^-k, k per row so that nothing overflows
+  // B fragments of Q^T (n = query row nt*8 + r): f16 of q * 2^k
   uint32_t qf[NTQ][KS][2];
-  float qsum[NTQ][2];  // sum over d of the scaled q, rows 2c, 2c+1 of each n-tile
-  float qfac[NTQ][2];  // 2^k * softmax scale * log2(e) of those rows
+  QuantRows<NTQ> rows;
 #pragma unroll
   for (int nt = 0; nt < NTQ; ++nt) {
     const T* qrow = reinterpret_cast<const T*>(w.qs + (nt * 8 + r) * kQRowBytes);
-    float amax = 0.f;
-    for (int d = c; d < D; d += 4) amax = fmaxf(amax, fabsf(float(qrow[d])));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    int kexp = 0;
-    if (amax >= 32768.f && amax < INFINITY) kexp = int(__float_as_uint(amax) >> 23) - 127 - 14;
-    const float qmul = __uint_as_float(uint32_t(127 - kexp) << 23);  // 2^-k
-    float sr = 0.f;
-    for (int d = c; d < D; d += 4) sr += __half2float(__float2half_rn(float(qrow[d]) * qmul));
-    sr += __shfl_xor_sync(0xffffffffu, sr, 1);
-    sr += __shfl_xor_sync(0xffffffffu, sr, 2);
-    const float fac = __uint_as_float(uint32_t(127 + kexp) << 23) * a.scale_log2;
-    qsum[nt][0] = __shfl_sync(0xffffffffu, sr, 8 * c);
-    qsum[nt][1] = __shfl_sync(0xffffffffu, sr, 8 * c + 4);
-    qfac[nt][0] = __shfl_sync(0xffffffffu, fac, 8 * c);
-    qfac[nt][1] = __shfl_sync(0xffffffffu, fac, 8 * c + 4);
+    const int kexp = min(quant_q_exponent<D>(qrow, c), 0);  // only downwards: f16 values of ordinary queries are exact
+    quant_rows_init<D>(rows, nt, qrow, kexp, a, w);
+    const float qmul = exp2_int(kexp);
 #pragma unroll
     for (int ks = 0; ks < KS; ++ks) {
       const T* q0 = qrow + 16 * ks + 4 * c;
@@ -1203,52 +1248,32 @@ __device__ __forceinline__ void consume_fp8(const DecodeArgs& a, const DecWarp& 
       qf[nt][ks][1] = *reinterpret_cast<const uint32_t*>(&h23);
     }
   }
+  quant_rows_limit(rows, w.chunk_hi);
   // Q now lives in registers: release the staging area to the producer
   __syncwarp();
   if (lane == 0) mbar_arrive(w.q_done_bar);
 
-  // per-query-row visibility limit: token t visible iff t < lim (a window with several queries per sequence, which
-  // also has lower limits, is served by the 16-bit consumer only)
-  int lim[NTQ][2];
-  int lim_min = w.chunk_hi;  // below it nothing is masked for any row of this warp
+  float acc[MTV][NTQ][4];
 #pragma unroll
   for (int nt = 0; nt < NTQ; ++nt)
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int row = w.row0 + nt * 8 + 2 * c + e;
-      int l = w.chunk_hi;
-      if (a.causal && row < R) l = min(l, w.kv_len - a.mq + row / a.q_per_kv + 1);
-      lim[nt][e] = l;
-      lim_min = min(lim_min, l);
-    }
-  lim_min = min(lim_min, __shfl_xor_sync(0xffffffffu, lim_min, 1));
-  lim_min = min(lim_min, __shfl_xor_sync(0xffffffffu, lim_min, 2));
-
-  float acc[MTV][NTQ][4];
-  float m_run[NTQ][2], l_run[NTQ][2], corr[NTQ][2];
-#pragma unroll
-  for (int nt = 0; nt < NTQ; ++nt) {
-#pragma unroll
     for (int mt = 0; mt < MTV; ++mt) acc[mt][nt][0] = acc[mt][nt][1] = acc[mt][nt][2] = acc[mt][nt][3] = 0.f;
-    m_run[nt][0] = m_run[nt][1] = -INFINITY;
-    l_run[nt][0] = l_run[nt][1] = 0.f;
-    corr[nt][0] = corr[nt][1] = 0.f;
-  }
 
+  // scale/shift words of a stage: [token][head][4 words] (tiled copies of replicated words), [token][head]
+  // (tiled copies of compact words) or [head][token] (4-byte copies)
+  const int ss_head = a.ss_tma == 1 ? hw * 4 : a.ss_tma == 2 ? hw : hw * w.tok_per_stage;
+  const int ss_step = a.ss_tma == 1 ? hb * 4 : a.ss_tma == 2 ? hb : 1;  // words from one token to the next
+  int st = 0;
+  uint32_t phase = 0;
   for (int tile = 0; tile < w.n_tiles; ++tile) {
-    const int st = tile % w.stages;
-    if (!mbar_wait(&w.full_bar[st], (tile / w.stages) & 1)) {
+    if (!mbar_wait(&w.full_bar[st], phase)) {
       if (lane == 0) atomicCAS(a.status, 0, 2);
       break;
     }
     const uint8_t* kst = w.stage_base + st * w.stage_bytes;
     const uint8_t* vst = kst + w.kv_bytes;
-    // scale/shift words: [head][token] after the 4-byte copies, [token][head][4 words] after the tiled ones
-    // scale/shift words of a stage: [token][head][4 words] (tiled copies of replicated words), [token][head]
-    // (tiled copies of compact words) or [head][token] (4-byte copies)
-    const uint32_t* ssk = reinterpret_cast<const uint32_t*>(kst + 2 * w.kv_bytes) + (a.ss_tma == 1 ? hw * 4 : a.ss_tma == 2 ? hw : hw * w.tok_per_stage);
+    const uint32_t* ssk = reinterpret_cast<const uint32_t*>(kst + 2 * w.kv_bytes) + ss_head;
     const uint32_t* ssv = ssk + a.ss_bytes / 4;
-    const int ss_step = a.ss_tma == 1 ? hb * 4 : a.ss_tma == 2 ? hb : 1;  // words from one token to the next
 #pragma unroll 1
     for (int sp = 0; sp < kSps; ++sp) {
       const int usub = w.sub + w.wph * sp;                                // this warp's sub-tile of the stage
@@ -1258,12 +1283,10 @@ __device__ __forceinline__ void consume_fp8(const DecodeArgs& a, const DecWarp& 
       const int boff = (tok0 >> box_shift) * box_bytes + hw * head_bytes + (tok0 & (a.box_tok - 1)) * 128;
 
       // ------------------------------------------- S^T = K Q^T (16 tokens x 8*NTQ)
-      float s[NTQ][4], s2[NTQ][4];  // two chains of dependent MMAs instead of one
+      // (one chain of dependent MMAs: a second one costs registers and four additions, 385.6 against 384.1 us)
+      float s[1][NTQ][4];
 #pragma unroll
-      for (int nt = 0; nt < NTQ; ++nt) {
-        s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
-        s2[nt][0] = s2[nt][1] = s2[nt][2] = s2[nt][3] = 0.f;
-      }
+      for (int nt = 0; nt < NTQ; ++nt) s[0][nt][0] = s[0][nt][1] = s[0][nt][2] = s[0][nt][3] = 0.f;
       {
         const uint8_t* k0 = kst + boff + r * 128 + c * 4;  // token r (chunk swizzle r & 7 = r); token r + 8 is 8 rows on, same swizzle
 #pragma unroll
@@ -1275,98 +1298,27 @@ __device__ __forceinline__ void consume_fp8(const DecodeArgs& a, const DecWarp& 
           cvt_e4m3x4(w0, ka[0], ka[2]);
           cvt_e4m3x4(w1, ka[1], ka[3]);
 #pragma unroll
-          for (int nt = 0; nt < NTQ; ++nt) mma_16816<false>((ks & 1) ? s2[nt] : s[nt], ka, qf[nt][ks][0], qf[nt][ks][1]);
+          for (int nt = 0; nt < NTQ; ++nt) mma_16816<false>(s[0][nt], ka, qf[nt][ks][0], qf[nt][ks][1]);
         }
       }
 
-      // ------------------ scale/shift of tokens r, r+8; mask; online softmax
-      const uint32_t kw0 = ssk[(tok0 + r) * ss_step], kw1 = ssk[(tok0 + r + 8) * ss_step];
-      const uint32_t vw0 = ssv[(tok0 + r) * ss_step], vw1 = ssv[(tok0 + r + 8) * ss_step];
-      const float ksc0 = half_bits_to_float(kw0 & 0xFFFFu), ksh0 = half_bits_to_float(kw0 >> 16);
-      const float ksc1 = half_bits_to_float(kw1 & 0xFFFFu), ksh1 = half_bits_to_float(kw1 >> 16);
-      float vsc0 = half_bits_to_float(vw0 & 0xFFFFu), vsh0 = half_bits_to_float(vw0 >> 16);
-      float vsc1 = half_bits_to_float(vw1 & 0xFFFFu), vsh1 = half_bits_to_float(vw1 >> 16);
-      const bool all_visible = t_sub + 16 <= lim_min;  // warp-uniform
-      float sc0[NTQ][2], sc1[NTQ][2];                  // scores of tokens r / r+8, log2 domain
-      bool need = false;
-#pragma unroll
-      for (int nt = 0; nt < NTQ; ++nt)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          sc0[nt][e] = fmaf(ksc0, s[nt][e] + s2[nt][e], ksh0 * qsum[nt][e]) * qfac[nt][e];
-          sc1[nt][e] = fmaf(ksc1, s[nt][2 + e] + s2[nt][2 + e], ksh1 * qsum[nt][e]) * qfac[nt][e];
-        }
-      if (!all_visible) {
-        const int t0 = t_sub + r, t1 = t_sub + r + 8;
-        // tokens past the end were not copied: their scale words are garbage
-        if (t0 >= w.chunk_hi) vsc0 = 0.f, vsh0 = 0.f;
-        if (t1 >= w.chunk_hi) vsc1 = 0.f, vsh1 = 0.f;
-#pragma unroll
-        for (int nt = 0; nt < NTQ; ++nt)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            if (t0 >= lim[nt][e]) sc0[nt][e] = -INFINITY;
-            if (t1 >= lim[nt][e]) sc1[nt][e] = -INFINITY;
-          }
-      }
-#pragma unroll
-      for (int nt = 0; nt < NTQ; ++nt)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) need |= fmaxf(sc0[nt][e], sc1[nt][e]) > m_run[nt][e] + kLazy;
-      if (__any_sync(0xffffffffu, need)) {
-#pragma unroll
-        for (int nt = 0; nt < NTQ; ++nt) {
-          float alpha[2];
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            float mx = fmaxf(sc0[nt][e], sc1[nt][e]);
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-            const float m_new = fmaxf(m_run[nt][e], mx);
-            alpha[e] = fast_exp2(m_run[nt][e] - (m_new == -INFINITY ? 0.f : m_new));
-            m_run[nt][e] = m_new;
-            l_run[nt][e] *= alpha[e];
-            corr[nt][e] *= alpha[e];
-          }
-#pragma unroll
-          for (int mt = 0; mt < MTV; ++mt) {
-            acc[mt][nt][0] *= alpha[0];
-            acc[mt][nt][1] *= alpha[1];
-            acc[mt][nt][2] *= alpha[0];
-            acc[mt][nt][3] *= alpha[1];
-          }
-        }
-      }
-      uint32_t pb[NTQ][2];
-#pragma unroll
-      for (int nt = 0; nt < NTQ; ++nt) {
-        float p0[2], p1[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const float m_use = m_run[nt][e] == -INFINITY ? 0.f : m_run[nt][e];
-          p0[e] = fast_exp2(sc0[nt][e] - m_use);
-          p1[e] = fast_exp2(sc1[nt][e] - m_use);
-          l_run[nt][e] += p0[e] + p1[e];
-          corr[nt][e] = fmaf(p0[e], vsh0, fmaf(p1[e], vsh1, corr[nt][e]));
-        }
-        pb[nt][0] = movmatrix_trans(pack2<false>(p0[0] * vsc0, p0[1] * vsc0));  // tokens 2c, 2c+1   of row r
-        pb[nt][1] = movmatrix_trans(pack2<false>(p1[0] * vsc1, p1[1] * vsc1));  // tokens 2c+8, 2c+9 of row r
-      }
+      const uint32_t kw[1][2] = {{ssk[(tok0 + r) * ss_step], ssk[(tok0 + r + 8) * ss_step]}};
+      const uint32_t vw[1][2] = {{ssv[(tok0 + r) * ss_step], ssv[(tok0 + r + 8) * ss_step]}};
+      uint32_t pb[1][NTQ][2];
+      quant_softmax(rows, s, kw, vw, 1.f, t_sub, 0, w.chunk_hi, r, acc, pb);
 
       // ------------------------------------------------- O^T += V^T P^T
       {
-        const uint8_t* v0 = vst + boff + (2 * c) * 128 + (r & 3) * 4;  // token 2c; +128: 2c+1; +1024: 2c+8; +1152: 2c+9
-        const int x0s = (2 * c) & 7, x1s = (2 * c + 1) & 7;            // chunk swizzles of the even / odd token
-        // Bytes of tokens past the end were never copied and may hold the NaN patterns of
-        // e4m3 (0 x NaN = NaN): they are cleared before the conversion.  After the byte
-        // permute, bytes 0 and 2 belong to the even token, bytes 1 and 3 to the odd one.
-        uint32_t vmask_a = 0xFFFFFFFFu, vmask_b = 0xFFFFFFFFu;
-        if (!all_visible) {
-          const int tv = t_sub + 2 * c;
-          vmask_a = (tv < w.chunk_hi ? 0x00FF00FFu : 0u) | (tv + 1 < w.chunk_hi ? 0xFF00FF00u : 0u);
-          vmask_b = (tv + 8 < w.chunk_hi ? 0x00FF00FFu : 0u) | (tv + 9 < w.chunk_hi ? 0xFF00FF00u : 0u);
+        const uint8_t* vb = vst + boff;
+        if (t_sub + 16 > w.chunk_hi) {
+          // Rows of tokens past the end were never copied and may hold the NaN patterns of e4m3 (0 x NaN = NaN): cleared
+          // (whole 128-byte rows, so the swizzle does not matter; nothing is copied into this stage any more).
+          for (int i = lane; i < 16 * 8; i += 32)
+            if (t_sub + (i >> 3) >= w.chunk_hi) *reinterpret_cast<uint4*>(const_cast<uint8_t*>(vb) + i * 16) = make_uint4(0, 0, 0, 0);
+          __syncwarp();
         }
+        const uint8_t* v0 = vb + (2 * c) * 128 + (r & 3) * 4;  // token 2c; +128: 2c+1; +1024: 2c+8; +1152: 2c+9
+        const int x0s = (2 * c) & 7, x1s = (2 * c + 1) & 7;    // chunk swizzles of the even / odd token
 #pragma unroll
         for (int wj = 0; wj < WJ; ++wj) {
           const int ch = (r >> 2) + 2 * wj;  // 16-byte chunk of word r + 8 wj
@@ -1376,62 +1328,40 @@ __device__ __forceinline__ void consume_fp8(const DecodeArgs& a, const DecWarp& 
           const uint32_t xd = *reinterpret_cast<const uint32_t*>(v0 + 1152 + (ch ^ x1s) * 16);
           // bytes (a0 b0 a1 b1) and (a2 b2 a3 b3): element e of the two tokens side by side
           uint32_t y01[2], y23[2], z01[2], z23[2];
-          cvt_e4m3x4(__byte_perm(xa, xb, 0x5140) & vmask_a, y01[0], y01[1]);
-          cvt_e4m3x4(__byte_perm(xa, xb, 0x7362) & vmask_a, y23[0], y23[1]);
-          cvt_e4m3x4(__byte_perm(xc, xd, 0x5140) & vmask_b, z01[0], z01[1]);
-          cvt_e4m3x4(__byte_perm(xc, xd, 0x7362) & vmask_b, z23[0], z23[1]);
+          cvt_e4m3x4(__byte_perm(xa, xb, 0x5140), y01[0], y01[1]);
+          cvt_e4m3x4(__byte_perm(xa, xb, 0x7362), y23[0], y23[1]);
+          cvt_e4m3x4(__byte_perm(xc, xd, 0x5140), z01[0], z01[1]);
+          cvt_e4m3x4(__byte_perm(xc, xd, 0x7362), z23[0], z23[1]);
 #pragma unroll
           for (int p = 0; p < 2; ++p) {
             const uint32_t vf[4] = {y01[p], y23[p], z01[p], z23[p]};  // rows r: d = 4(r+8wj)+p, rows r+8: d+2
 #pragma unroll
-            for (int nt = 0; nt < NTQ; ++nt) mma_16816<false>(acc[wj * 2 + p][nt], vf, pb[nt][0], pb[nt][1]);
+            for (int nt = 0; nt < NTQ; ++nt) mma_16816<false>(acc[wj * 2 + p][nt], vf, pb[0][nt][0], pb[0][nt][1]);
           }
         }
       }
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(&w.empty_bar[st]);
+    if (++st == w.stages) st = 0, phase ^= 1;
   }
 
-  // full row sums (each thread saw tokens r and r+8 of every sub-tile)
+  quant_rows_finish<D>(rows, w);
 #pragma unroll
   for (int nt = 0; nt < NTQ; ++nt)
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      float l = l_run[nt][e], cs = corr[nt][e];
-#pragma unroll
-      for (int o = 4; o < 32; o <<= 1) {
-        l += __shfl_xor_sync(0xffffffffu, l, o);
-        cs += __shfl_xor_sync(0xffffffffu, cs, o);
-      }
-      l_run[nt][e] = l;
-      corr[nt][e] = cs;
-    }
-
-  // the ring is no longer in use once every consumer warp got here
-  asm volatile("bar.sync 1, %0;" ::"n"(kDecConsumerWarps * 32) : "memory");
-#pragma unroll
-  for (int nt = 0; nt < NTQ; ++nt) {
 #pragma unroll
     for (int mt = 0; mt < MTV; ++mt)
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int d = 4 * (r + 8 * (mt >> 1)) + (mt & 1) + (q >> 1) * 2;
         const int rr = nt * 8 + 2 * c + (q & 1);
-        w.mine[rr * kCmbRow + d] = acc[mt][nt][q] + corr[nt][q & 1];
+        w.mine[rr * kCmbRow + d] = acc[mt][nt][q] + rows.corr[nt][q & 1];
       }
-    if (r == 0) {
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        w.mine[(nt * 8 + 2 * c + e) * kCmbRow + D] = m_run[nt][e];
-        w.mine[(nt * 8 + 2 * c + e) * kCmbRow + D + 1] = l_run[nt][e];
-      }
-    }
-  }
 }
 
-template <int D, int MT, int kFmt, bool kBf16, int NG = 1>
-__global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt>::kCtasPerSm) decode_splitk_kernel(const __grid_constant__ DecodeArgs a) {
+// HB: kv heads per CTA where the consumer wants to know them at compile time (int4, one quantisation group), else 0
+template <int D, int MT, int kFmt, bool kBf16, int NG, int HB>
+__global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt, MT>::kCtasPerSm) decode_splitk_kernel(const __grid_constant__ DecodeArgs a) {
   using Stage = DecStage<D, kFmt, NG>;
   constexpr bool kInt4 = kFmt == kFmtInt4, kFp8 = kFmt == kFmtFp8, kQuant = kFmt == kFmtInt4 || kFmt == kFmtFp8;
   using T = typename Half2Type<kBf16>::T;
@@ -1454,7 +1384,7 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt>::kCtasPerSm) d
   const int rblk = blockIdx.z % a.row_blocks;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int hb = a.hb;
+  const int hb = HB > 0 ? HB : a.hb;
   const int wph = kDecConsumerWarps / hb;  // consumer warps per kv head
   constexpr int kSps = Stage::kSubTiles;
   const int TOK = 16 * wph * kSps;
@@ -1704,7 +1634,7 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt>::kCtasPerSm) d
   w.chunk_lo = chunk_lo, w.chunk_hi = chunk_hi, w.kv_len = kv_len, w.n_tiles = n_tiles;
   w.tok_per_stage = TOK, w.kv_bytes = kv_bytes, w.stage_bytes = stage_bytes, w.row_bytes = row_bytes, w.stages = kDecStages;
   if constexpr (kInt4 && NG == 1)
-    consume_int4<D, MT, kBf16>(a, w);
+    consume_int4<D, MT, kBf16, HB>(a, w);
   else if constexpr (kInt4)
     consume_int4_groups<D, MT, kBf16, NG>(a, w);
   else if constexpr (kFp8)
@@ -1861,7 +1791,7 @@ int decode_chunk_tokens(int kv_bound, int split_k) {
   return c < kDecChunkAlign ? kDecChunkAlign : c;
 }
 
-template <int D, int MT, int kFmt, bool kBf16, int NG = 1>
+template <int D, int MT, int kFmt, bool kBf16, int NG, int HB>
 static int launch_decode_t(const DecodeArgs& a_in, int head_blocks, cudaStream_t stream) {
   using Stage = DecStage<D, kFmt, NG>;
   constexpr bool kQuant = kFmt == kFmtInt4 || kFmt == kFmtFp8;
@@ -1874,7 +1804,7 @@ static int launch_decode_t(const DecodeArgs& a_in, int head_blocks, cudaStream_t
   const size_t stage_bytes = 2 * size_t(kv_bytes) + 2 * size_t(ss_bytes);
   const size_t qbytes = size_t(kDecConsumerWarps) * ROWS * (D * 2);
   const size_t cmb = size_t(kDecConsumerWarps) * ROWS * (D + 2) * 4;
-  int stages = int(DecOccupancy<kFmt>::kRingBudget / stage_bytes);
+  int stages = int(DecOccupancy<kFmt, MT>::kRingBudget / stage_bytes);
   stages = stages > kDecMaxStages ? kDecMaxStages : stages;
   const int q_stages = kQuant ? int((qbytes + stage_bytes - 1) / stage_bytes) : 0;  // only the quantised paths stage Q
   if (stages < 2 || q_stages > stages) return set_error(XFB200_E_UNSUPPORTED, "decode: shared-memory ring too small for this shape");
@@ -1886,9 +1816,9 @@ static int launch_decode_t(const DecodeArgs& a_in, int head_blocks, cudaStream_t
   a.ss_bytes = ss_bytes;
   const size_t ring = stages * stage_bytes + 1024;  // the kernel aligns the ring to 1024 B
   const size_t smem = ring > cmb ? ring : cmb;
-  auto kern = decode_splitk_kernel<D, MT, kFmt, kBf16, NG>;
+  auto kern = decode_splitk_kernel<D, MT, kFmt, kBf16, NG, HB>;
   // 227 KB per CTA includes the static part (the mbarriers)
-  if (smem + 1024 > size_t(227 * 1024) / DecOccupancy<kFmt>::kCtasPerSm) return set_error(XFB200_E_UNSUPPORTED, "decode: shared memory %zu B exceeds 227 KB", smem);
+  if (smem + 1024 > size_t(227 * 1024) / DecOccupancy<kFmt, MT>::kCtasPerSm) return set_error(XFB200_E_UNSUPPORTED, "decode: shared memory %zu B exceeds 227 KB", smem);
   // per instantiation and device (the attribute belongs to the device's context): largest size opted into so far
   static size_t configured[kMaxDevices] = {0};
   const int dev = current_device();
@@ -1912,8 +1842,17 @@ static int launch_decode_t(const DecodeArgs& a_in, int head_blocks, cudaStream_t
 
 template <int D, int kFmt, bool kBf16, int NG = 1>
 static int launch_decode_mt(const DecodeArgs& a, int mt, int head_blocks, cudaStream_t stream) {
-  if (mt == 1) return launch_decode_t<D, 1, kFmt, kBf16, NG>(a, head_blocks, stream);
-  return launch_decode_t<D, 2, kFmt, kBf16, NG>(a, head_blocks, stream);
+  if constexpr (kFmt == kFmtInt4 && NG == 1) {
+    switch (a.hb) {
+      case 1: return mt == 1 ? launch_decode_t<D, 1, kFmt, kBf16, NG, 1>(a, head_blocks, stream) : launch_decode_t<D, 2, kFmt, kBf16, NG, 1>(a, head_blocks, stream);
+      case 2: return mt == 1 ? launch_decode_t<D, 1, kFmt, kBf16, NG, 2>(a, head_blocks, stream) : launch_decode_t<D, 2, kFmt, kBf16, NG, 2>(a, head_blocks, stream);
+      case 4: return mt == 1 ? launch_decode_t<D, 1, kFmt, kBf16, NG, 4>(a, head_blocks, stream) : launch_decode_t<D, 2, kFmt, kBf16, NG, 4>(a, head_blocks, stream);
+      default: return mt == 1 ? launch_decode_t<D, 1, kFmt, kBf16, NG, 8>(a, head_blocks, stream) : launch_decode_t<D, 2, kFmt, kBf16, NG, 8>(a, head_blocks, stream);
+    }
+  } else {
+    if (mt == 1) return launch_decode_t<D, 1, kFmt, kBf16, NG, 0>(a, head_blocks, stream);
+    return launch_decode_t<D, 2, kFmt, kBf16, NG, 0>(a, head_blocks, stream);
+  }
 }
 
 }  // namespace xfb

@@ -167,7 +167,7 @@ py::object prefill(const View& q, const View& k, const View& v, const Sequences*
 //   Where chunks of 1280 tokens fill the machine four times over: those (measured optimum for every cache format at 8 kv heads per
 // CTA: 24-32 chunks of a 32k context).
 //   Below: what a small model of the launch says is fastest.  A CTA costs about 3 us before and after its tokens; these come at
-// its share of the memory bandwidth, at most 90 GB/s; the CTAs run in waves of one per SM (two for quantised caches); partials
+// its share of the memory bandwidth, at most 90 GB/s; the CTAs run in waves of one per SM (two for quantised caches and up to 8 query rows); partials
 // are written and read once at 5 TB/s, and the merge itself costs 2 us.  Two sequences of 16384 keys, 2 kv heads, went from 128
 // chunks (256 CTAs, two waves, 128 partials per row) to 64: 16.4 + 28.7 us to the figures at decode_merge_kernel.
 int64_t split_k(int64_t batch, int64_t kv_bound, int64_t kv_heads, int64_t rows, int64_t row_bytes, bool quantised) {
@@ -177,7 +177,8 @@ int64_t split_k(int64_t batch, int64_t kv_bound, int64_t kv_heads, int64_t rows,
   const int64_t bound = (kv_bound + 127) / 128 * 128;
   auto chunks = [&](int64_t c) { return (bound + c - 1) / c; };
   if (batch * (kv_heads / hb0) * chunks(std::min<int64_t>(bound, 1280)) >= 4 * kSms) return chunks(std::min<int64_t>(bound, 1280));
-  const int64_t tile_rows = quantised ? 8 : 16, row_blocks = (rows + 2 * tile_rows - 1) / (2 * tile_rows), slots = quantised ? 2 * kSms : kSms;
+  const bool two = quantised && rows <= 8;  // CTAs per SM, as the library picks it
+  const int64_t tile_rows = quantised ? 8 : 16, row_blocks = (rows + 2 * tile_rows - 1) / (2 * tile_rows), slots = two ? 2 * kSms : kSms;
   int64_t best = 128;
   double best_us = 1e30;
   for (int64_t c = 128; c <= std::min<int64_t>(bound, 1280); c += 128) {
@@ -186,7 +187,7 @@ int64_t split_k(int64_t batch, int64_t kv_bound, int64_t kv_heads, int64_t rows,
     if (!quantised)
       while (hb > 1 && batch * (kv_heads / hb) * row_blocks * n * 2 <= kSms) hb /= 2;
     const int64_t ctas = batch * (kv_heads / hb) * row_blocks * n, waves = (ctas + slots - 1) / slots;
-    const double gbs = std::min(quantised ? 45.0 : 90.0, 6400.0 / double(std::min(ctas, slots)));
+    const double gbs = std::min(two ? 45.0 : 90.0, 6400.0 / double(std::min(ctas, slots)));
     const double us = double(waves) * (3.0 + double(std::min(c, bound) * hb * 2 * row_bytes) / (gbs * 1e3)) +
                       (n > 1 ? 2.0 + 2.0 * double(batch * kv_heads * n * rows) * 516.0 / 5e6 : 0.0);
     if (us < best_us * 0.98) best_us = us, best = c;
