@@ -1,11 +1,69 @@
-"""The order in which the prefill kernel takes the sequences of a packed batch."""
+"""Launches that begin before the kernel ahead of them has ended, and the order in which the prefill kernel takes sequences:
+results must be those of calls that are waited for, and of the oracle."""
 
 import pytest
 import torch
 
+import xformers_b200.ops as xops
 from gpu_utils import assert_o_lse, gpu, rand_qkv, ref, require_cuda
 from xformers_b200.ops import fmha
 from xformers_b200.ops.fmha import attn_bias as ab
+
+
+@gpu
+@pytest.mark.parametrize("capture", [False, True])
+@pytest.mark.parametrize("kv_heads,mq", [(8, 1), (1, 2)])
+def test_steps_back_to_back(kv_heads, mq, capture):
+    """Decoding steps whose every kernel reads what the one before it wrote (cache, lengths, partials, scratch that the
+    allocator hands out again)."""
+    require_cuda()
+    B, pad, G, D, steps = 3, 2048, 8, 128, 12
+    g = torch.Generator(device="cuda").manual_seed(11)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda", dtype=torch.bfloat16)
+    xq, xk, xv = rnd(1, B * mq, kv_heads, G, D), rnd(1, B * mq, kv_heads, 1, D), rnd(1, B * mq, kv_heads, 1, D)
+    ck0, cv0 = rnd(1, B * pad, kv_heads, 1, D), rnd(1, B * pad, kv_heads, 1, D)
+    lens0 = [5, 1400, 2000]
+
+    def run(wait, graph):
+        ck, cv, x = ck0.clone(), cv0.clone(), xq.clone()
+        bias = ab.BlockDiagonalCausalWithOffsetPaddedKeysMask.from_seqlens(q_seqlen=[mq] * B, kv_padding=pad, kv_seqlen=lens0, device="cuda")
+        k, v = (c.expand(-1, -1, -1, G, -1) for c in (ck, cv))
+
+        def step():
+            q = xops.rope_padded(x, xk, xv, ck, cv, bias)
+            if wait:
+                torch.cuda.synchronize()
+            parts = [fmha.memory_efficient_attention_partial(q, k, v, bias) for _ in range(2)]
+            if wait:
+                torch.cuda.synchronize()
+            out, lse = fmha.merge_attentions([o for o, _ in parts], [l for _, l in parts])
+            x.copy_(out)
+            bias.k_seqinfo.seqlen.add_(1)
+            return out, lse
+
+        outs = []
+        if graph:
+            warm = torch.cuda.Stream()
+            with torch.cuda.stream(warm):
+                step()
+            warm.synchronize()
+            cg = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(cg):
+                res = step()
+            ck.copy_(ck0), cv.copy_(cv0), x.copy_(xq), bias.k_seqinfo.seqlen.copy_(torch.tensor(lens0, dtype=torch.int32, device="cuda"))
+            for _ in range(steps):
+                cg.replay()
+                outs.append(tuple(t.clone() for t in res))
+        else:
+            for _ in range(steps):
+                outs.append(tuple(t.clone() for t in step()))
+        return outs, ck, cv
+
+    got, ck, cv = run(False, capture)
+    want, ck_w, cv_w = run(True, False)
+    assert torch.equal(ck, ck_w) and torch.equal(cv, cv_w)
+    for (o, l), (ow, lw) in zip(got, want):
+        assert torch.equal(o, ow) and torch.equal(l, lw)
 
 
 @gpu

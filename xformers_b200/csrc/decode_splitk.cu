@@ -1372,7 +1372,6 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt, MT>::kCtasPerS
 
   // bytes in flight per SM are what hide HBM latency: the ring takes ~200 KB,
   // i.e. 3 stages of 64 KB (bf16, D = 128) up to 12 stages of 17 KB (int4)
-  const int kDecStages = a.stages;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   __shared__ uint64_t full_bar[kDecMaxStages];
   __shared__ uint64_t empty_bar[kDecMaxStages];
@@ -1388,6 +1387,19 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt, MT>::kCtasPerS
   const int wph = kDecConsumerWarps / hb;  // consumer warps per kv head
   constexpr int kSps = Stage::kSubTiles;
   const int TOK = 16 * wph * kSps;
+
+  const int kDecStages = a.stages;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kDecStages; ++i) {
+      mbar_init(&full_bar[i], kFp8 ? 33 : 1);  // fp8: + one arrival per lane of the copy warp (scale/shift copies)
+      mbar_init(&empty_bar[i], kDecConsumerWarps);
+    }
+    mbar_init(&q_done_bar, kDecConsumerWarps);
+    mbar_fence_init();
+    if (a.copy_mode == 3) prefetch_tensormap(&a.tm_k), prefetch_tensormap(&a.tm_v);
+  }
+  grid_dep_wait();
+  grid_dep_launch();
 
   int kv_len = a.seqlen_k != nullptr ? min(max(a.seqlen_k[b], 0), a.kv_padding) : a.kv_padding;
   // a window is a sequence that starts win_skip keys later: the first key the first query of the sequence sees
@@ -1426,16 +1438,7 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt, MT>::kCtasPerS
   // fill those before every consumer warp has taken its Q fragments
   uint8_t* q_smem = stage_base + a.q_first_stage * stage_bytes;     // 8 warps * 16*MT rows * D*2 B
   constexpr int kQRowBytes = D * 2;
-
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < kDecStages; ++i) {
-      mbar_init(&full_bar[i], kFp8 ? 33 : 1);  // fp8: + one arrival per lane of the copy warp (scale/shift copies)
-      mbar_init(&empty_bar[i], kDecConsumerWarps);
-    }
-    mbar_init(&q_done_bar, kDecConsumerWarps);
-    mbar_fence_init();
-  }
-  __syncthreads();
+  __syncthreads();  // the barriers
 
   if (warp == kDecConsumerWarps) {
     // ------------------------------------------------------------ producer
@@ -1704,6 +1707,8 @@ template <int D>
 __global__ void __launch_bounds__(kMergeWarpsPerCta * 32) decode_merge_kernel(const __grid_constant__ DecodeArgs a) {
   constexpr int V = D / 32;
   __shared__ float red[kMergeWarpsPerCta][D + 4];
+  grid_dep_wait();
+  grid_dep_launch();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int step = kMergeWarpsPerRow;
   const int part = warp % step;
@@ -1828,16 +1833,15 @@ static int launch_decode_t(const DecodeArgs& a_in, int head_blocks, cudaStream_t
     if (dev >= 0) configured[dev] = smem;
   }
   dim3 grid(a.split_k, a.batch, head_blocks * a.row_blocks);
-  kern<<<grid, kDecThreads, smem, stream>>>(a);
-  int rc = check_launch("decode_splitk_kernel");
-  if (rc != XFB200_OK) return rc;
+  cudaError_t e = launch_early(kern, grid, kDecThreads, smem, stream, a);
+  if (e != cudaSuccess) return cuda_fail("decode_splitk_kernel launch", e);
   if (a.split_k > 1) {
     const int64_t rows = int64_t(a.batch) * a.kv_heads * a.rows;
     constexpr int per_cta = kMergeWarpsPerCta / kMergeWarpsPerRow;
-    decode_merge_kernel<D><<<unsigned((rows + per_cta - 1) / per_cta), kMergeWarpsPerCta * 32, 0, stream>>>(a);
-    rc = check_launch("decode_merge_kernel");
+    e = launch_early(decode_merge_kernel<D>, unsigned((rows + per_cta - 1) / per_cta), kMergeWarpsPerCta * 32, 0, stream, a);
+    if (e != cudaSuccess) return cuda_fail("decode_merge_kernel launch", e);
   }
-  return rc;
+  return XFB200_OK;
 }
 
 template <int D, int kFmt, bool kBf16, int NG = 1>

@@ -71,4 +71,20 @@ int prefill_sm100_supported(const xfb200_prefill_params* p);
 int prefill_sm100_launch(const xfb200_prefill_params* p, cudaStream_t stream);
 int prefill_generic_launch(const xfb200_prefill_params* p, cudaStream_t stream);
 
+// Launch that may begin while the kernel ahead of it in the stream still runs.  Only for kernels whose every CTA calls
+// grid_dep_wait() before it touches memory: what is saved is the launch itself and what the kernel does before that call, 1-2 us
+// of a decoding step's 3-6 us kernels.  In a captured stream it becomes an edge of the same kind.
+template <typename... P>
+cudaError_t launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const P&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = stream;
+  cfg.attrs = &attr, cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  if (e != cudaSuccess) cudaGetLastError();  // (returned, not kept)
+  return e;
+}
+
 }  // namespace xfb

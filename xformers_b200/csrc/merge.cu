@@ -12,6 +12,7 @@
 #include <cuda_fp16.h>
 
 #include "internal.h"
+#include "ptx.cuh"
 
 namespace xfb {
 
@@ -58,6 +59,8 @@ constexpr int kMaxSplitsInRegs = 32;
 
 template <typename Tin, typename Tout, int V>
 __global__ void __launch_bounds__(kMergeWarps * 32) merge_kernel(const __grid_constant__ MergeArgs a) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int lane = threadIdx.x & 31;
   const int64_t row = int64_t(blockIdx.x) * kMergeWarps + (threadIdx.x >> 5);
   const int64_t rows = int64_t(a.B) * a.M * a.G * a.H;
@@ -147,11 +150,8 @@ static int launch_merge_v(const MergeArgs& a, int vec, cudaStream_t stream) {
   const int64_t rows = int64_t(a.B) * a.M * a.G * a.H;
   if (rows == 0) return XFB200_OK;
   const unsigned grid = unsigned((rows + kMergeWarps - 1) / kMergeWarps);
-  if (vec == 4)
-    merge_kernel<Tin, Tout, 4><<<grid, kMergeWarps * 32, 0, stream>>>(a);
-  else
-    merge_kernel<Tin, Tout, 1><<<grid, kMergeWarps * 32, 0, stream>>>(a);
-  return check_launch("merge_kernel");
+  const cudaError_t e = launch_early(vec == 4 ? merge_kernel<Tin, Tout, 4> : merge_kernel<Tin, Tout, 1>, grid, kMergeWarps * 32, 0, stream, a);
+  return e != cudaSuccess ? cuda_fail("merge_kernel launch", e) : XFB200_OK;
 }
 
 template <typename Tin>

@@ -268,6 +268,12 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// Launches that may begin before the kernel ahead of them in the stream has ended (launch_early): nothing that kernel wrote may
+// be read, and nothing it reads may be written, before grid_dep_wait(), which returns when it has ended and its writes are visible.
+// grid_dep_launch() lets the next such launch begin once every CTA has got there (or ended).
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

@@ -15,6 +15,7 @@
 #include <algorithm>
 
 #include "internal.h"
+#include "ptx.cuh"
 
 namespace xfb {
 
@@ -131,6 +132,8 @@ template <typename T, bool kF64, bool kVec, bool kAdj, int kQuant = 0>
 __global__ void __launch_bounds__(kRopeThreads, kVec ? 4 : 2) rope_padded_kernel(const __grid_constant__ xfb200_rope_params p, const int tok_per_cta) {
   extern __shared__ float2 cs_table[];
   __shared__ int cache_rows[kRopeMaxTok];  // cache row of each of the CTA's tokens
+  grid_dep_wait();
+  grid_dep_launch();
   // blockIdx.x = group of queries inside the sequence, blockIdx.y = sequence
   const int b = blockIdx.y;
   const int q1 = p.seqstart_q[b + 1];
@@ -374,8 +377,8 @@ int launch_rope(const xfb200_rope_params& p, cudaStream_t st) {
       cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
       if (e != cudaSuccess) return cuda_fail("rope_padded: shared memory", e);
     }
-    kernel<<<grid, kRopeThreads, smem, st>>>(p, tok_per_cta);
-    return check_launch("rope_padded_kernel");
+    const cudaError_t e = launch_early(kernel, grid, kRopeThreads, smem, st, p, tok_per_cta);
+    return e != cudaSuccess ? cuda_fail("rope_padded_kernel launch", e) : XFB200_OK;
   };
   if (p.cache_format == 2) {
     const int per_row = pairs / E;
