@@ -1,4 +1,4 @@
-"""Launches that begin before the kernel ahead of them has ended, and the order in which the prefill kernel takes sequences:
+"""Launches that begin before the kernel ahead of them has ended, and the order and size of the prefill kernel's work items:
 results must be those of calls that are waited for, and of the oracle."""
 
 import pytest
@@ -85,3 +85,19 @@ def test_order_of_sequences(n, heads):
     out, lse = fmha.memory_efficient_attention_forward_requires_grad(q, k, v, bias, op=fmha.b200.FwOp)
     ro, rl = ref(q, k, v, bias)
     assert_o_lse(out, lse, ro, rl, torch.bfloat16, f"{n} sequences")
+
+
+@gpu
+@pytest.mark.parametrize("mask", ["none", "causal", "bottom_right", "window"])
+@pytest.mark.parametrize("m", [1, 128, 129, 2304, 2305])
+@pytest.mark.parametrize("D", [64, 80, 128])
+def test_items_of_one_tile(D, m, mask):
+    """8 heads: up to 2304 rows (144 tiles) a work item is one tile of 128 rows, from 2305 rows on it is two."""
+    require_cuda()
+    keys = {"none": 300, "causal": m, "bottom_right": m + 77, "window": m}[mask]
+    bias = {"none": None, "causal": ab.LowerTriangularMask(), "bottom_right": ab.LowerTriangularFromBottomRightMask(),
+            "window": ab.LowerTriangularFromBottomRightLocalAttentionMask(100) if m > 1 else ab.LowerTriangularMask()}[mask]
+    q, k, v = (t[:, :, 0] for t in rand_qkv(1, m, keys, 1, 8, D, torch.float16, seed=m, gqa=False))
+    out, lse = fmha.memory_efficient_attention_forward_requires_grad(q, k, v, bias, op=fmha.b200.FwOp)
+    ro, rl = ref(q, k, v, bias)
+    assert_o_lse(out, lse, ro, rl, torch.float16, f"{mask} m={m}")

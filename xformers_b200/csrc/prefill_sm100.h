@@ -30,7 +30,8 @@ struct Sm100Args {
   int32_t heads_per_wave;  // persistent kernel: (batch, head) pairs whose row blocks are handed out together (>= 1)
   int32_t out_dtype;
   float scale_log2;
-  int32_t q_tiles;  // blocks of 256 query rows per sequence (static bound)
+  int32_t q_tiles;  // blocks of query rows per sequence (static bound): 256 rows, or item_rows in the persistent kernel
+  int32_t item_rows;  // persistent kernel: query rows of a work item, 256 (two tiles) or 128 (one)
   uint32_t epoch;   // differs from launch to launch, never 0
   int32_t debug_flags;
   long long wait_budget;  // SM clocks after which a wait gives up

@@ -262,9 +262,10 @@ __device__ __forceinline__ bool decode_item(const Sm100Args& a, int order, int i
     it.klen = a.seqlen_k != nullptr ? a.seqlen_k[it.b] : a.seqstart_k[it.b + 1] - it.k_row0;
     it.tb = 0;
   }
-  it.m0 = qt * kBM * kTiles;
+  it.m0 = qt * a.item_rows;
   if (it.m0 >= it.qlen) return false;
   it.shift = (a.bottom_right ? it.klen - it.qlen : 0) - a.kv_offset;
+  it.qlen = min(it.qlen, it.m0 + a.item_rows);  // (an item of one tile has no row of the other)
   it.shift2 = -a.kv_offset2;
   it.n_base = 0;
   if (a.window_left >= 0) it.n_base = max(0, it.m0 + it.shift - a.window_left) / kBN * kBN;
