@@ -298,12 +298,15 @@ __device__ __forceinline__ bool decode_item(const Sm100Args& a, int order, int i
 //   kExact   the head dim is D
 //   kPadded  the head dim a.head_dim is smaller than D; the copies fill the columns behind it with zeros, the products
 //            leave out what lies wholly behind it, the output is written up to it
-//   kBiased  an additive bias; the head dim may be D or smaller
-constexpr int kExact = 0, kPadded = 1, kBiased = 2;
+//   kBiased  an additive bias of any type; the head dim may be D or smaller
+//   kBiasedSame  the same for a bias of the type of q, which the step then knows at compile time (with the type asked for at
+//                every pair of scores, a step of 128 keys took 6000 clocks, without a bias 2100: 2 x 2048 x 2048, 8 heads,
+//                bf16: 96 -> 82 us)
+constexpr int kExact = 0, kPadded = 1, kBiased = 2, kBiasedSame = 3;
 template <int D, bool kBf16, int kVariant>
 __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(const __grid_constant__ Sm100Args a) {
   using L = Smem<D>;
-  constexpr bool kPad = kVariant != kExact, kBias = kVariant == kBiased;
+  constexpr bool kPad = kVariant != kExact, kBias = kVariant == kBiased || kVariant == kBiasedSame, kBiasSame = kVariant == kBiasedSame;
   constexpr int kHalves = D / 64;
   extern __shared__ uint8_t smem_dyn[];
   uint8_t* smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);  // an offset, so that the compiler keeps seeing shared memory
@@ -900,12 +903,15 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
       // scores, and reading memory that way costs one sector request per element (2048 x 2048 x 16 heads, bf16: 600 us).
       // A warp therefore reads its 32 rows in units of 64 bytes per row, four lanes to a row and 16 bytes to a lane, holds
       // the units of a step in registers from before the wait for the scores on, and turns one after the other into
-      // rows through 2 KB of shared memory (16-byte chunks XOR-ed with row / 2, no bank conflict either way): 99 us for the
+      // rows through 2 KB of shared memory (16-byte chunks XOR-ed with row / 2, no bank conflict either way): 82 us for the
       // same call (34 GFLOP, 134 MB of bias).  A unit is
       // 32 columns of a 16-bit bias (four units: a step) or 16 of an f32 one (four: half a step).
+      const bool bias_f32 = !kBiasSame && a.bias_dtype == XFB200_F32;
+      const bool bias_bf16 = kBiasSame ? kBf16 : a.bias_dtype == XFB200_BF16;
+      const uint64_t inv2 = f2_pack(a.inv_scale, a.inv_scale);
       uint8_t* const bias_smem = smem + L::kBias + warp * L::kBiasUnit;
       auto bias_load = [&](uint4* w, int64_t off, int mt0, int qlen, int col_first, int n_keys) {
-        const int esz = a.bias_dtype == XFB200_F32 ? 4 : 2, per16 = 16 / esz;
+        const int esz = bias_f32 ? 4 : 2, per16 = 16 / esz;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int r = mt0 + (warp & 3) * 32 + i * 8 + (lane >> 2);
@@ -934,7 +940,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
         }
       };
       auto bias_prefetch = [&](int64_t off, int mt0, int qlen, int col_first, int n_keys) {
-        const int esz = a.bias_dtype == XFB200_F32 ? 4 : 2;
+        const int esz = bias_f32 ? 4 : 2;
         const int r = mt0 + row;
         const uint8_t* src = reinterpret_cast<const uint8_t*>(a.bias) + (off + int64_t(r) * a.bias_m) * esz;
         for (int col = col_first; col < col_first + kBN; col += 128 / esz)
@@ -953,7 +959,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           __syncwarp();
         };
         auto add = [&](int c, float x) { sc[c] = __float_as_uint(fmaf(x, a.inv_scale, __uint_as_float(sc[c]))); };
-        if (a.bias_dtype == XFB200_F32) {
+        if (bias_f32) {
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             uint4 mine[4];
@@ -970,9 +976,10 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
         to_rows(chunk, mine);
         auto add2 = [&](int c, uint32_t x) {
           float lo, hi;
-          if (a.bias_dtype == XFB200_BF16) unpack_pair<true>(x, lo, hi);
+          if (bias_bf16) unpack_pair<true>(x, lo, hi);
           else unpack_pair<false>(x, lo, hi);
-          add(c, lo), add(c + 1, hi);
+          f2_unpack(ffma2(f2_pack(lo, hi), inv2, f2_pack(__uint_as_float(sc[c]), __uint_as_float(sc[c + 1]))), lo, hi);
+          sc[c] = __float_as_uint(lo), sc[c + 1] = __float_as_uint(hi);
         };
 #pragma unroll
         for (int k = 0; k < 4; ++k)
@@ -1080,7 +1087,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
               XFB_TMEM_ST_32(tmem_s, sa);
               bias_add(sb, bw, 1);
               XFB_TMEM_ST_32(tmem_s + 32, sb);
-              if (a.bias_dtype == XFB200_F32) bias_load(bw, it.bias_off, mt0, it.qlen, n0 + 64, klen);
+              if (bias_f32) bias_load(bw, it.bias_off, mt0, it.qlen, n0 + 64, klen);
             }
             float mx = fmaxf(chunk_max(reinterpret_cast<float*>(sa)), chunk_max(reinterpret_cast<float*>(sb)));
             if constexpr (kBias) tc_wait_st();
@@ -1172,7 +1179,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
 template <int D, bool kBf16, int kVariant>
 static int launch_t(const Sm100Args& a, cudaStream_t stream) {
   auto kern = prefill_sm100_persist_kernel<D, kBf16, kVariant>;
-  constexpr int smem = kVariant == kBiased ? Smem<D>::kTotalBiased : Smem<D>::kTotal;
+  constexpr int smem = kVariant == kBiased || kVariant == kBiasedSame ? Smem<D>::kTotalBiased : Smem<D>::kTotal;
   static_assert(smem <= 227 * 1024, "shared memory of one CTA");
   static bool configured[kMaxDevices] = {false};  // the attribute belongs to the device's context
   if (first_use_on_device(configured)) {
@@ -1208,6 +1215,8 @@ static int persist_launch_d(const Sm100Args& a, bool bf16, cudaStream_t stream) 
 }
 
 int prefill_sm100_persist_launch(Sm100Args a, int head_dim, bool bf16, cudaStream_t stream) {
+  if (a.bias != nullptr && a.bias_dtype == (bf16 ? XFB200_BF16 : XFB200_F16))
+    return head_dim > 64 ? persist_launch_d<128, pst::kBiasedSame>(a, bf16, stream) : persist_launch_d<64, pst::kBiasedSame>(a, bf16, stream);
   if (a.bias != nullptr) return head_dim > 64 ? persist_launch_d<128, pst::kBiased>(a, bf16, stream) : persist_launch_d<64, pst::kBiased>(a, bf16, stream);
   if (head_dim == 128) return persist_launch_d<128, pst::kExact>(a, bf16, stream);
   if (head_dim == 64) return persist_launch_d<64, pst::kExact>(a, bf16, stream);
