@@ -101,3 +101,59 @@ def test_items_of_one_tile(D, m, mask):
     out, lse = fmha.memory_efficient_attention_forward_requires_grad(q, k, v, bias, op=fmha.b200.FwOp)
     ro, rl = ref(q, k, v, bias)
     assert_o_lse(out, lse, ro, rl, torch.float16, f"{mask} m={m}")
+
+
+@gpu
+@pytest.mark.parametrize("m,heads", [(200, 4), (2500, 16)])
+def test_prefills_back_to_back(m, heads):
+    """Prefill calls that read the output of the one before, on launches smaller and larger than the machine."""
+    require_cuda()
+    q0, k, v = (t[:, :, 0] for t in rand_qkv(1, m, m, 1, heads, 128, torch.bfloat16, seed=3, gqa=False))
+
+    def run(wait):
+        q, outs = q0, []
+        for _ in range(8):
+            q = fmha.memory_efficient_attention_forward(q, k, v, ab.LowerTriangularMask(), op=fmha.b200.FwOp)
+            q = fmha.memory_efficient_attention_forward(q, q, v, None, op=fmha.b200.FwOp) * 3
+            if wait:
+                torch.cuda.synchronize()
+            outs.append(q)
+        return outs
+
+    for a, b in zip(run(False), run(True)):
+        assert torch.equal(a, b)
+
+
+@gpu
+def test_capture_behind_copies_and_joined_streams():
+    """Captured launches whose predecessor is a copy, and whose stream has just joined another one."""
+    require_cuda()
+    q, k, v = (t[:, :, 0] for t in rand_qkv(1, 300, 300, 1, 4, 128, torch.bfloat16, seed=5, gqa=False))
+    qg, kg, vg = rand_qkv(2, 1, 3000, 2, 8, 128, torch.bfloat16, seed=6)
+    x, y = torch.zeros_like(q), torch.zeros_like(qg)
+
+    def work(side):
+        main = torch.cuda.current_stream()
+        x.copy_(q)
+        a = fmha.memory_efficient_attention_forward(x, k, v, ab.LowerTriangularMask(), op=fmha.b200.FwOp)
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            y.copy_(qg)
+            b, lse = fmha.memory_efficient_attention_partial(y, kg, vg, op=fmha.b200_splitk.FwOp)
+        c = fmha.memory_efficient_attention_forward(a, k, v, None, op=fmha.b200.FwOp)
+        main.wait_stream(side)
+        d, _ = fmha.memory_efficient_attention_partial(b, kg, vg, op=fmha.b200_splitk.FwOp)
+        m, _ = fmha.merge_attentions([b, d], [lse, lse])
+        return c, m
+
+    side = torch.cuda.Stream()
+    want = [t.clone() for t in work(side)]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = work(side)
+    for _ in range(5):
+        x.zero_(), y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
