@@ -44,3 +44,18 @@ def test_small_pages(kv_heads, group, page, split_k, quant):
     assert_o_lse(out, lse, ro, rl, dtype, f"pages of {page}")
     out_pad, lse_pad = run(k_pad, v_pad, pad_bias)
     assert torch.equal(out, out_pad) and torch.equal(lse, lse_pad), "page placement must not change a single bit"
+
+
+@gpu
+def test_nan_behind_a_vanishing_weight():
+    """A NaN in V makes the output NaN whatever the weight of its chunk, also one that underflows to zero in the merge."""
+    require_cuda()
+    q = torch.ones(1, 1, 1, 8, 128, device="cuda", dtype=torch.bfloat16)
+    k = torch.zeros(1, 512, 1, 1, 128, device="cuda", dtype=torch.bfloat16)
+    k[:, 300] = 40.0  # a score of 450; the keys of the other chunks weigh exp(-450)
+    v = torch.ones(1, 512, 1, 1, 128, device="cuda", dtype=torch.bfloat16)
+    v[0, 5, 0, 0, 7] = float("nan")
+    bias = ab.BlockDiagonalPaddedKeysMask.from_seqlens([1], 512, [512], device="cuda")
+    op = type("Op", (S.FwOp,), {"SPLIT_K": 4})
+    out = fmha.memory_efficient_attention_forward(q, k.expand(-1, -1, -1, 8, -1), v.expand(-1, -1, -1, 8, -1), bias, op=op)
+    assert out[..., 7].isnan().all() and (out[..., :7] == 1).all() and (out[..., 8:] == 1).all()

@@ -1757,7 +1757,7 @@ __global__ void __launch_bounds__(kMergeWarpsPerCta * 32) decode_merge_kernel(co
         const float w = l[u] > -INFINITY ? __expf(l[u] - mx) : 0.f;
         den += w;
 #pragma unroll
-        for (int i = 0; i < V; ++i) acc[i] += w > 0.f ? w * x[u][i] : 0.f;
+        for (int i = 0; i < V; ++i) acc[i] += l[u] > -INFINITY ? w * x[u][i] : 0.f;  // (0 x NaN stays NaN)
       }
     }
   }
