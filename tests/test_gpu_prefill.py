@@ -590,3 +590,27 @@ def test_additive_bias_units_of_the_tcgen05_kernel(Mkv, wide, D, bias_dtype, cau
     ro, rl = oracle.ref_attention_with_lse(q.float().cpu(), k.float().cpu(), v.float().cpu(), add)
     assert_o_lse(out, lse, ro, rl, dtype, f"bias {bias_dtype} of {Mkv} columns")
     _status_ok()
+
+
+@gpu
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("bias_dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("D", [40, 64, 80, 128, 160])
+@pytest.mark.parametrize("wide", [304, 301])
+def test_bias_entries_of_hidden_keys_are_not_used(wide, D, bias_dtype, value):
+    """Above the diagonal the bias may hold anything (a buffer of which only the lower triangle was filled): rows on 16-byte
+    boundaries and rows that are not, diagonal tiles of several key steps, both prefill kernels."""
+    require_cuda()
+    B, M, H, dtype = 2, 300, 3, torch.bfloat16
+    g = torch.Generator().manual_seed(D)
+    q, k, v = (torch.randn(B, M, H, D, generator=g).to(dtype).cuda() for _ in range(3))
+    t = torch.randn(B, H, M, M, generator=g).to(bias_dtype)
+    hidden = torch.ones(M, M, dtype=torch.bool).triu(1)
+    buf = torch.full((B, H, M, wide), value, dtype=bias_dtype)
+    buf[..., :M] = t.masked_fill(hidden, value)
+    bias = ab.LowerTriangularMaskWithTensorBias(buf.cuda()[..., :M])
+    out, lse = fmha.memory_efficient_attention_forward_requires_grad(q, k, v, bias, op=P.FwOp)
+    add = t.float().masked_fill(hidden, float("-inf"))
+    ro, rl = oracle.ref_attention_with_lse(q.float().cpu(), k.float().cpu(), v.float().cpu(), add)
+    assert_o_lse(out, lse, ro, rl, dtype, f"hidden bias entries of {value}")
+    _status_ok()

@@ -914,28 +914,33 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
       const bool bias_bf16 = kBiasSame ? kBf16 : a.bias_dtype == XFB200_BF16;
       const uint64_t inv2 = f2_pack(a.inv_scale, a.inv_scale);
       uint8_t* const bias_smem = smem + L::kBias + warp * L::kBiasUnit;
-      auto bias_load = [&](uint4* w, int64_t off, int mt0, int qlen, int col_first, int n_keys) {
+      // Row r reads its visible keys only, [r + rel_lo, min(r + rel_hi, n_keys)), and has 0 for the others: their scores are -inf
+      // already, and what the bias holds there, a NaN perhaps, must not meet that.  (Masking behind the addition instead costs the
+      // step registers: 75.5 -> 86.7 us for 2 x 2048 x 2048, 8 heads, no mask at all.)
+      auto bias_load = [&](uint4* w, int64_t off, int mt0, int qlen, int col_first, int n_keys, int rel_lo, int rel_hi) {
         const int esz = bias_f32 ? 4 : 2, per16 = 16 / esz;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int r = mt0 + (warp & 3) * 32 + i * 8 + (lane >> 2);
+          const int lo = r + rel_lo, hi = min(r + rel_hi, n_keys);
           const uint8_t* src = reinterpret_cast<const uint8_t*>(a.bias) + (off + int64_t(r) * a.bias_m) * esz;
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             const int col = col_first + (u * 4 + (lane & 3)) * per16;
             uint4 x = make_uint4(0, 0, 0, 0);
-            if (r < qlen && col < n_keys) {
-              if (a.bias_vec && col + per16 <= n_keys) {
+            if (r < qlen && col < hi) {
+              auto seen = [&](int k) { return col + k < hi && col + k >= lo; };
+              if (a.bias_vec && col + per16 <= hi && col >= lo) {
                 x = __ldg(reinterpret_cast<const uint4*>(src + col * esz));
               } else if (esz == 4) {
                 const uint32_t* e = reinterpret_cast<const uint32_t*>(src) + col;
-                x.x = e[0];
-                if (col + 1 < n_keys) x.y = e[1];
-                if (col + 2 < n_keys) x.z = e[2];
-                if (col + 3 < n_keys) x.w = e[3];
+                if (seen(0)) x.x = e[0];
+                if (seen(1)) x.y = e[1];
+                if (seen(2)) x.z = e[2];
+                if (seen(3)) x.w = e[3];
               } else {
                 const uint16_t* e = reinterpret_cast<const uint16_t*>(src) + col;
-                auto el = [&](int k) -> uint32_t { return col + k < n_keys ? e[k] : 0; };
+                auto el = [&](int k) -> uint32_t { return seen(k) ? e[k] : 0; };
                 x = make_uint4(el(0) | el(1) << 16, el(2) | el(3) << 16, el(4) | el(5) << 16, el(6) | el(7) << 16);
               }
             }
@@ -1034,10 +1039,13 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           const bool need_mask = (n0 + kBN > klen) || (causal && n0 + kBN - 1 > mt0 + shift + a.window_right) ||
                                  (a.window_left >= 0 && n0 < mt0 + kBM - 1 + shift - a.window_left);
           uint4 bw[kBias ? 16 : 1];
+          int rel_lo = 0, rel_hi = 0;  // visible keys of row r: from r + rel_lo, below r + rel_hi
           if constexpr (kBias) {
             // asked for before the wait for the scores, which hides most of their latency; the next step's are asked
             // into the L2 at the same time
-            bias_load(bw, it.bias_off, mt0, it.qlen, n0, klen);
+            rel_lo = a.window_left >= 0 ? shift - a.window_left : -0x3fffffff;
+            rel_hi = causal ? shift + a.window_right + 1 : 0x3fffffff;
+            bias_load(bw, it.bias_off, mt0, it.qlen, n0, klen, rel_lo, rel_hi);
             bias_prefetch(it.bias_off, mt0, it.qlen, n0 + kBN, j + 1 < jhi ? klen : 0);
           }
           ok = mbar_wait(&bar->s_full[t], cnt & 1, abort_flag, budget);
@@ -1091,7 +1099,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
               XFB_TMEM_ST_32(tmem_s, sa);
               bias_add(sb, bw, 1);
               XFB_TMEM_ST_32(tmem_s + 32, sb);
-              if (bias_f32) bias_load(bw, it.bias_off, mt0, it.qlen, n0 + 64, klen);
+              if (bias_f32) bias_load(bw, it.bias_off, mt0, it.qlen, n0 + 64, klen, rel_lo, rel_hi);
             }
             float mx = fmaxf(chunk_max(reinterpret_cast<float*>(sa)), chunk_max(reinterpret_cast<float*>(sb)));
             if constexpr (kBias) tc_wait_st();
