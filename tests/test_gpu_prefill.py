@@ -614,3 +614,37 @@ def test_bias_entries_of_hidden_keys_are_not_used(wide, D, bias_dtype, value):
     ro, rl = oracle.ref_attention_with_lse(q.float().cpu(), k.float().cpu(), v.float().cpu(), add)
     assert_o_lse(out, lse, ro, rl, dtype, f"hidden bias entries of {value}")
     _status_ok()
+
+
+@gpu
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("low", [-1e9, -3e37, -2e38, float("-inf")])
+@pytest.mark.parametrize("bias_dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("D", [40, 64, 80, 128, 160])
+def test_rows_of_one_large_bias(D, bias_dtype, low, causal):
+    """Rows whose every entry is the same large negative number (a query that is padding): the scores drown in it, the result is
+    the mean over the visible keys.  Rows of -inf are zeros."""
+    require_cuda()
+    B, M, H, dtype = 1, 200, 2, torch.float16 if D in (64, 80) else torch.bfloat16
+    g = torch.Generator().manual_seed(D)
+    q, k, v = (torch.randn(B, M, H, D, generator=g).to(dtype).cuda() for _ in range(3))
+    t = torch.randn(B, H, M, M, generator=g).to(bias_dtype)
+    rows = [3, 127, 128, 199]
+    t[:, :, rows] = low
+    bias = ab.LowerTriangularMaskWithTensorBias(t.cuda()) if causal else t.cuda()
+    out, lse = fmha.memory_efficient_attention_forward_requires_grad(q, k, v, bias, op=P.FwOp)
+    assert out.isfinite().all()
+    for r in rows:
+        n = r + 1 if causal else M
+        mean = v[:, :n].float().mean(1) * (low > float("-inf"))
+        assert (out[:, r].float() - mean).abs().max() <= ATOL_O[dtype]
+        want = float(torch.tensor(low).to(bias_dtype))
+        if want > float("-inf"):  # (log n is lost in it too; two roundings of f32)
+            assert ((lse[:, :, r].double() - want).abs() <= 2.0**-22 * abs(want)).all()
+        else:
+            assert torch.isneginf(lse[:, :, r]).all()
+    keep = [r for r in range(M) if r not in rows]
+    add = t.float().masked_fill(torch.ones(M, M, dtype=torch.bool).triu(1) & causal, float("-inf"))
+    ro, rl = oracle.ref_attention_with_lse(q.float().cpu(), k.float().cpu(), v.float().cpu(), add)
+    assert_o_lse(out[:, keep], lse[:, :, keep], ro[:, keep], rl[:, :, keep], dtype, f"rows beside rows of {low}")
+    _status_ok()

@@ -36,11 +36,10 @@ struct Sm100Args {
   int32_t debug_flags;
   long long wait_budget;  // SM clocks after which a wait gives up
   // additive bias (persistent kernel, dense batches): element strides of [batch, G, H, mq, mkv], unit stride on mkv;
-  // the kernel adds bias / scale to q k^T, so that the softmax sees q k^T * scale + bias
+  // the softmax sees (q k^T * scale + bias) * log2 e
   const void* bias;
   int32_t bias_dtype;
   int32_t bias_vec;  // every row of the bias starts on a 16-byte boundary
-  float inv_scale;
   int64_t bias_b, bias_g, bias_h, bias_m;
 };
 

@@ -125,7 +125,7 @@ int prefill_sm100_launch(const xfb200_prefill_params* p, cudaStream_t stream) {
   }
   a.debug_flags = p->debug_flags;
   a.wait_budget = p->wait_budget_kcycles > 0 ? 1000LL * p->wait_budget_kcycles : kDefaultWaitBudgetCycles;
-  a.bias = p->bias, a.bias_dtype = p->bias_dtype, a.inv_scale = 1.f / p->scale;
+  a.bias = p->bias, a.bias_dtype = p->bias_dtype;
   a.bias_b = p->bias_stride_b, a.bias_g = p->bias_stride_g, a.bias_h = p->bias_stride_h, a.bias_m = p->bias_stride_m;
   {
     const int64_t per16 = p->bias_dtype == XFB200_F32 ? 4 : 8;

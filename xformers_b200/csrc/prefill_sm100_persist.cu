@@ -49,8 +49,7 @@
 // the step has no loop and no per-chunk test.  On diagonal and ragged tiles a
 // small loop first writes -inf over the hidden scores in tensor memory; the step
 // itself is one piece of code for every tile, which the instruction cache likes.
-// An additive bias is added in the first pass (bias / scale; a kernel variant of its
-// own).  When the first half of P (keys 64-127) is stored the softmax
+// An additive bias is added in the first pass (kernel variants of their own).  When the first half of P (keys 64-127) is stored the softmax
 // arrives on a barrier of its own and the MMA warp issues that half of PV while
 // the other half is still being computed.  Measured
 // alternatives on the causal 4k case: one pass with a stale reference, a vote per
@@ -835,7 +834,10 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
       const uint32_t lane_sel = uint32_t((warp & 3) * 32) << 16;
       const uint32_t tmem_s = tmem + t * 128 + lane_sel;
       const uint32_t tmem_o = tmem + 256 + t * 128 + lane_sel;
-      const float sl2 = a.scale_log2;
+      // what brings the scores to log2 units; with an additive bias they are brought there before it is added, since the bias itself
+      // times 1 / scale would overflow where the bias does not, and a large score would lose against its own maximum what the
+      // product rounds
+      const float sl2 = kBias ? 1.f : a.scale_log2;
       const uint64_t sc2 = f2_pack(sl2, sl2);
       int seq = 0;
       int cnt = 0;  // steps of this tile so far, over all items
@@ -872,7 +874,10 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           float e[16];
 #pragma unroll
           for (int i = 0; i < 16; i += 2)
-            f2_unpack(ffma2(f2_pack(__uint_as_float(sr[h + i]), __uint_as_float(sr[h + i + 1])), sc2, nm2), e[i], e[i + 1]);
+            if constexpr (kBias)
+              f2_unpack(fadd2(f2_pack(__uint_as_float(sr[h + i]), __uint_as_float(sr[h + i + 1])), nm2), e[i], e[i + 1]);
+            else
+              f2_unpack(ffma2(f2_pack(__uint_as_float(sr[h + i]), __uint_as_float(sr[h + i + 1])), sc2, nm2), e[i], e[i + 1]);
 #pragma unroll
           for (int i = 0; i < 16; ++i) e[i] = fast_exp2(e[i]);
 #pragma unroll
@@ -912,7 +917,8 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
       // 32 columns of a 16-bit bias (four units: a step) or 16 of an f32 one (four: half a step).
       const bool bias_f32 = !kBiasSame && a.bias_dtype == XFB200_F32;
       const bool bias_bf16 = kBiasSame ? kBf16 : a.bias_dtype == XFB200_BF16;
-      const uint64_t inv2 = f2_pack(a.inv_scale, a.inv_scale);
+      constexpr float kLog2e = 1.4426950408889634f;
+      const uint64_t scale2 = f2_pack(a.scale_log2, a.scale_log2), log2e2 = f2_pack(kLog2e, kLog2e);
       uint8_t* const bias_smem = smem + L::kBias + warp * L::kBiasUnit;
       // Row r reads its visible keys only, [r + rel_lo, min(r + rel_hi, n_keys)), and has 0 for the others: their scores are -inf
       // already, and what the bias holds there, a NaN perhaps, must not meet that.  (Masking behind the addition instead costs the
@@ -955,8 +961,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
         for (int col = col_first; col < col_first + kBN; col += 128 / esz)
           if (r < qlen && col < n_keys) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + int64_t(col) * esz));
       };
-      // the scores of columns [32 chunk, 32 chunk + 32) of this thread's row += bias / scale (so that the step's scale *
-      // log2 e applies to the sum)
+      // the scores of columns [32 chunk, 32 chunk + 32) of this thread's row become (score * scale + bias) * log2 e
       auto bias_add = [&](uint32_t* sc, const uint4* w, int chunk) {
         auto to_rows = [&](int u, uint4 (&mine)[4]) {
 #pragma unroll
@@ -967,7 +972,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           for (int k = 0; k < 4; ++k) mine[k] = *reinterpret_cast<const uint4*>(bias_smem + lane * 64 + ((k ^ ((lane >> 1) & 3)) << 4));
           __syncwarp();
         };
-        auto add = [&](int c, float x) { sc[c] = __float_as_uint(fmaf(x, a.inv_scale, __uint_as_float(sc[c]))); };
+        auto add = [&](int c, float x) { sc[c] = __float_as_uint(fmaf(__uint_as_float(sc[c]), a.scale_log2, x * kLog2e)); };
         if (bias_f32) {
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
@@ -987,7 +992,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           float lo, hi;
           if (bias_bf16) unpack_pair<true>(x, lo, hi);
           else unpack_pair<false>(x, lo, hi);
-          f2_unpack(ffma2(f2_pack(lo, hi), inv2, f2_pack(__uint_as_float(sc[c]), __uint_as_float(sc[c + 1]))), lo, hi);
+          f2_unpack(ffma2(f2_pack(__uint_as_float(sc[c]), __uint_as_float(sc[c + 1])), scale2, fmul2(f2_pack(lo, hi), log2e2)), lo, hi);
           sc[c] = __float_as_uint(lo), sc[c + 1] = __float_as_uint(hi);
         };
 #pragma unroll
