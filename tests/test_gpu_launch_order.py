@@ -1,6 +1,8 @@
 """Launches that begin before the kernel ahead of them has ended, and the order and size of the prefill kernel's work items:
 results must be those of calls that are waited for, and of the oracle."""
 
+import time
+
 import pytest
 import torch
 
@@ -157,3 +159,28 @@ def test_capture_behind_copies_and_joined_streams():
         graph.replay()
         torch.cuda.synchronize()
         assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@gpu
+def test_free_sms_stay_free_between_two_launches():
+    """Two launches that leave SMs free, one behind the other: a kernel of another stream runs beside the first of them, it does
+    not wait for its end (as it does where the second one's CTAs already sit on those SMs)."""
+    require_cuda()
+    q, k, v = (t[:, :, 0] for t in rand_qkv(1, 16384, 16384, 1, 32, 128, torch.bfloat16, seed=8, gqa=False))
+    inp = fmha.Inputs(q, k, v, None)
+    x, side = torch.zeros(1024, device="cuda"), torch.cuda.Stream()
+    shares = []
+    for _ in range(4):  # (the first loads the kernels)
+        start, small, end = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+        torch.cuda.synchronize()
+        start.record()
+        for _ in range(2):
+            fmha.b200.FwOp._apply(inp, False, sm_margin=8)  # 3.5 ms each
+        end.record()
+        time.sleep(0.0005)  # both are with the GPU now
+        with torch.cuda.stream(side):
+            x.add_(1)
+            small.record()
+        torch.cuda.synchronize()
+        shares.append(start.elapsed_time(small) / start.elapsed_time(end))
+    assert min(shares[1:]) < 0.3, f"the other stream's kernel ended after {shares} of both launches"

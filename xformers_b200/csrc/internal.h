@@ -74,6 +74,8 @@ int prefill_generic_launch(const xfb200_prefill_params* p, cudaStream_t stream);
 // Launch that may begin while the kernel ahead of it in the stream still runs.  Only for kernels whose every CTA calls
 // grid_dep_wait() before it touches memory: what is saved is the launch itself and what the kernel does before that call, 1-2 us
 // of a decoding step's 3-6 us kernels.  In a captured stream it becomes an edge of the same kind.
+//   A kernel that leaves SMs free for other streams (sm_margin) neither is launched this way nor lets the next one begin: CTAs that
+// only wait would fill those SMs.
 template <typename... P>
 cudaError_t launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const P&... args) {
   cudaLaunchAttribute attr{};

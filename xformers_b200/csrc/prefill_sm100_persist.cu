@@ -359,7 +359,9 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
     // (barriers, tensor memory and its allocation do not wait for the kernel ahead in the stream; everything below does)
     grid_dep_wait();
     // (not with a bias: 128 items of one launch and the next one's on the SMs beside them, 82.5 -> 83.6 us for 2 x 2048 x 2048)
-    if constexpr (!kBias) grid_dep_launch();
+    // (nor where SMs are to stay free for another stream's kernels: the CTAs of the next launch would take these and wait there)
+    if constexpr (!kBias)
+      if (a.sm_margin == 0) grid_dep_launch();
 
     // Next announced item (every announced item has key steps): its number, -1 after the last one, -2 when the
     // wait ran out.  `take` copies what the caller needs out of the descriptor before the slot is handed back.
@@ -1208,6 +1210,10 @@ static int launch_t(const Sm100Args& a, cudaStream_t stream) {
   int sms = sm_count() - a.sm_margin;
   if (sms < 1) sms = 1;
   const unsigned grid = unsigned(items < sms ? items : sms);
+  if (a.sm_margin > 0) {  // the free SMs are for others from its first CTA to its last
+    kern<<<grid, kThreads, smem, stream>>>(a);
+    return check_launch("prefill_sm100_persist_kernel");
+  }
   const cudaError_t e = launch_early(kern, grid, kThreads, smem, stream, a);
   return e != cudaSuccess ? cuda_fail("prefill_sm100_persist_kernel launch", e) : XFB200_OK;
 }
