@@ -166,3 +166,26 @@ def test_front_leaves_the_unusual_to_python(monkeypatch):
     _both(monkeypatch, run(q, k, v), takes=True)
     with pytest.raises(ValueError):  # the Python path's message, not a crash
         xops.memory_efficient_attention_forward(q, k[:, :, :2], v, None)
+
+
+@gpu
+@pytest.mark.parametrize("op", [None, "named"])
+def test_front_leaves_changed_operators_to_python(op, monkeypatch):
+    """What a program sets on the operator classes themselves counts: settings and methods."""
+    require_cuda()
+    gen = torch.Generator().manual_seed(7)
+    decode, prefill = fmha.b200_splitk.FwOp, fmha.b200.FwOp
+    qd = _mk(gen, 1, 1, 2, 4, 128)
+    kd, vd = (_mk(gen, 1, 4096, 2, 1, 128).expand(-1, -1, -1, 4, -1) for _ in range(2))
+    q, k, v = (_mk(gen, 1, 33, 4, 64) for _ in range(3))
+    step = lambda: xops.memory_efficient_attention_forward(qd, kd, vd, None, op=op and decode)
+    prompt = lambda: xops.memory_efficient_attention_forward(q, k, v, ab.LowerTriangularMask(), op=op and prefill)
+    splits, paths = [], []
+    for call, cls, name, value in ((step, decode, "SPLIT_K", 3), (step, decode, "get_split_k", classmethod(lambda c, *a, **kw: splits.append(a) or 2)),
+                                   (prompt, prefill, "KERNEL_PATH", _lib.PREFILL_MMA_SYNC), (prompt, prefill, "_WAIT_BUDGET_KCYCLES", 100000),
+                                   (prompt, prefill, "apply", classmethod(lambda c, inp, needs_gradient: paths.append(1) or (torch.zeros_like(inp.query), None)))):
+        with monkeypatch.context() as m:
+            m.setattr(cls, name, value)
+            _both(m, call, takes=False)
+        _both(monkeypatch, call, takes=True)
+    assert splits and len(paths) == 2

@@ -59,6 +59,17 @@ _OPS = {
     (b200.FwOp, None): _FORCE_PREFILL,
 }
 _Tensor = torch.Tensor
+_DECODE_CLS, _PREFILL_CLS = b200_splitk.FwOp.__dict__, b200.FwOp.__dict__  # (views: they follow the classes)
+_SPLIT, _DECODE_APPLY, _DECODE_REASONS = (_DECODE_CLS[n] for n in ("get_split_k", "apply", "not_supported_reasons"))
+_PREFILL_APPLY, _PREFILL_REASONS = (_PREFILL_CLS[n] for n in ("apply", "not_supported_reasons"))
+
+
+def _as_shipped() -> bool:
+    """The front knows the operators as they are; settings and methods replaced on the classes themselves are the Python path's."""
+    d, p = _DECODE_CLS, _PREFILL_CLS
+    return (d["SPLIT_K"] is None and d["NUM_GROUPS"] == 1 and d["get_split_k"] is _SPLIT and d["apply"] is _DECODE_APPLY
+            and d["not_supported_reasons"] is _DECODE_REASONS and p["KERNEL_PATH"] == _lib.PREFILL_AUTO and not p["_WAIT_BUDGET_KCYCLES"]
+            and not p["_DEBUG_FLAGS"] and p["apply"] is _PREFILL_APPLY and p["not_supported_reasons"] is _PREFILL_REASONS)
 
 
 def forward(q, k, v, bias: Any, p: float, scale: Optional[float], op: Any, output_dtype: Optional[torch.dtype], flags: int,
@@ -67,6 +78,8 @@ def forward(q, k, v, bias: Any, p: float, scale: Optional[float], op: Any, outpu
     front, spec, force = _lib.front, _BIASES.get(type(bias)), _OPS.get(op)
     # (a tensor subclass -- a parameter, a fake tensor -- goes the long way)
     if front is None or spec is None or force is None or p != 0.0 or type(q) is not _Tensor or type(k) is not _Tensor or type(v) is not _Tensor:
+        return None
+    if not _as_shipped():
         return None
     family, takes, mask, window = spec
     flags |= takes | force
