@@ -248,3 +248,12 @@ def test_split_k_heuristic_is_static():
     assert 16 <= s <= 256 and f(64, 32768, 8, 256) == s
     assert f(1, 128, 1, 256) == 1
     assert fmha.b200_splitk.FwOp_S8.get_split_k(64, 32768, 8, 256) == 8
+
+
+@pytest.mark.parametrize("quantised", [False, True])
+@pytest.mark.parametrize("rows", [1, 8, 9, 16, 17, 64])
+def test_split_k_stays_in_range_for_long_contexts(rows, quantised):
+    """The library takes 1024 chunks at most; chunks of 1280 keys are the longest, so 1310720 keys are what that covers."""
+    f = fmha.b200_splitk.FwOp.get_split_k
+    for bound in list(range(200_000, 1_310_720, 7_001)) + [611_461, 618_789, 619_807, 1_310_720]:
+        assert 1 <= f(1, bound, 8, 256, rows, quantised) <= 1024

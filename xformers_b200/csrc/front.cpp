@@ -179,10 +179,11 @@ int64_t split_k(int64_t batch, int64_t kv_bound, int64_t kv_heads, int64_t rows,
   if (batch * (kv_heads / hb0) * chunks(std::min<int64_t>(bound, 1280)) >= 4 * kSms) return chunks(std::min<int64_t>(bound, 1280));
   const bool two = quantised && rows <= 8;  // CTAs per SM, as the library picks it
   const int64_t tile_rows = quantised ? 8 : 16, row_blocks = (rows + 2 * tile_rows - 1) / (2 * tile_rows), slots = two ? 2 * kSms : kSms;
-  int64_t best = 128;
+  int64_t best = std::min<int64_t>(bound, 1280);
   double best_us = 1e30;
   for (int64_t c = 128; c <= std::min<int64_t>(bound, 1280); c += 128) {
     const int64_t n = chunks(c);
+    if (n > 1024) continue;  // (more than the library takes)
     int64_t hb = hb0;  // as the library picks it
     if (!quantised)
       while (hb > 1 && batch * (kv_heads / hb) * row_blocks * n * 2 <= kSms) hb /= 2;
