@@ -235,6 +235,11 @@ typedef struct {
 
 XFB200_API size_t xfb200_decode_scratch_bytes(int32_t batch, int32_t mq, int32_t kv_heads, int32_t q_per_kv, int32_t head_dim,
                                    int32_t split_k);
+/* The number of chunks a launch should have (1..1024), from bounds known on the host: kv_bound, the most keys a
+ * sequence may have (of a window, window_size + mq - 1); rows = mq * q_per_kv; row_bytes, the bytes of a key of one
+ * kv head; quantised, an int4 or fp8 cache. */
+XFB200_API int32_t xfb200_decode_split_k(int32_t batch, int64_t kv_bound, int32_t kv_heads, int32_t rows, int32_t row_bytes,
+                                         int32_t quantised);
 XFB200_API int xfb200_decode_forward(const xfb200_decode_params* p, void* stream);
 
 /* Split-K decode that allocates nothing.  No counterpart in the reference.

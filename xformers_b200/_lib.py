@@ -36,6 +36,7 @@ EXPORTED_SYMBOLS = (
     "xfb200_prefill_device_status",
     "xfb200_decode_device_status",
     "xfb200_decode_scratch_bytes",
+    "xfb200_decode_split_k",
     "xfb200_decode_forward",
     "xfb200_decode_forward_static_scratch",
     "xfb200_merge_attentions",
@@ -237,6 +238,8 @@ def load() -> C.CDLL:
     lib.xfb200_decode_device_status.restype = C.c_int
     lib.xfb200_decode_scratch_bytes.argtypes = [C.c_int32] * 6
     lib.xfb200_decode_scratch_bytes.restype = C.c_size_t
+    lib.xfb200_decode_split_k.argtypes = [C.c_int32, C.c_int64] + [C.c_int32] * 4
+    lib.xfb200_decode_split_k.restype = C.c_int32
     lib.xfb200_decode_forward.argtypes = [C.POINTER(DecodeParams), C.c_void_p]
     lib.xfb200_decode_forward.restype = C.c_int
     lib.xfb200_decode_forward_static_scratch.argtypes = [C.POINTER(DecodeParams), C.c_void_p]
@@ -253,7 +256,7 @@ def load() -> C.CDLL:
         raise RuntimeError(f"the extension module xformers_b200._front cannot be loaded ({e}): build it with `python -m xformers_b200.build`") from e
     address = lambda f: C.cast(f, C.c_void_p).value
     _front.bind(address(lib.xfb200_prefill_forward), address(lib.xfb200_decode_forward), address(lib.xfb200_decode_scratch_bytes),
-                address(lib.xfb200_merge_attentions), address(lib.xfb200_rope_padded))
+                address(lib.xfb200_decode_split_k), address(lib.xfb200_merge_attentions), address(lib.xfb200_rope_padded))
     global front
     front = _front
     _LIB = lib

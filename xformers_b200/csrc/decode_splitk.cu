@@ -17,6 +17,8 @@
 // exist for each sequence in a fixed order, so results are bit-reproducible.
 // Lengths and page tables are read from device memory at run time; the grid
 // depends on static bounds only.
+#include <algorithm>
+
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -1796,6 +1798,31 @@ int decode_chunk_tokens(int kv_bound, int split_k) {
   return c < kDecChunkAlign ? kDecChunkAlign : c;
 }
 
+constexpr int kDecMaxSplits = 1024;
+
+// Tiles of query rows of one kv head in a CTA (1 or 2, of 16 rows for a 16-bit cache, of 8 for a quantised one), and the CTAs they take.
+static int row_tiles(int64_t rows, bool quantised) { return rows <= (quantised ? 8 : 16) ? 1 : 2; }
+static int num_row_blocks(int64_t rows, bool quantised) {
+  const int64_t per_cta = (quantised ? 8 : 16) * row_tiles(rows, quantised);
+  return int((rows + per_cta - 1) / per_cta);
+}
+
+// kv heads per CTA: the largest of 8, 4, 2, 1 that divides kv_heads -- fewer while the grid would still fit the machine at
+// once: an SM takes in at most some 90-110 GB/s, so a short context is read faster by all of them (4 sequences of 1000 keys, 8
+// heads: 32 CTAs of 512 KB at 8 heads each, 128 of 128 KB at 2).  A 16-bit cache only: the stripes of a quantised one are
+// short, and copied whole.
+static int largest_head_block(int kv_heads) {
+  int hb = 8;
+  while (kv_heads % hb) hb >>= 1;
+  return hb;
+}
+static int heads_per_cta(int64_t batch, int kv_heads, int row_blocks, int64_t split_k, bool quantised) {
+  int hb = largest_head_block(kv_heads);
+  if (!quantised)
+    while (hb > 1 && batch * (kv_heads / hb) * row_blocks * split_k * 2 <= sm_count()) hb >>= 1;
+  return hb;
+}
+
 template <int D, int MT, int kFmt, bool kBf16, int NG, int HB>
 static int launch_decode_t(const DecodeArgs& a_in, int head_blocks, cudaStream_t stream) {
   using Stage = DecStage<D, kFmt, NG>;
@@ -1870,6 +1897,41 @@ extern "C" size_t xfb200_decode_scratch_bytes(int32_t batch, int32_t mq, int32_t
   return o + l;
 }
 
+// Chunks into which the keys of a sequence are cut.  From static bounds only, never from lengths on the device, so that a
+// captured call may be replayed after they changed.
+//   Where chunks of 1280 tokens fill the machine four times over: those (measured optimum for every cache format at 8 kv heads per
+// CTA: 24-32 chunks of a 32k context).
+//   Below: what a small model of the launch says is fastest.  A CTA costs about 3 us before and after its tokens; these come at
+// its share of the memory bandwidth, at most 90 GB/s; the CTAs run in waves of one per SM (two where that many fit); partials
+// are written and read once at 5 TB/s (516 bytes a row, head dim 128; 64, with half of that, keeps the same rule), and the merge costs 2 us.  Two sequences of 16384 keys, 2 kv heads, went from 128
+// chunks (256 CTAs, two waves, 128 partials per row) to 64: 16.4 + 28.7 us to the figures at decode_merge_kernel.
+extern "C" int32_t xfb200_decode_split_k(int32_t batch, int64_t kv_bound, int32_t kv_heads, int32_t rows, int32_t row_bytes,
+                                         int32_t quantised) {
+  using namespace xfb;
+  if (batch < 1 || kv_bound < 1 || kv_heads < 1 || rows < 1) return 1;
+  const bool quant = quantised != 0;
+  const int64_t bound = (kv_bound + kDecChunkAlign - 1) / kDecChunkAlign * kDecChunkAlign, longest = std::min<int64_t>(bound, 1280);
+  auto chunks = [&](int64_t c) { return (bound + c - 1) / c; };
+  const int row_blocks = num_row_blocks(rows, quant), sms = sm_count();
+  if (batch * int64_t(kv_heads / largest_head_block(kv_heads)) * chunks(longest) >= 4 * sms) return int32_t(chunks(longest));
+  const bool one_tile = row_tiles(rows, quant) == 1;
+  const int per_sm = !quant ? DecOccupancy<kFmtPlain, 1>::kCtasPerSm : one_tile ? DecOccupancy<kFmtInt4, 1>::kCtasPerSm : DecOccupancy<kFmtInt4, 2>::kCtasPerSm;
+  const int64_t slots = int64_t(per_sm) * sms;
+  int64_t best = longest;
+  double best_us = 1e30;
+  for (int64_t c = kDecChunkAlign; c <= longest; c += kDecChunkAlign) {
+    const int64_t n = chunks(c);
+    if (n > kDecMaxSplits) continue;
+    const int hb = heads_per_cta(batch, kv_heads, row_blocks, n, quant);
+    const int64_t ctas = batch * (kv_heads / hb) * row_blocks * n, waves = (ctas + slots - 1) / slots;
+    const double gbs = std::min(90.0 / per_sm, 6400.0 / double(std::min(ctas, slots)));
+    const double us = double(waves) * (3.0 + double(c * hb * 2 * row_bytes) / (gbs * 1e3)) +
+                      (n > 1 ? 2.0 + 2.0 * double(batch * kv_heads * n * rows) * 516.0 / 5e6 : 0.0);
+    if (us < best_us * 0.98) best_us = us, best = c;
+  }
+  return int32_t(chunks(best));
+}
+
 extern "C" int xfb200_decode_forward(const xfb200_decode_params* p, void* stream) {
   using namespace xfb;
   if (p == nullptr) return set_error(XFB200_E_INVALID, "decode: null params");
@@ -1891,17 +1953,14 @@ extern "C" int xfb200_decode_forward(const xfb200_decode_params* p, void* stream
   if (fp8 && (p->k_scale_shift == nullptr || p->v_scale_shift == nullptr))
     return set_error(XFB200_E_INVALID, "decode: an fp8 cache needs k_scale_shift and v_scale_shift");
   if (fp8 && p->head_dim != 128) return set_error(XFB200_E_UNSUPPORTED, "decode: fp8 cache with head_dim %d (only 128)", p->head_dim);
-  if (p->split_k < 1 || p->split_k > 1024) return set_error(XFB200_E_INVALID, "decode: split_k %d out of range", p->split_k);
+  if (p->split_k < 1 || p->split_k > kDecMaxSplits) return set_error(XFB200_E_INVALID, "decode: split_k %d out of range", p->split_k);
   if (p->kv_padding < 1) return set_error(XFB200_E_INVALID, "decode: kv_padding must be positive");
   if (p->block_tables != nullptr && (p->page_size < 1 || p->block_table_stride < 1))
     return set_error(XFB200_E_INVALID, "decode: paged cache needs page_size and block_table_stride");
   if (p->mask_type != XFB200_MASK_NONE && p->mask_type != XFB200_MASK_CAUSAL_BOTTOM_RIGHT)
     return set_error(XFB200_E_UNSUPPORTED, "decode: mask_type %d", p->mask_type);
   const int R = p->mq * p->q_per_kv;
-  // query rows of one kv head per CTA: 16 or 32 (16-bit cache), 8 or 16 (int4 cache)
-  const int tile_rows = (int4 || fp8) ? 8 : 16;
-  const int mt = R <= tile_rows ? 1 : 2;
-  const int row_blocks = (R + tile_rows * mt - 1) / (tile_rows * mt);
+  const int mt = row_tiles(R, int4 || fp8), row_blocks = num_row_blocks(R, int4 || fp8);
   if (p->split_k > 1 && p->scratch == nullptr) return set_error(XFB200_E_INVALID, "decode: split_k > 1 needs scratch");
   if (p->split_k > 1 && (reinterpret_cast<uintptr_t>(p->scratch) & 255)) return set_error(XFB200_E_INVALID, "decode: scratch must be 256-B aligned");
 
@@ -1940,14 +1999,7 @@ extern "C" int xfb200_decode_forward(const xfb200_decode_params* p, void* stream
     a.status = words + kWordDecodeStatus;
   }
 
-  // kv heads per CTA: the largest of 8, 4, 2, 1 that divides kv_heads -- fewer while the grid would still fit the machine at
-  // once: an SM takes in at most some 110 GB/s, so a short context is read faster by all of them (4 sequences of 1000 keys, 8
-  // heads: 32 CTAs of 512 KB at 8 heads each, 128 of 128 KB at 2).  A 16-bit cache only: the stripes of a quantised one are
-  // short, and copied whole.
-  int hb = 8;
-  while (p->kv_heads % hb) hb >>= 1;
-  if (!int4 && !fp8)
-    while (hb > 1 && int64_t(p->batch) * (p->kv_heads / hb) * row_blocks * p->split_k * 2 <= sm_count()) hb >>= 1;
+  const int hb = heads_per_cta(p->batch, p->kv_heads, row_blocks, p->split_k, int4 || fp8);
   a.hb = hb;
   const int head_blocks = p->kv_heads / hb;
 

@@ -28,13 +28,15 @@ using OptTensor = std::optional<Tensor>;
 decltype(&xfb200_prefill_forward) g_prefill = nullptr;
 decltype(&xfb200_decode_forward) g_decode = nullptr;
 decltype(&xfb200_decode_scratch_bytes) g_scratch_bytes = nullptr;
+decltype(&xfb200_decode_split_k) g_split_k = nullptr;
 decltype(&xfb200_merge_attentions) g_merge = nullptr;
 decltype(&xfb200_rope_padded) g_rope = nullptr;
 
-void bind(uintptr_t prefill, uintptr_t decode, uintptr_t scratch_bytes, uintptr_t merge, uintptr_t rope) {
+void bind(uintptr_t prefill, uintptr_t decode, uintptr_t scratch_bytes, uintptr_t split_k, uintptr_t merge, uintptr_t rope) {
   g_prefill = reinterpret_cast<decltype(g_prefill)>(prefill);
   g_decode = reinterpret_cast<decltype(g_decode)>(decode);
   g_scratch_bytes = reinterpret_cast<decltype(g_scratch_bytes)>(scratch_bytes);
+  g_split_k = reinterpret_cast<decltype(g_split_k)>(split_k);
   g_merge = reinterpret_cast<decltype(g_merge)>(merge);
   g_rope = reinterpret_cast<decltype(g_rope)>(rope);
 }
@@ -162,40 +164,6 @@ py::object prefill(const View& q, const View& k, const View& v, const Sequences*
   return rc == XFB200_OK ? result(out, lse) : py::none();
 }
 
-// Chunks into which the keys of a sequence are cut.  From static bounds only, never from lengths on the device, so that a
-// captured call may be replayed after they changed.
-//   Where chunks of 1280 tokens fill the machine four times over: those (measured optimum for every cache format at 8 kv heads per
-// CTA: 24-32 chunks of a 32k context).
-//   Below: what a small model of the launch says is fastest.  A CTA costs about 3 us before and after its tokens; these come at
-// its share of the memory bandwidth, at most 90 GB/s; the CTAs run in waves of one per SM (two for quantised caches and up to 8 query rows); partials
-// are written and read once at 5 TB/s, and the merge itself costs 2 us.  Two sequences of 16384 keys, 2 kv heads, went from 128
-// chunks (256 CTAs, two waves, 128 partials per row) to 64: 16.4 + 28.7 us to the figures at decode_merge_kernel.
-int64_t split_k(int64_t batch, int64_t kv_bound, int64_t kv_heads, int64_t rows, int64_t row_bytes, bool quantised) {
-  constexpr int64_t kSms = 148;
-  int64_t hb0 = 8;
-  while (kv_heads % hb0) hb0 /= 2;
-  const int64_t bound = (kv_bound + 127) / 128 * 128;
-  auto chunks = [&](int64_t c) { return (bound + c - 1) / c; };
-  if (batch * (kv_heads / hb0) * chunks(std::min<int64_t>(bound, 1280)) >= 4 * kSms) return chunks(std::min<int64_t>(bound, 1280));
-  const bool two = quantised && rows <= 8;  // CTAs per SM, as the library picks it
-  const int64_t tile_rows = quantised ? 8 : 16, row_blocks = (rows + 2 * tile_rows - 1) / (2 * tile_rows), slots = two ? 2 * kSms : kSms;
-  int64_t best = std::min<int64_t>(bound, 1280);
-  double best_us = 1e30;
-  for (int64_t c = 128; c <= std::min<int64_t>(bound, 1280); c += 128) {
-    const int64_t n = chunks(c);
-    if (n > 1024) continue;  // (more than the library takes)
-    int64_t hb = hb0;  // as the library picks it
-    if (!quantised)
-      while (hb > 1 && batch * (kv_heads / hb) * row_blocks * n * 2 <= kSms) hb /= 2;
-    const int64_t ctas = batch * (kv_heads / hb) * row_blocks * n, waves = (ctas + slots - 1) / slots;
-    const double gbs = std::min(two ? 45.0 : 90.0, 6400.0 / double(std::min(ctas, slots)));
-    const double us = double(waves) * (3.0 + double(std::min(c, bound) * hb * 2 * row_bytes) / (gbs * 1e3)) +
-                      (n > 1 ? 2.0 + 2.0 * double(batch * kv_heads * n * rows) * 516.0 / 5e6 : 0.0);
-    if (us < best_us * 0.98) best_us = us, best = c;
-  }
-  return chunks(best);
-}
-
 py::object decode(const View& q, const View& k, const View& v, const Sequences* s, const Call& c) {
   const int64_t D = q.D;
   if (!(c.flags & kDecodeTakesBias) || c.bias != nullptr || (D != 64 && D != 128) || !q.rows16()) return py::none();
@@ -268,8 +236,8 @@ py::object decode(const View& q, const View& k, const View& v, const Sequences* 
   }
   if (p.kv_padding < 1) return py::none();
   p.kv_rows = q.B * k.M;
-  p.split_k = int32_t(split_k(batch, window ? std::min<int64_t>(p.kv_padding, p.window_size + mq - 1) : p.kv_padding, p.kv_heads, mq * p.q_per_kv,
-                              k.D * k.t.element_size(), words));
+  p.split_k = g_split_k(p.batch, window ? std::min<int64_t>(p.kv_padding, p.window_size + mq - 1) : p.kv_padding, p.kv_heads, p.mq * p.q_per_kv,
+                        int32_t(k.D * k.t.element_size()), words);
   p.scale = c.scale;
   Tensor out = new_out(q, c.out_dtype), lse;
   if (c.flags & (kWantLse | kPartial)) lse = at::empty({q.G, q.H, total}, q.t.options().dtype(at::kFloat));
@@ -458,7 +426,9 @@ py::object rope(const Tensor& xq, const Tensor& xk, const Tensor& xv, const Tens
 PYBIND11_MODULE(_front, m) {
   m.doc() = "Host front of the xformers_b200 operators (see csrc/front.cpp)";
   m.def("bind", &bind);
-  m.def("split_k", &split_k);
+  m.def("split_k", [](int32_t batch, int64_t kv_bound, int32_t kv_heads, int32_t rows, int32_t row_bytes, bool quantised) {
+    return g_split_k(batch, kv_bound, kv_heads, rows, row_bytes, quantised);
+  });
   m.def("dense", &dense);
   m.def("varlen", &varlen);
   m.def("merge", &merge);

@@ -231,11 +231,10 @@ class FwOp(AttentionFwOpBase):
     @classmethod
     def get_split_k(cls, batch: int, kv_bound: int, kv_heads: int, row_bytes: int, rows: int = 8, quantised: bool = False) -> int:
         """Number of key chunks per sequence: ``SPLIT_K`` where a subclass fixes
-        it, else the host front's rule (``split_k`` in csrc/front.cpp)."""
+        it, else the library's rule (``xfb200_decode_split_k``)."""
         if cls.SPLIT_K is not None:
             return max(1, int(cls.SPLIT_K))
-        _lib.load()
-        return _lib.front.split_k(batch, kv_bound, kv_heads, rows, row_bytes, quantised)
+        return _lib.load().xfb200_decode_split_k(batch, kv_bound, kv_heads, rows, row_bytes, quantised)
 
     @classmethod
     def apply(cls, inp: Inputs, needs_gradient: bool) -> Tuple[torch.Tensor, Optional[Context]]:
