@@ -189,3 +189,22 @@ def test_front_leaves_changed_operators_to_python(op, monkeypatch):
             _both(m, call, takes=False)
         _both(monkeypatch, call, takes=True)
     assert splits and len(paths) == 2
+
+
+@gpu
+def test_calls_without_the_front(monkeypatch):
+    """Every kind of call that the front serves, with no front at all."""
+    require_cuda()
+    gen = torch.Generator().manual_seed(9)
+    bias, rows = _bias("BlockDiagonalCausalWithOffsetPaddedKeysMask", [1] * 3, [50, 90, 64], 96, 32)
+    xq, xk, xv = _mk(gen, 1, 3, 2, 4, 64), _mk(gen, 1, 3, 2, 1, 64), _mk(gen, 1, 3, 2, 1, 64)
+    q, k, v = (_mk(gen, 1, 33, 4, 64) for _ in range(3))
+    got = []
+    for f in (_lib.front, None):
+        monkeypatch.setattr(_lib, "front", f)
+        ck, cv = (torch.ones(1, rows, 2, 1, 64, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        r = xops.rope_padded(xq, xk, xv, ck, cv, bias)
+        o, l = fmha.memory_efficient_attention_partial(r, ck.expand(-1, -1, -1, 4, -1), cv.expand(-1, -1, -1, 4, -1), bias)
+        got.append((ck, cv, r, o, l, *fmha.merge_attentions([o, o], [l, l]), xops.memory_efficient_attention_forward(q, k, v, ab.LowerTriangularMask())))
+    monkeypatch.undo()
+    _same(*got)

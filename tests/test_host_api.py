@@ -4,6 +4,8 @@ dispatch rules, the C-ABI library's exports."""
 import ctypes
 import os
 import re
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -257,3 +259,21 @@ def test_split_k_stays_in_range_for_long_contexts(rows, quantised):
     f = fmha.b200_splitk.FwOp.get_split_k
     for bound in list(range(200_000, 1_310_720, 7_001)) + [611_461, 618_789, 619_807, 1_310_720]:
         assert 1 <= f(1, bound, 8, 256, rows, quantised) <= 1024
+
+
+def test_package_works_without_the_host_front():
+    """The front only spares calls the Python path: without the module (or with one built for another torch) the package imports, says
+    so, and its operators are available."""
+    code = """
+import sys, warnings
+sys.modules["xformers_b200._front"] = None
+with warnings.catch_warnings(record=True) as seen:
+    warnings.simplefilter("always")
+    from xformers_b200.ops import fmha
+from xformers_b200 import _lib
+assert _lib.front is None and any("_front" in str(w.message) for w in seen)
+assert all(op.is_available() for op in fmha.ALL_FW_OPS)
+assert fmha.b200_splitk.FwOp.get_split_k(64, 32768, 8, 256) == 26
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr

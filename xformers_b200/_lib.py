@@ -9,10 +9,9 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import warnings
 from pathlib import Path
 from typing import Any, Optional
-
-import torch  # noqa: F401  (the extension module is linked against its libraries)
 
 ABI_VERSION = 4
 
@@ -210,12 +209,28 @@ def library_path() -> Path:
 
 
 _LIB: Optional[C.CDLL] = None
-front: Any = None  # the extension module _front (csrc/front.cpp), once load() has bound it to the library
+front: Any = None  # the extension module _front (csrc/front.cpp), once load() has bound it to the library; None without it
+
+
+def _load_front(lib: C.CDLL) -> Any:
+    """The extension module ``_front`` bound to ``lib``; ``None`` (and a warning) when it is missing or was built for another
+    torch: every call then takes the Python path, which runs the same kernels and costs 50 us more."""
+    try:
+        import torch  # noqa: F401  (the module is linked against its libraries)
+
+        from . import _front
+    except ImportError as e:
+        warnings.warn(f"xformers_b200._front cannot be loaded ({e}): calls take the slower Python path; `python -m xformers_b200.build` builds it", RuntimeWarning)
+        return None
+    address = lambda f: C.cast(f, C.c_void_p).value
+    _front.bind(address(lib.xfb200_prefill_forward), address(lib.xfb200_decode_forward), address(lib.xfb200_decode_scratch_bytes),
+                address(lib.xfb200_decode_split_k), address(lib.xfb200_merge_attentions), address(lib.xfb200_rope_padded))
+    return _front
 
 
 def load() -> C.CDLL:
     """Load the library once; raise a clear error if it is absent."""
-    global _LIB
+    global _LIB, front
     if _LIB is not None:
         return _LIB
     path = library_path()
@@ -250,15 +265,7 @@ def load() -> C.CDLL:
     lib.xfb200_rope_padded.restype = C.c_int
     if lib.xfb200_abi_version() != ABI_VERSION:
         raise RuntimeError(f"{path}: ABI version {lib.xfb200_abi_version()} != {ABI_VERSION}")
-    try:
-        from . import _front
-    except ImportError as e:
-        raise RuntimeError(f"the extension module xformers_b200._front cannot be loaded ({e}): build it with `python -m xformers_b200.build`") from e
-    address = lambda f: C.cast(f, C.c_void_p).value
-    _front.bind(address(lib.xfb200_prefill_forward), address(lib.xfb200_decode_forward), address(lib.xfb200_decode_scratch_bytes),
-                address(lib.xfb200_decode_split_k), address(lib.xfb200_merge_attentions), address(lib.xfb200_rope_padded))
-    global front
-    front = _front
+    front = _load_front(lib)
     _LIB = lib
     return lib
 
