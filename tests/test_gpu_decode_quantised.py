@@ -60,3 +60,42 @@ def test_quantised_tile_edges(fmt, D, kv_heads, group, mq, split_k):
 def test_quantised_query_magnitudes(fmt, dtype, mag):
     require_cuda()
     _run(fmt, 2, 8, 128, dtype, mag)
+
+
+def _int4_rows(scale, shift, n):
+    """Rows of the int4 format: [rows] scales and shifts, [rows, D] nibbles -> [rows, 1 + D / 8] words."""
+    half = lambda x: x.half().view(torch.int16).long() & 0xFFFF
+    packed = (n.long().view(n.shape[0], -1, 8) << torch.arange(0, 32, 4)).sum(-1)
+    w = torch.cat([(half(scale) | half(shift) << 16)[:, None], packed], 1)
+    return torch.where(w >= 1 << 31, w - (1 << 32), w).int()
+
+
+@gpu
+@pytest.mark.parametrize("peaks", ["one per sub-tile", "any weight"])
+@pytest.mark.parametrize("kv_heads,group", [(1, 8), (2, 16), (8, 4)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_int4_columns_are_equally_accurate(D, kv_heads, group, peaks):
+    """f32 output.  The tensor core cuts the products of a sub-tile off against the largest of them, so their place in the 16
+    bits counts: neighbouring columns that hold the same values must give the same bits.  The weights are powers of two (f16
+    holds them and V's scales exactly), so that these cuts and those of the running sum are the error."""
+    require_cuda()
+    N = 4096
+    g = torch.Generator().manual_seed(D)
+    q = torch.zeros(1, 1, kv_heads, group, D, dtype=torch.bfloat16)
+    q[..., 0] = 1
+    kn = torch.zeros(N, D, dtype=torch.int32)
+    kn[:, 0] = 2
+    kn[::16, 0] = 15
+    if peaks == "any weight":
+        kn[:, 0] = torch.randint(0, 16, (N,), generator=g)
+    vn = torch.randint(0, 16, (N, D // 2), generator=g).repeat_interleave(2, -1)
+    vs = 1 + torch.randint(0, 1024, (N,), generator=g) / 1024.0
+    cache = lambda words: words.cuda().view(1, N, 1, 1, -1).expand(-1, -1, kv_heads, -1, -1).contiguous().expand(-1, -1, -1, group, -1)
+    k, v = cache(_int4_rows(torch.ones(N), torch.full((N,), -15.0), kn)), cache(_int4_rows(vs, torch.zeros(N), vn))
+    out, _ = fmha.memory_efficient_attention_partial(q.cuda(), k, v, None, scale=0.6931471805599453, op=S.FwOp_S1, output_dtype=torch.float32)
+    assert torch.equal(out[..., 0::2], out[..., 1::2])
+    p = torch.exp2(kn[:, 0].double() - 15)
+    want = (p[:, None] * vn.double() * vs[:, None].double()).sum(0) / p.sum()
+    # a warp adds its sub-tiles of 16 keys (8 warps share the heads) to f32 sums that are cut off, not rounded: 2^-23 each; one
+    # more 2^-22 for the exponentials and the sum over the warps.  Measured: 3.1e-6, 6.2e-6, 2.6e-5 with 1, 2, 8 kv heads.
+    assert ((out.double().cpu() - want) / want).abs().max() <= N // 16 * kv_heads // 8 * 2.0**-23 + 2.0**-22

@@ -656,12 +656,13 @@ __device__ __forceinline__ void quant_rows_finish(QuantRows<NTQ>& q, const DecWa
 //  * A nibble is used almost where it sits, as a subnormal f16, which the tensor
 //    cores multiply exactly: (w << 2) & 0x003C003C is the pair (n_e, n_{e+4}) *
 //    2^-22 and (w << 2) & 0x03C003C0 the pair n * 2^-18; w >> 6 has the upper byte
-//    of each half in the same places.  A word costs two shifts and four ANDs for
-//    8 nibbles.  The power of two is taken out of the output rows (V) and of K's
-//    scale; K's even elements are brought to 2^-18 too, because the tensor core
-//    aligns subnormals by their exponent field, so that the sum of the products
-//    keeps all its bits only for those in the upper bits (LSE error up to 4e-6
-//    instead of 1e-6 with the plain w & 0x000F000F).
+//    of each half in the same places.  The first kind is multiplied by 16 on the
+//    FMA pipe: the tensor core aligns subnormals by their exponent field, so that
+//    the sum of the products keeps all its bits only for those in the upper bits
+//    (K without it: LSE error up to 4e-6 instead of 1e-6; V: f32 output off by
+//    5.2e-6 in those columns instead of 3.1e-6, what nibbles made normal numbers
+//    give).  A word costs two shifts, four ANDs and two products for 8 nibbles.  The
+//    power of two is taken out of the output rows (V) and of K's scale.
 //  * K: thread (r, c) reads word 4i + c of tokens r and r + 8; its nibble pairs
 //    (e, e + 4) are the k-slots (2c, 2c+1) / (2c+8, 2c+9) of k-steps 2i and
 //    2i + 1.  Q^T is loaded in the same permuted order of d.
@@ -675,9 +676,10 @@ __device__ __forceinline__ void quant_rows_finish(QuantRows<NTQ>& q, const DecWa
 //    so that one's loads and unpacking fill the other's waits and the softmax's
 //    overhead is paid once for 32 tokens.
 // 64 sequences of 1024 to 32768 keys, 8 kv heads, 64 query heads, pages of 256:
-// 388 -> 274 us (2.84 -> 4.02 TB/s); 128 query heads 924 -> 463 us, 32 query heads
-// on 4 kv heads, pages of 64, 221 -> 156 us.  The issue slots are what is left:
-// about 290 instructions per sub-tile were 437.
+// 388 -> 290 us (2.84 -> 3.80 TB/s; 280 with V's even elements left where they
+// are).  About 310 instructions per sub-tile were 437; neither the issue slots (2.3 of
+// 4) nor the integer pipe (55 %) are full, so what is left is their dependent latency
+// with four warps per scheduler.
 // ---------------------------------------------------------------------------
 template <int D, int NTQ, bool kBf16, int HB>
 __device__ __forceinline__ void consume_int4(const DecodeArgs& a, const DecWarp& w) {
@@ -692,12 +694,12 @@ __device__ __forceinline__ void consume_int4(const DecodeArgs& a, const DecWarp&
   const int lane = w.lane, r = lane >> 2, c = lane & 3;
   const int hw = w.hw;
 
-  // nibble pairs (e, e+4) of a packed word as f16 pairs: n * 2^-22 for even e, n * 2^-18 for odd e
+  // nibble pairs (e, e+4) of a packed word as f16 pairs n * 2^-18
   auto unpack4 = [](uint32_t x, uint32_t (&out)[4]) {
     const uint32_t lo = x << 2, hi = x >> 6;
-    out[0] = lo & 0x003C003Cu;
+    out[0] = (lo & 0x003C003Cu) * 16u;
     out[1] = lo & 0x03C003C0u;
-    out[2] = hi & 0x003C003Cu;
+    out[2] = (hi & 0x003C003Cu) * 16u;
     out[3] = hi & 0x03C003C0u;
   };
 
@@ -765,8 +767,6 @@ __device__ __forceinline__ void consume_int4(const DecodeArgs& a, const DecWarp&
           uint32_t u0[4], u1[4];
           unpack4(k0[u * u_step * rw + 1 + 4 * i + c], u0);
           unpack4(k0[(u * u_step + 8) * rw + 1 + 4 * i + c], u1);
-#pragma unroll
-          for (int e = 0; e < 4; e += 2) u0[e] *= 16u, u1[e] *= 16u;  // (on the FMA pipe)
           const uint32_t ka[4] = {u0[0], u1[0], u0[1], u1[1]};
           const uint32_t kb[4] = {u0[2], u1[2], u0[3], u1[3]};
 #pragma unroll
@@ -819,7 +819,7 @@ __device__ __forceinline__ void consume_int4(const DecodeArgs& a, const DecWarp&
       for (int q = 0; q < 4; ++q) {
         const int d = 8 * (WPT * r + (mt >> 2)) + (mt & 3) + (q >> 1) * 4;
         const int rr = nt * 8 + 2 * c + (q & 1);
-        w.mine[rr * kCmbRow + d] = fmaf(acc[mt][nt][q], (mt & 1) ? 262144.f : 4194304.f, rows.corr[nt][q & 1]);
+        w.mine[rr * kCmbRow + d] = fmaf(acc[mt][nt][q], 262144.f, rows.corr[nt][q & 1]);
       }
 }
 
