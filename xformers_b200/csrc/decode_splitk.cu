@@ -1816,10 +1816,10 @@ static int largest_head_block(int kv_heads) {
   while (kv_heads % hb) hb >>= 1;
   return hb;
 }
-static int heads_per_cta(int64_t batch, int kv_heads, int row_blocks, int64_t split_k, bool quantised) {
+static int heads_per_cta(int64_t batch, int kv_heads, int row_blocks, int64_t split_k, bool quantised, int sms) {
   int hb = largest_head_block(kv_heads);
   if (!quantised)
-    while (hb > 1 && batch * (kv_heads / hb) * row_blocks * split_k * 2 <= sm_count()) hb >>= 1;
+    while (hb > 1 && batch * (kv_heads / hb) * row_blocks * split_k * 2 <= sms) hb >>= 1;
   return hb;
 }
 
@@ -1922,7 +1922,7 @@ extern "C" int32_t xfb200_decode_split_k(int32_t batch, int64_t kv_bound, int32_
   for (int64_t c = kDecChunkAlign; c <= longest; c += kDecChunkAlign) {
     const int64_t n = chunks(c);
     if (n > kDecMaxSplits) continue;
-    const int hb = heads_per_cta(batch, kv_heads, row_blocks, n, quant);
+    const int hb = heads_per_cta(batch, kv_heads, row_blocks, n, quant, sms);
     const int64_t ctas = batch * (kv_heads / hb) * row_blocks * n, waves = (ctas + slots - 1) / slots;
     const double gbs = std::min(90.0 / per_sm, 6400.0 / double(std::min(ctas, slots)));
     const double us = double(waves) * (3.0 + double(c * hb * 2 * row_bytes) / (gbs * 1e3)) +
@@ -1999,7 +1999,7 @@ extern "C" int xfb200_decode_forward(const xfb200_decode_params* p, void* stream
     a.status = words + kWordDecodeStatus;
   }
 
-  const int hb = heads_per_cta(p->batch, p->kv_heads, row_blocks, p->split_k, int4 || fp8);
+  const int hb = heads_per_cta(p->batch, p->kv_heads, row_blocks, p->split_k, int4 || fp8, sm_count());
   a.hb = hb;
   const int head_blocks = p->kv_heads / hb;
 
