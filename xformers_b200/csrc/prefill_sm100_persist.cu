@@ -924,9 +924,20 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
       uint8_t* const bias_smem = smem + L::kBias + warp * L::kBiasUnit;
       // Row r reads its visible keys only, [r + rel_lo, min(r + rel_hi, n_keys)), and has 0 for the others: their scores are -inf
       // already, and what the bias holds there, a NaN perhaps, must not meet that.  (Masking behind the addition instead costs the
-      // step registers: 75.5 -> 86.7 us for 2 x 2048 x 2048, 8 heads, no mask at all.)
-      auto bias_load = [&](uint4* w, int64_t off, int mt0, int qlen, int col_first, int n_keys, int rel_lo, int rel_hi) {
+      // step registers: 75.5 -> 86.7 us for 2 x 2048 x 2048, 8 heads, no mask at all.)  `whole`: a step of which every row and key
+      // counts, and rows on 16-byte boundaries; its loads need no test (the tests cost that call 3.4 us).
+      auto bias_load = [&](uint4* w, int64_t off, int mt0, int qlen, int col_first, int n_keys, int rel_lo, int rel_hi, bool whole) {
         const int esz = bias_f32 ? 4 : 2, per16 = 16 / esz;
+        if (whole) {
+          const int r = mt0 + (warp & 3) * 32 + (lane >> 2);
+          const uint8_t* src = reinterpret_cast<const uint8_t*>(a.bias) + (off + int64_t(r) * a.bias_m + col_first + (lane & 3) * per16) * esz;
+          const int64_t step = 8 * a.bias_m * esz;
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) w[u * 4 + i] = __ldg(reinterpret_cast<const uint4*>(src + i * step + u * 64));
+          return;
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int r = mt0 + (warp & 3) * 32 + i * 8 + (lane >> 2);
@@ -1046,13 +1057,15 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           const bool need_mask = (n0 + kBN > klen) || (causal && n0 + kBN - 1 > mt0 + shift + a.window_right) ||
                                  (a.window_left >= 0 && n0 < mt0 + kBM - 1 + shift - a.window_left);
           uint4 bw[kBias ? 16 : 1];
+          bool whole = false;
           int rel_lo = 0, rel_hi = 0;  // visible keys of row r: from r + rel_lo, below r + rel_hi
           if constexpr (kBias) {
             // asked for before the wait for the scores, which hides most of their latency; the next step's are asked
             // into the L2 at the same time
             rel_lo = a.window_left >= 0 ? shift - a.window_left : -0x3fffffff;
             rel_hi = causal ? shift + a.window_right + 1 : 0x3fffffff;
-            bias_load(bw, it.bias_off, mt0, it.qlen, n0, klen, rel_lo, rel_hi);
+            whole = a.bias_vec && !need_mask && mt0 + kBM <= it.qlen;
+            bias_load(bw, it.bias_off, mt0, it.qlen, n0, klen, rel_lo, rel_hi, whole);
             bias_prefetch(it.bias_off, mt0, it.qlen, n0 + kBN, j + 1 < jhi ? klen : 0);
           }
           ok = mbar_wait(&bar->s_full[t], cnt & 1, abort_flag, budget);
@@ -1106,7 +1119,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
               XFB_TMEM_ST_32(tmem_s, sa);
               bias_add(sb, bw, 1);
               XFB_TMEM_ST_32(tmem_s + 32, sb);
-              if (bias_f32) bias_load(bw, it.bias_off, mt0, it.qlen, n0 + 64, klen, rel_lo, rel_hi);
+              if (bias_f32) bias_load(bw, it.bias_off, mt0, it.qlen, n0 + 64, klen, rel_lo, rel_hi, whole);
             }
             float mx = fmaxf(chunk_max(reinterpret_cast<float*>(sa)), chunk_max(reinterpret_cast<float*>(sb)));
             if constexpr (kBias) tc_wait_st();
