@@ -122,8 +122,8 @@ typedef struct {
    * fmha/attn_bias.py:43; tests/test_mem_eff_attention.py:1440-1449): NULL, or
    * [batch, G, H, mq, mkv] with unit stride on the last axis and element strides
    * below (0 = broadcast), added to q k^T * scale before the mask and the softmax.
-   * Dense batches only; runs on the persistent tcgen05 kernel (head dim 64 / 128) or on
-   * the mma.sync kernel. */
+   * Dense batches only; runs on the persistent tcgen05 kernel (head dims up to 128) or on
+   * the mma.sync kernel.  What it holds at a key that the mask hides is not used. */
   const void* bias;
   int32_t bias_dtype; /* XFB200_BF16 | XFB200_F16 | XFB200_F32 */
   int32_t window_right; /* XFB200_MASK_LOCAL_BOTTOM_RIGHT: keys j <= i + shift + window_right (>= 0); else ignored */

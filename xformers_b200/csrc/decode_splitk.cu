@@ -1,10 +1,10 @@
 // Split-K decode attention: few queries per sequence against a long KV cache.
 //
 // HBM-bound.  One CTA owns (sequence b, key chunk s, block of kv heads): a
-// producer warp streams that chunk of the cache into a 3-deep shared-memory
-// ring with 1-D bulk TMA copies (whole token stripes, all heads of the block
-// at once when they are contiguous, so every request is >= 256 B and
-// 16-B aligned), 8 consumer warps do QK^T and PV with warp-level
+// producer warp streams that chunk of the cache into a shared-memory ring of 3
+// to 12 stages, with tiled TMA copies (16-bit and fp8 caches: a run of tokens
+// with all heads of the block) or bulk ones (int4 rows, and whatever a tensor
+// map cannot describe), 8 consumer warps do QK^T and PV with warp-level
 // mma.sync.m16n8k16 (query heads of a GQA group are the M rows, tokens the N
 // columns; K/V are never expanded), the online softmax lives in registers.
 // The int4 row-wise cache is unpacked in registers, nibbles becoming subnormal
@@ -452,8 +452,8 @@ __device__ __forceinline__ void consume_plain(const DecodeArgs& a, const DecWarp
 // S^T = K Q^T and the K dimension of O^T = V^T P^T, the query rows (8 per
 // n-tile) are the N columns, so no MMA row is padding when the GQA group has 8
 // query heads.  Both products run in f16 whatever the type of Q.
-//   Issue slots bound these consumers, and a warp's sub-tile is one chain of
-// dependent steps, so the softmax is arranged for few instructions:
+//   Instructions and their latency bound these consumers, and a warp's sub-tile is one
+// chain of dependent steps, so the softmax is arranged for few instructions:
 //  * scale and shift of a key are applied to the score, relative to the row's
 //    reference maximum at once: (s * scale + shift * sum(q)) * fac - ref is
 //    three instructions, and its exponential the probability.
@@ -651,7 +651,7 @@ __device__ __forceinline__ void quant_rows_finish(QuantRows<NTQ>& q, const DecWa
 
 // ---------------------------------------------------------------------------
 // int4 row-wise cache.  The integer pipe that unpacks the nibbles (16 lanes per
-// clock and scheduler) and the issue slots bound this path, so everything is
+// clock and scheduler) and the latency of what it does bound this path, so everything is
 // arranged to spend as few operations per nibble as possible:
 //  * A nibble is used almost where it sits, as a subnormal f16, which the tensor
 //    cores multiply exactly: (w << 2) & 0x003C003C is the pair (n_e, n_{e+4}) *
@@ -677,9 +677,9 @@ __device__ __forceinline__ void quant_rows_finish(QuantRows<NTQ>& q, const DecWa
 //    overhead is paid once for 32 tokens.
 // 64 sequences of 1024 to 32768 keys, 8 kv heads, 64 query heads, pages of 256:
 // 388 -> 290 us (2.84 -> 3.80 TB/s; 280 with V's even elements left where they
-// are).  About 310 instructions per sub-tile were 437; neither the issue slots (2.3 of
-// 4) nor the integer pipe (55 %) are full, so what is left is their dependent latency
-// with four warps per scheduler.
+// are).  314 instructions per sub-tile were 437; neither the issue slots (2.3 of 4)
+// nor the integer pipe (56 %) are full, so what is left is their dependent latency with
+// four warps per scheduler.
 // ---------------------------------------------------------------------------
 template <int D, int NTQ, bool kBf16, int HB>
 __device__ __forceinline__ void consume_int4(const DecodeArgs& a, const DecWarp& w) {

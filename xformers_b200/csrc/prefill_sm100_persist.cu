@@ -1,7 +1,8 @@
 // Attention forward (prefill) on tcgen05: one persistent CTA per SM.
 //
 // A work item is a block of 256 query rows of one (sequence, query head): two
-// 128-row query tiles that share every K/V tile TMA brings in.  Items are
+// 128-row query tiles that share every K/V tile TMA brings in.  (One tile, where
+// the tiles of the whole launch are no more than the SMs.)  Items are
 // handed out by one atomic counter, heaviest first (the last row block of every
 // head, then the one before, ...) inside groups of heads whose keys and values
 // fit the L2 together, so the SMs stay evenly loaded whatever the sequence
@@ -214,8 +215,8 @@ __device__ __forceinline__ void give_up(const Sm100Args& a, int code) {
 // Order in which the sequences of a packed batch are taken: longest first (lane r holds the sequence of rank r).  Contexts of a
 // chunked prefill differ by an order of magnitude, and items are only ordered inside a sequence: the long ones must not come
 // last (8 sequences of 835 to 6822 keys, 150 to 480 new tokens each: 206 -> 191 us with the rotary pass; simulated item by item the
-// launch goes from 162 to 128, 120 being the mean over the SMs).  A warp ranks up to 32 sequences; a longer batch keeps its order, its
-// items are many.
+// launch goes from 162 to 128, 120 being the mean over the SMs).  A warp ranks up to 32 sequences, one per lane; a longer batch keeps
+// the order it came in (not measured there: one long context behind many short ones still ends the launch alone).
 __device__ __forceinline__ int sequence_order(const Sm100Args& a, int lane) {
   if (a.seqstart_q == nullptr || a.batch > 32) return lane;
   int keys = -1;
@@ -914,7 +915,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
       // scores, and reading memory that way costs one sector request per element (2048 x 2048 x 16 heads, bf16: 600 us).
       // A warp therefore reads its 32 rows in units of 64 bytes per row, four lanes to a row and 16 bytes to a lane, holds
       // the units of a step in registers from before the wait for the scores on, and turns one after the other into
-      // rows through 2 KB of shared memory (16-byte chunks XOR-ed with row / 2, no bank conflict either way): 82 us for the
+      // rows through 2 KB of shared memory (16-byte chunks XOR-ed with row / 2, no bank conflict either way): 69 us for the
       // same call (34 GFLOP, 134 MB of bias).  A unit is
       // 32 columns of a 16-bit bias (four units: a step) or 16 of an f32 one (four: half a step).
       const bool bias_f32 = !kBiasSame && a.bias_dtype == XFB200_F32;

@@ -148,7 +148,7 @@ class LocalAttentionFromBottomRightMask(AttentionBias):
 
 class LowerTriangularMaskWithTensorBias(LowerTriangularMask):
     """Causal mask plus an additive tensor ``[B, (G,) H, Mq, Mkv]``
-    (tests/test_mem_eff_attention.py:1431-1449); runs on the mma.sync prefill kernel."""
+    (tests/test_mem_eff_attention.py:1431-1449); runs on the prefill kernels."""
 
     HOLDS_DENSE_TENSOR = True
 

@@ -298,7 +298,8 @@ class FwOp_Tcgen05(FwOp):
 
 
 class FwOp_Tcgen05_Persistent(FwOp_Tcgen05):
-    """tcgen05 kernel, one persistent CTA per SM pulling blocks of 256 query rows (the default)."""
+    """tcgen05 kernel, one persistent CTA per SM pulling blocks of 256 query rows, or of 128 where those are no more than the
+    SMs (the default)."""
 
     NAME = "b200F-tc5-persistent"
     KERNEL_PATH = _lib.PREFILL_TCGEN05_PERSISTENT
