@@ -16,8 +16,7 @@
 //   warps 8-11   output: O_t / l -> global memory, log-sum-exp.  They work on
 //                item i while every other warp is already on item i + 1, so
 //                the tensor pipe does not wait for the write-back.
-//   warp 12/13   MMA issuer of tile 0 / 1 (one lane issues); the two pass a
-//                token so that their blocks of MMAs alternate on the tensor pipe
+//   warp 12/13   MMA issuer of P_t V of tile 0 / 1 (one lane issues)
 //   warp 14      scheduler + TMA producer: pulls the next item one item ahead of
 //                time, works out its geometry once and announces it to the other
 //                warps through a small ring of descriptors in shared memory,
@@ -25,38 +24,38 @@
 //                on across item boundaries.  Items in which no query sees any
 //                key (possible when the key axis is sharded) never enter the
 //                ring: this warp writes their zeros and -inf itself.
-//   warp 15      idle
+//   warp 15      MMA issuer of Q_t K^T, both tiles in turn
 //
-// Tensor memory (all 512 columns): S0 | S1 | O0 | O1, fp32.  The probabilities
-// P_t overwrite the last 64 columns of S_t as packed 16-bit pairs (keys 64-127
-// in columns 64-95, keys 0-63 in columns 96-127) and feed the PV product
-// straight from tensor memory.  tcgen05 operations issued by one
-// thread complete in order: when the barrier of QK(t, j) fires, PV(t, j-1) has
-// finished, so the softmax may rescale O_t and overwrite S_t / P_t without
-// further hand-shakes; across items the first PV of a tile waits until the
+// Tensor memory: S | P0 | P1 | O0 | O1.  There is one buffer of scores: as soon
+// as the softmax of a tile has its 128 scores in registers, the buffer goes to
+// Q K^T of the other tile, which is through long before that tile's softmax asks
+// for it.  So nothing a tile's softmax waits for hangs on its own last step except
+// P V (P_t is free and O_t may be rescaled once that is through), and the two
+// tiles stay half a step apart: one is in its exponentials while the other reads
+// scores and looks for the maximum.  Across items the first PV of a tile waits until the
 // output warps have read the previous O_t out of tensor memory.
 //
-// Softmax: thread = row.  A step reads the row's 128 scores out of tensor memory
-// twice.  First for their maximum: if it exceeds the row's reference maximum by
-// more than 2^8 the row is re-based at once (O_t is quiescent at that point, see
-// above), otherwise the reference stays and nothing is rescaled -- one vote and
-// one rarely taken branch per step.  Then for the probabilities, which are stored
-// back as P chunk by chunk.  The second pass starts with the two chunks (of 32
-// columns) the first one ended with, straight from registers, and P goes into
-// columns 64-127 in the order in which it is produced (keys 64-127 first), so
-// that only the first 64 columns are read a second time and their loads fly
-// behind the exponentials of the other half.  A warp runs almost alone on its
-// scheduler: every vote, branch or wait it executes is a bubble nobody fills, so
-// the step has no loop and no per-chunk test.  On diagonal and ragged tiles a
+// What bounds a step of 2 x 128 rows x 128 keys: 2048 clocks of MMAs and 2048 clocks of exponentials
+// (4 per clock and scheduler).  Its period is 2760 clocks (D = 128, no mask), given by the buffer
+// of scores: per tile 220 to read it, 570-650 for the MMAs, the rest barriers and latency of the
+// pipe.  Before, P_t overwrote S_t, so that the scores of the next step had to wait for softmax
+// and P V of this one: 3500 clocks.
+//
+// Instruction fetch is what such a kernel trips over: softmax and issuers run different
+// code side by side, two tiles half a step apart, and the cache of an SM holds little.  With the
+// issuers unrolled per tile, a lane chosen by `lane == 0` (every MMA operand is then brought to uniform registers one by one),
+// and long wait loops, the kernel had 110 KB of code, 21 % of the instruction requests missed (the former design: 10 %) and the
+// schedule above took 3900 clocks.  Hence: one copy of the code for both tiles, short loops,
+// elect.sync, a warp index known to be uniform, a wait loop of a few instructions, one place
+// per role that reports an error: 60 KB, 0.6 % misses.
+//
+// Softmax: thread = row.  If the maximum of a step exceeds the row's reference maximum by
+// more than 2^8 the row is re-based at once; otherwise the reference stays and nothing is rescaled -- one vote and
+// one rarely taken branch per step.  Then the probabilities are formed and stored as P chunk by chunk.  On diagonal and ragged tiles a
 // small loop first writes -inf over the hidden scores in tensor memory; the step
-// itself is one piece of code for every tile, which the instruction cache likes.
-// An additive bias is added in the first pass (kernel variants of their own).  When the first half of P (keys 64-127) is stored the softmax
-// arrives on a barrier of its own and the MMA warp issues that half of PV while
-// the other half is still being computed.  Measured
-// alternatives on the causal 4k case: one pass with a stale reference, a vote per
-// chunk and a fix-up path (10 % slower: the votes and branches); the whole row in
-// registers as in the one-CTA-per-block kernel; two threads per row; part of the
-// exponentials as a cubic on the FMA pipe (slower at every fraction).
+// itself is one piece of code for every tile.
+// An additive bias is added behind the load (kernel variants of their own).  When the first half of P (keys 0-63) is stored the softmax
+// arrives on a barrier of its own and the PV warp issues that half while the other half is still being computed.
 //
 // Masks are index arithmetic on (row, key) positions; K/V heads of a GQA group
 // are indexed, never expanded; V rows past a sequence's end are zeroed in
@@ -81,14 +80,14 @@ constexpr int kBN = 128;    // keys per step
 constexpr int kStages = 2;  // depth of the K and of the V ring
 constexpr int kSched = 4;   // depth of the ring that announces work items
 constexpr int kThreads = 512;
-constexpr int kOutWarp0 = 8, kMmaWarp0 = 12, kTmaWarp = 14;
-constexpr int kItemReaders = 14;  // warps that read every announced item (all but the scheduler and the idle one)
+constexpr int kOutWarp0 = 8, kPvWarp0 = 12, kTmaWarp = 14, kQkWarp = 15;
+constexpr int kItemReaders = 15;  // warps that read every announced item (all but the scheduler)
 // registers per thread after setmaxnreg; the sum over the 16 warps must fit what the CTA was launched with
 #ifndef XFB_PST_REGS_SOFTMAX
-#define XFB_PST_REGS_SOFTMAX 176
+#define XFB_PST_REGS_SOFTMAX 184
 #endif
 #ifndef XFB_PST_REGS_OUT
-#define XFB_PST_REGS_OUT 80
+#define XFB_PST_REGS_OUT 64
 #endif
 #ifndef XFB_PST_REGS_AUX
 #define XFB_PST_REGS_AUX 80
@@ -114,10 +113,11 @@ struct __align__(8) Barriers {
   uint64_t sched_full[kSched], sched_empty[kSched];
   uint64_t q_full[kTiles], q_empty[kTiles];
   uint64_t k_full[kStages], v_full[kStages], k_empty[kStages], v_empty[kStages];
-  uint64_t s_full[kTiles], p_half[kTiles], p_full[kTiles];  // p_half: the probabilities of keys 64-127 are stored
+  uint64_t s_full[kTiles], s_empty;          // s_empty: the scores are in registers (the two tiles share one buffer)
+  uint64_t p_half[kTiles], p_full[kTiles];   // p_half: the probabilities of keys 0-63 are stored
+  uint64_t pv_done[kTiles];                  // P_t has been read, O_t is quiescent
   uint64_t o_full[kTiles], o_empty[kTiles];
   uint64_t stats_full[kTiles], stats_empty[kTiles];
-  uint64_t turn[kTiles];  // token of the tensor pipe: the two MMA warps issue their blocks alternately
   Item sched_item[kSched];
   uint32_t tmem_base;
   uint32_t abort_flag;
@@ -138,6 +138,16 @@ struct Smem {
   static constexpr int kTotalBiased = kTotal + 8 * kBiasUnit;
 };
 static_assert(sizeof(Barriers) <= 1024, "barrier block");
+
+// Columns of the tensor memory: scores (fp32, one buffer in which the two tiles take turns), probabilities (16-bit pairs), output
+// (fp32).  At D = 128 these are all 512 columns; at D = 64 a buffer of scores per tile would fit, but then nothing keeps the
+// tiles half a step apart (4 x 4096 rows, 32 heads, no mask: 778 us with two buffers, 664 with one).
+template <int D>
+struct Tmem {
+  static constexpr uint32_t kS = 0;
+  __device__ static constexpr uint32_t p(int t) { return kBN + t * (kBN / 2); }
+  __device__ static constexpr uint32_t o(int t) { return 2 * kBN + t * D; }
+};
 
 // Packed fp32 pairs live in 64-bit registers; building and splitting them with
 // mov.b64 keeps everything in registers (no address-taken locals).
@@ -191,9 +201,9 @@ __device__ __forceinline__ uint32_t pack_pair(float lo, float hi) {
 }
 
 #ifdef XFB_PST_PROFILE
-// Timing build only: per-CTA cycle counters of the softmax warps (8 slots each, 0-63) and, with
-// -DXFB_PST_PROFILE_MMA, of the two MMA issuers (64-79 / 80-95), read back with xfb200_debug_read_prefill_profile.
-__device__ long long g_prof[160][96];
+// Timing build only: per-CTA cycle counters of the softmax warps (16 slots each, 0-127) and of the two MMA issuers
+// (128-143 / 144-159), read back with xfb200_debug_read_prefill_profile.
+__device__ long long g_prof[160][160];
 #define XFB_PROF_DECL(n) long long prof_acc[n] = {0}; long long prof_t = clock64();
 #define XFB_PROF_LAP(k) { const long long _n = clock64(); prof_acc[k] += _n - prof_t; prof_t = _n; }
 #define XFB_PROF_COUNT(k) { prof_acc[k] += 1; }
@@ -202,7 +212,7 @@ __device__ long long g_prof[160][96];
 #define XFB_PROF_DECL(n)
 #define XFB_PROF_LAP(k)
 #define XFB_PROF_COUNT(k)
-#define XFB_PROF_STORE(base, n)
+#define XFB_PROF_STORE(base, n) {}
 #endif
 
 // Records the first code a launch gives up with (kept until the host reads it) and marks the
@@ -306,6 +316,7 @@ constexpr int kExact = 0, kPadded = 1, kBiased = 2, kBiasedSame = 3;
 template <int D, bool kBf16, int kVariant>
 __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(const __grid_constant__ Sm100Args a) {
   using L = Smem<D>;
+  using T = Tmem<D>;
   constexpr bool kPad = kVariant != kExact, kBias = kVariant == kBiased || kVariant == kBiasedSame, kBiasSame = kVariant == kBiasedSame;
   constexpr int kHalves = D / 64;
   extern __shared__ uint8_t smem_dyn[];
@@ -313,7 +324,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
   Barriers* bar = reinterpret_cast<Barriers*>(smem + L::kBar);
   float2* stats = reinterpret_cast<float2*>(smem + L::kStats);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int n_items = a.q_tiles * a.groups * a.heads_per_group * a.batch;
   const long long budget = a.wait_budget;
   const int head_dim = kPad ? a.head_dim : D;
@@ -329,9 +340,9 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
       }
       for (int i = 0; i < kStages; ++i) {
         mbar_init(&bar->k_full[i], 1);
-        mbar_init(&bar->k_empty[i], kTiles);  // released by both MMA warps
+        mbar_init(&bar->k_empty[i], 1);
         mbar_init(&bar->v_full[i], 1);
-        mbar_init(&bar->v_empty[i], kTiles);
+        mbar_init(&bar->v_empty[i], kTiles);  // released by both PV warps
       }
       for (int t = 0; t < kTiles; ++t) {
         mbar_init(&bar->q_full[t], 1);
@@ -339,16 +350,17 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
         mbar_init(&bar->s_full[t], 1);
         mbar_init(&bar->p_half[t], 4);  // one arrival per softmax warp of the tile
         mbar_init(&bar->p_full[t], 4);
+        mbar_init(&bar->pv_done[t], 1);
         mbar_init(&bar->o_full[t], 1);
         mbar_init(&bar->o_empty[t], 128);
         mbar_init(&bar->stats_full[t], 128);
         mbar_init(&bar->stats_empty[t], 128);
-        mbar_init(&bar->turn[t], 1);
       }
+      mbar_init(&bar->s_empty, 4);
       bar->abort_flag = 0;
       mbar_fence_init();
     }
-    if (warp == kMmaWarp0) {
+    if (warp == kQkWarp) {
       tmem_alloc(&bar->tmem_base, 512);
       tmem_relinquish();
     }
@@ -378,22 +390,23 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
       return idx;
     };
 
-    if (warp >= kMmaWarp0) {
+    if (warp >= kPvWarp0) {
       asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsAux));
       if (warp == kTmaWarp) {
         // ============================================ scheduler + TMA producer
-        // Lane 0 waits and issues; all lanes run the loop, because pulling an item (a broadcast)
-        // and writing the rows of an item without visible keys are done by the whole warp.
-        if (lane == 0) {
+        // All lanes run the loop, because pulling an item (a broadcast) and writing the rows of an item without
+        // visible keys are done by the whole warp; one lane issues the copies.
+        if (elect_one()) {
           prefetch_tensormap(&a.tm_q);
           prefetch_tensormap(&a.tm_k);
           prefetch_tensormap(&a.tm_v);
         }
         const int order = sequence_order(a, lane);
-        int seq = 0;              // items announced
-        int kstep = 0;            // K/V steps loaded, over all items
-        int aq[kTiles] = {0, 0};  // items in which tile t took part so far
-        bool ok = true;
+        int seq = 0;           // items announced
+        int ks = 0, kph = 1;   // K stage / parity its release is waited for with
+        int vs = 0, vph = 1;
+        uint32_t qph = 3;      // parities of the two Q buffers
+        int code = 0;
         // Pulls item numbers until one has key steps.  Row blocks past the end of their sequence are
         // skipped; blocks whose rows see no key at all get their result here: zeros and -inf.
         auto next_item = [&](Item& it) {
@@ -412,6 +425,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
             const int chunks = head_dim * osz / 16;
             uint8_t* ob = reinterpret_cast<uint8_t*>(a.out);
             const int64_t base = int64_t(it.tb) * a.os.b + int64_t(it.q_row0 + it.m0) * a.os.m + int64_t(it.g) * a.os.g + int64_t(it.h) * a.os.h;
+#pragma unroll 1
             for (int i = lane; i < nrows * chunks; i += 32) {
               const int r = i / chunks, c = i % chunks;
               *reinterpret_cast<uint4*>(ob + (base + int64_t(r) * a.os.m) * osz + c * 16) = make_uint4(0, 0, 0, 0);
@@ -419,75 +433,79 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
             if (a.lse != nullptr) {
               const int64_t lo = a.seqstart_q != nullptr ? int64_t(it.g) * a.lse_g + int64_t(it.h) * a.lse_h + it.q_row0 + it.m0
                                                          : int64_t(it.b) * a.lse_b + int64_t(it.g) * a.lse_g + int64_t(it.h) * a.lse_h + it.m0;
+#pragma unroll 1
               for (int r = lane; r < nrows; r += 32) a.lse[lo + r] = -INFINITY;
             }
           }
         };
-        Item cur, nxt;
-        next_item(cur);
-        while (ok) {
-          const int slot = seq % kSched;
-          if (lane == 0) {
-            if (seq >= kSched && !mbar_wait(&bar->sched_empty[slot], (seq / kSched - 1) & 1, abort_flag, budget)) {
-              give_up(a, 10);
-              ok = false;
-            } else {
-              bar->sched_item[slot] = cur;
-              mbar_arrive(&bar->sched_full[slot]);  // (release: the descriptor is visible to whoever sees the phase)
-            }
+        // one tile of 128 rows (Q, K or V), as blocks of 64 columns
+        auto load_tile = [&](int at, const CUtensorMap* tm, uint64_t* full, int head, int row, int tb) {
+          if (elect_one()) {
+            mbar_expect_tx(full, L::kKV);
+#pragma unroll
+            for (int hf = 0; hf < kHalves; ++hf) tma_load_4d(smem + at + hf * kHalfBytes, tm, full, hf * 64, head, row, tb);
           }
-          ok = __shfl_sync(0xffffffffu, int(ok), 0) != 0;
+        };
+        // The V tile of a step is loaded behind the K tile of the step after it: its stage comes free a softmax later
+        // than the K stage, which must not wait for that.
+        int pend_row = -1, pend_head = 0, pend_tb = 0;
+        auto load_pending_v = [&]() -> bool {
+          if (pend_row < 0) return true;
+          if (!mbar_wait(&bar->v_empty[vs], vph, abort_flag, budget)) {
+            code = 12;
+            return false;
+          }
+          load_tile(L::kV + vs * L::kKV, &a.tm_v, &bar->v_full[vs], pend_head, pend_row, pend_tb);
+          if (++vs == kStages) vs = 0, vph ^= 1;
+          pend_row = -1;
+          return true;
+        };
+        Item cur;
+        next_item(cur);
+        while (true) {
+          const int slot = seq % kSched;
+          if (!mbar_wait(&bar->sched_empty[slot], ((seq / kSched) & 1) ^ 1, abort_flag, budget)) {
+            code = 10;
+            break;
+          }
+          if (lane == 0) {
+            bar->sched_item[slot] = cur;
+            mbar_arrive(&bar->sched_full[slot]);  // (release: the descriptor is visible to whoever sees the phase)
+          }
           ++seq;
-          if (!ok || cur.idx < 0) break;
-          // Loads are issued in the order in which what they wait for comes free at the end of the previous
-          // item: the K tile of the first step (its stage is released one step before the end), Q of tile 0,
-          // the V tile of the first step, Q of tile 1, then the remaining steps.  A Q load that waited for
-          // the very last QK of the previous item must not hold back the first K tile.
-          auto load_q = [&](int t) {
-            if (!ok || (t == 0 ? cur.jhi[0] <= cur.jlo[0] : cur.jhi[1] <= cur.jlo[1])) return;
-            if (aq[t] > 0 && !mbar_wait(&bar->q_empty[t], (aq[t] - 1) & 1, abort_flag, budget)) {
-              give_up(a, 13);
-              ok = false;
-              return;
-            }
-            ++aq[t];
-            mbar_expect_tx(&bar->q_full[t], L::kQTile);
-#pragma unroll
-            for (int hf = 0; hf < kHalves; ++hf)
-              tma_load_4d(smem + L::kQ + t * L::kQTile + hf * kHalfBytes, &a.tm_q, &bar->q_full[t], hf * 64, cur.head,
-                          cur.q_row0 + cur.m0 + t * kBM, cur.tb);
-          };
+          if (cur.idx < 0) {
+            load_pending_v();
+            break;
+          }
+          Item nxt;
           bool have_next = false;
-          for (int j = cur.j_begin; j < cur.j_end; ++j, ++kstep) {
-            if (lane == 0 && ok) {
-              const int st = kstep % kStages, use = kstep / kStages;
-              const int row = cur.k_row0 + cur.n_base + j * kBN;
-              if (use > 0 && !mbar_wait(&bar->k_empty[st], (use - 1) & 1, abort_flag, budget)) {
-                give_up(a, 11);
-                ok = false;
-              }
-              // (testing aid: the CTA that got the first item leaves out its last key tile, so that the wait for it runs out)
-              if (ok && !((a.debug_flags & 1) && cur.idx == 0 && j == cur.j_end - 1)) {
-                mbar_expect_tx(&bar->k_full[st], L::kKV);
-#pragma unroll
-                for (int hf = 0; hf < kHalves; ++hf)
-                  tma_load_4d(smem + L::kK + st * L::kKV + hf * kHalfBytes, &a.tm_k, &bar->k_full[st], hf * 64, cur.kv_head, row, cur.tb);
-              }
-              if (j == cur.j_begin) load_q(0);
-              if (ok && use > 0 && !mbar_wait(&bar->v_empty[st], (use - 1) & 1, abort_flag, budget)) {
-                give_up(a, 12);
-                ok = false;
-              }
-              if (ok) {
-                mbar_expect_tx(&bar->v_full[st], L::kKV);
-#pragma unroll
-                for (int hf = 0; hf < kHalves; ++hf)
-                  tma_load_4d(smem + L::kV + st * L::kKV + hf * kHalfBytes, &a.tm_v, &bar->v_full[st], hf * 64, cur.kv_head, row, cur.tb);
-              }
-              if (j == cur.j_begin) load_q(1);
+#pragma unroll 1
+          for (int j = cur.j_begin; j < cur.j_end; ++j) {
+            const int row = cur.k_row0 + cur.n_base + j * kBN;
+            if (!mbar_wait(&bar->k_empty[ks], kph, abort_flag, budget)) {
+              code = 11;
+              break;
             }
-            ok = __shfl_sync(0xffffffffu, int(ok), 0) != 0;
-            if (!ok) break;
+            // (testing aid: the CTA that got the first item leaves out its last key tile, so that the wait for it runs out)
+            if (!((a.debug_flags & 1) && cur.idx == 0 && j == cur.j_end - 1))
+              load_tile(L::kK + ks * L::kKV, &a.tm_k, &bar->k_full[ks], cur.kv_head, row, cur.tb);
+            if (++ks == kStages) ks = 0, kph ^= 1;
+            if (!load_pending_v()) break;
+            if (j == cur.j_begin) {
+              // Q behind what does not wait for it: its buffers come free with the very last QK^T of the previous item
+#pragma unroll 1
+              for (int t = 0; t < kTiles; ++t) {
+                if (t == 0 ? cur.jhi[0] <= cur.jlo[0] : cur.jhi[1] <= cur.jlo[1]) continue;
+                if (!mbar_wait(&bar->q_empty[t], (qph >> t) & 1, abort_flag, budget)) {
+                  code = 13;
+                  break;
+                }
+                qph ^= 1u << t;
+                load_tile(L::kQ + t * L::kQTile, &a.tm_q, &bar->q_full[t], cur.head, cur.q_row0 + cur.m0 + t * kBM, cur.tb);
+              }
+              if (code != 0) break;
+            }
+            pend_row = row, pend_head = cur.kv_head, pend_tb = cur.tb;
             // The first two steps fit the rings at once; from here on every load waits for a stage to
             // come free, so this is the moment to pull the next item: its latency costs nothing.
             if (!have_next && (j == cur.j_begin + 1 || j == cur.j_end - 1)) {
@@ -495,33 +513,20 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
               have_next = true;
             }
           }
-          if (!ok) break;
+          if (code != 0) break;
           cur = nxt;
         }
-        if (!ok) *abort_flag = 1;
-      } else if (warp == kMmaWarp0 || warp == kMmaWarp0 + 1) {
-        // ================================================= MMA issuer of tile t
-        // tcgen05.mma is issued almost synchronously (the queue in front of the
-        // tensor pipe is about one instruction deep), so every clock this lane
-        // spends on anything else -- a satisfied mbarrier wait alone costs ~90 --
-        // is a clock the tensor pipe idles.  Hence one issuing warp per query tile:
-        // while one waits for its softmax, the other keeps the pipe fed.
-#if !defined(XFB_PST_PROFILE_MMA)
-#define XFB_MPROF_DECL(n)
-#define XFB_MPROF_LAP(k)
-#define XFB_MPROF_COUNT(k)
-#define XFB_MPROF_STORE(b, n)
-#else
-#define XFB_MPROF_DECL(n) XFB_PROF_DECL(n)
-#define XFB_MPROF_LAP(k) XFB_PROF_LAP(k)
-#define XFB_MPROF_COUNT(k) XFB_PROF_COUNT(k)
-#define XFB_MPROF_STORE(b, n) XFB_PROF_STORE(b, n)
-#endif
-        const int t = warp - kMmaWarp0;
-        constexpr uint32_t idesc_qk = umma_idesc(kBM, kBN, kBf16, false, false);
-        // (a padded head dim: QK^T in steps of 16 columns, PV in a width that is a multiple of 16)
-        const uint32_t idesc_pv = umma_idesc(kBM, kPad ? (head_dim + 15) / 16 * 16 : D, kBf16, false, true);
-        const int qk_steps = kPad ? (head_dim + 15) / 16 : D / 16;
+        if (code != 0) {
+          if (lane == 0) give_up(a, code);
+          *abort_flag = 1;
+        }
+      } else {
+        // ====================================================== MMA issuers
+        // Warp 15 issues every QK^T, warps 12 and 13 the PV of tile 0 and 1.  A thread that issues tcgen05.mma stands still
+        // while two or so are ahead of it in the tensor pipe, and for some 140 clocks at every commit; what one of the
+        // three warps loses in that way, or in a wait, the others fill.  Their code is kept small (one copy for both
+        // tiles, short loops): it shares the instruction cache with the softmax.
+        XFB_PROF_DECL(16)
         // Shared-memory descriptors: the upper word is constant (stride between
         // 8-row groups = 1024 B, version 1, 128B swizzle); the lower word holds
         // (address >> 4) and the leading-dimension offset, so stepping through a
@@ -532,289 +537,229 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(kDescHi));
           return d;
         };
-        const uint32_t q_lo = (smem_u32(smem + L::kQ + t * L::kQTile) >> 4) | (1u << 16);
-        const uint32_t k_lo0 = (smem_u32(smem + L::kK) >> 4) | (1u << 16);
-        const uint32_t v_lo0 = (smem_u32(smem + L::kV) >> 4) | ((kHalfBytes >> 4) << 16);
-        const uint32_t tmem_s = tmem + t * 128, tmem_o = tmem + 256 + t * 128;
-        auto issue_qk_part = [&](int k_stage, int kk_lo, int kk_hi) {
-          const uint32_t kl = k_lo0 + k_stage * (L::kKV >> 4);
-#pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) {
-            if (kk < kk_lo || kk >= kk_hi || (kPad && kk >= qk_steps)) continue;
-            const uint32_t off = ((kk / 4) * kHalfBytes + (kk % 4) * 32) >> 4;
-            umma_ss(tmem_s, desc(q_lo + off), desc(kl + off), idesc_qk, kk > 0);
-          }
-        };
-        // the part of P_t V_j over keys [16 kk_lo, 16 kk_hi) of the step; `accumulate` false: its first product overwrites O_t
-        auto issue_pv = [&](int v_stage, int kk_lo, int kk_hi, bool accumulate) {
-          const uint32_t vl = v_lo0 + v_stage * (L::kKV >> 4);
-#pragma unroll
-          for (int kk = 0; kk < kBN / 16; ++kk) {
-            if (kk < kk_lo || kk >= kk_hi) continue;
-            // A = P_t: packed 16-bit pairs, 8 columns of tensor memory per 16 keys
-            // (the pairs of keys 0-63 sit in columns 96-127, those of keys 64-127 in columns 64-95)
-            umma_ts(tmem_o, tmem_s + (kk < 4 ? 96 + kk * 8 : 32 + kk * 8), desc(vl + ((kk * 16 * 128) >> 4)), idesc_pv, (accumulate || kk > kk_lo) ? 1u : 0u);
-          }
-        };
-
-        int seq = 0;
-        bool ok = true;
-        // what this warp needs to know about an item: its key steps, the ones its tile takes part in, the sequence end
-        struct Steps {
-          int j_begin, j_end, jlo, jhi, n_base, klen;
-        };
-        Steps cur, nxt;
-        auto pop_with_steps = [&](Steps& st) -> int {
-          return pop_item(seq, [&](const Item& it) {
-            st.j_begin = it.j_begin, st.j_end = it.j_end, st.n_base = it.n_base, st.klen = it.klen;
-            st.jlo = t == 0 ? it.jlo[0] : it.jlo[1];
-            st.jhi = t == 0 ? it.jhi[0] : it.jhi[1];
-          });
-        };
-        int ci = pop_with_steps(cur);
-        if (ci == -2) {
-          if (lane == 0) give_up(a, 20);
-          ok = false;
-        }
-        if (ci >= 0) {
-          int j = cur.j_begin;
-          int ks = 0, kph = 0;  // K stage / phase of step (cur, j)
-          int vs = 0, vph = 0;  // V stage / phase of step (cur, j)
-          int cnt = 0;          // products of this query tile so far, over all items
-          int kq = 0;           // items whose first QK of this tile has been issued
-          int kp = 0;           // items whose last PV of this tile has been issued
-          int turn_ph = 0;
-          XFB_MPROF_DECL(16)
-          {
-            // the very first step: nothing to multiply by V yet
-            const bool act = j >= cur.jlo && j < cur.jhi;
-            if (act) ok = mbar_wait(&bar->q_full[t], 0, abort_flag, budget);
-            ok = ok && mbar_wait(&bar->k_full[0], 0, abort_flag, budget);
-            if (!ok && lane == 0) give_up(a, 21);
-            if (ok) {
-              tc_fence_after();
-              if (lane == 0) {
-                if (act) {
-                  issue_qk_part(0, 0, D / 16);
-                  tc_commit(&bar->s_full[t]);
-                  if (j == cur.jhi - 1) tc_commit(&bar->q_empty[t]);
+        int seq = 0, code = 0;
+        int st = 0, ph = 0;  // K (or V) stage / phase of the step
+        if (warp == kQkWarp) {
+          constexpr uint32_t idesc_qk = umma_idesc(kBM, kBN, kBf16, false, false);
+          // (a padded head dim: steps of 16 columns as far as it goes)
+          const int qk_steps = kPad ? (head_dim + 15) / 16 : D / 16;
+          const uint32_t q_lo = (smem_u32(smem + L::kQ) >> 4) | (1u << 16);
+          const uint32_t k_lo = (smem_u32(smem + L::kK) >> 4) | (1u << 16);
+          uint32_t sph = 1, qph = 0;  // parities: buffer of the scores (released), Q tiles (loaded)
+          while (code == 0) {
+            int j, j_end, jlo0, jhi0, jlo1, jhi1;
+            const int idx = pop_item(seq, [&](const Item& d) {
+              j = d.j_begin, j_end = d.j_end;
+              jlo0 = d.jlo[0], jhi0 = d.jhi[0], jlo1 = d.jlo[1], jhi1 = d.jhi[1];
+            });
+            if (idx < 0) {
+              if (idx == -2) code = 20;
+              break;
+            }
+#pragma unroll 1
+            for (; j < j_end; ++j) {
+              if (!mbar_wait(&bar->k_full[st], ph, abort_flag, budget)) {
+                code = 21;
+                break;
+              }
+              XFB_PROF_LAP(1)  // wait for K
+#pragma unroll 1
+              for (int t = 0; t < kTiles; ++t) {
+                const int jlo = t == 0 ? jlo0 : jlo1, jhi = t == 0 ? jhi0 : jhi1;
+                if (j < jlo || j >= jhi) continue;
+                bool ok = true;
+                if (j == jlo) {
+                  ok = mbar_wait(&bar->q_full[t], (qph >> t) & 1, abort_flag, budget);
+                  qph ^= 1u << t;
                 }
-                tc_commit(&bar->k_empty[0]);
-                if (t == 1) mbar_arrive(&bar->turn[0]);  // tile 0 opens every iteration
-              }
-              if (act) ++kq;
-            }
-          }
-          while (ok) {
-            XFB_MPROF_LAP(0)
-            // ---- the step after (cur, j): same item, or the first step of the next item with steps
-            bool has_next = true, same_item = true;
-            int nj = j + 1;
-            if (nj >= cur.j_end) {
-              same_item = false;
-              const int ni = pop_with_steps(nxt);
-              if (ni == -2) {
-                if (lane == 0) give_up(a, 20);
-                ok = false;
-                break;
-              }
-              has_next = ni >= 0;
-              nj = nxt.j_begin;
-            }
-            XFB_MPROF_LAP(1)  // pulling the next item
-            const int nx_jlo = same_item ? cur.jlo : nxt.jlo, nx_jhi = same_item ? cur.jhi : nxt.jhi;
-            const bool act = j >= cur.jlo && j < cur.jhi;
-            const bool act_next = has_next && nj >= nx_jlo && nj < nx_jhi;
-            const bool first_qk_next = act_next && nj == nx_jlo;
-            int ks1 = ks + 1, kph1 = kph;
-            if (ks1 == kStages) ks1 = 0, kph1 ^= 1;
-            ok = mbar_wait(&bar->v_full[vs], vph, abort_flag, budget);
-            if (ok && has_next) ok = mbar_wait(&bar->k_full[ks1], kph1, abort_flag, budget);
-            if (!ok) {
-              if (lane == 0) give_up(a, 22);
-              break;
-            }
-            // The first QK of the next item needs its Q tile.  If that has not landed yet, the token is not
-            // held back for it: the block ends after the PV and the QK follows out of turn (late_qk).
-            XFB_MPROF_LAP(2)  // waits for V and the next K
-            bool late_qk = false;
-            if (first_qk_next) {
-              int ready = 0;
-              if (lane == 0) ready = mbar_try_wait(&bar->q_full[t], kq & 1) ? 1 : 0;
-              late_qk = __shfl_sync(0xffffffffu, ready, 0) == 0;
-            }
-            const int n0 = cur.n_base + j * kBN;
-            if (n0 + kBN > cur.klen) {
-              // V rows past the end of the sequence may hold anything; P is 0 there.
-              // Both MMA warps write the same zeros: no ordering between them is needed.
-              const int first = max(cur.klen - n0, 0);
-              uint8_t* vt = smem + L::kV + vs * L::kKV;
-              for (int hf = 0; hf < kHalves; ++hf)
-                for (int i = first * 8 + lane; i < kBN * 8; i += 32) *reinterpret_cast<uint4*>(vt + hf * kHalfBytes + i * 16) = make_uint4(0, 0, 0, 0);
-              fence_proxy_async_smem();
-              __syncwarp();
-            }
-            // If both warps issued at will, their MMAs would interleave one by one,
-            // both tiles would finish together and both softmaxes would run at the
-            // same time with the tensor pipe idle.  Blocks (PV, next QK) are
-            // therefore issued alternately, which keeps the two tiles half a period
-            // apart; the token is passed a few MMAs before the end of a block so
-            // that the hand-over latency is hidden.  The token is waited for before
-            // P: it normally arrives first, and even a satisfied wait costs ~90 clocks
-            // that would otherwise sit between the softmax and its PV.
-            ok = mbar_wait(&bar->turn[t], turn_ph, abort_flag, budget);
-            turn_ph ^= 1;
-            if (!ok) {
-              if (lane == 0) give_up(a, 25 + t);
-              break;
-            }
-            XFB_MPROF_LAP(4)  // wait for the token
-            if (act) {
-              // The probabilities of keys 64-127 are stored first: their half of the product runs while the
-              // softmax is still busy with keys 0-63.
-              ok = mbar_wait(&bar->p_half[t], cnt & 1, abort_flag, budget);
-              // the first PV of an item overwrites O_t: the output warps must have read the previous one
-              if (ok && j == cur.jlo && kp > 0) ok = mbar_wait(&bar->o_empty[t], (kp - 1) & 1, abort_flag, budget);
-              if (ok) {
+                // the scores that were here before have to be in registers
+                if (!ok || !mbar_wait(&bar->s_empty, sph, abort_flag, budget)) {
+                  code = 23 + t;
+                  break;
+                }
+                sph ^= 1;
                 tc_fence_after();
-                if (lane == 0) issue_pv(vs, kBN / 32, kBN / 16, j > cur.jlo);
-                ok = mbar_wait(&bar->p_full[t], cnt & 1, abort_flag, budget);
+                XFB_PROF_LAP(2)  // wait for Q, for the buffer of the scores
+                if (elect_one()) {
+                  uint32_t ql = q_lo + t * (L::kQTile >> 4), kl = k_lo + st * (L::kKV >> 4);
+#pragma unroll 1
+                  for (int hf = 0; hf < kHalves; ++hf) {
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+                      if (!kPad || hf * 4 + kk < qk_steps) umma_ss(tmem + T::kS, desc(ql + kk * 2), desc(kl + kk * 2), idesc_qk, kk > 0 ? 1u : uint32_t(hf));
+                    ql += kHalfBytes >> 4, kl += kHalfBytes >> 4;
+                  }
+                  tc_commit(&bar->s_full[t]);
+                  if (j == jhi - 1) tc_commit(&bar->q_empty[t]);
+                }
+                __syncwarp();
+                XFB_PROF_LAP(3)  // QK^T issued
+                XFB_PROF_COUNT(7)
               }
-              if (!ok) {
-                if (lane == 0) give_up(a, 23 + t);
-                break;
-              }
-              tc_fence_after();
+              if (code != 0) break;
+              if (elect_one()) tc_commit(&bar->k_empty[st]);
+              if (++st == kStages) st = 0, ph ^= 1;
             }
-            XFB_MPROF_LAP(3)  // V tail, wait for P (and for the output warps at the first PV of an item)
-            if (lane == 0) {
-              if (act) {
-                issue_pv(vs, 0, kBN / 32, true);
-                if (j == cur.jhi - 1) tc_commit(&bar->o_full[t]);
-              }
-              tc_commit(&bar->v_empty[vs]);
-              if (act_next && !late_qk) {
-                issue_qk_part(ks1, 0, D / 32);
-                mbar_arrive(&bar->turn[1 - t]);
-                issue_qk_part(ks1, D / 32, D / 16);
-                tc_commit(&bar->s_full[t]);
-                if (nj == nx_jhi - 1) tc_commit(&bar->q_empty[t]);
-              } else {
-                mbar_arrive(&bar->turn[1 - t]);
-              }
-              if (has_next && !late_qk) tc_commit(&bar->k_empty[ks1]);
-            }
-            XFB_MPROF_LAP(5)  // issuing the block
-            if (late_qk) {
-              XFB_MPROF_COUNT(8)
-              ok = mbar_wait(&bar->k_full[ks1], kph1, abort_flag, budget);
-              if (ok && first_qk_next) ok = mbar_wait(&bar->q_full[t], kq & 1, abort_flag, budget);
-              if (!ok) {
-                if (lane == 0) give_up(a, 27 + t);
-                break;
-              }
-              tc_fence_after();
-              if (lane == 0) {
-                issue_qk_part(ks1, 0, D / 16);
-                tc_commit(&bar->s_full[t]);
-                if (nj == nx_jhi - 1) tc_commit(&bar->q_empty[t]);
-                tc_commit(&bar->k_empty[ks1]);
-              }
-            }
-            XFB_MPROF_LAP(6)  // a QK issued out of turn
-            XFB_MPROF_COUNT(7)
-            if (act) {
-              ++cnt;
-              if (j == cur.jhi - 1) ++kp;
-            }
-            if (first_qk_next) ++kq;
-            if (!has_next) break;
-            if (!same_item) cur = nxt;
-            j = nj;
-            ks = ks1, kph = kph1;
-            if (++vs == kStages) vs = 0, vph ^= 1;
           }
-          XFB_MPROF_STORE(64 + t * 16, 16)
+        } else {
+          const int t = warp - kPvWarp0;
+          // (a padded head dim: a width that is a multiple of 16)
+          const uint32_t idesc_pv = umma_idesc(kBM, kPad ? (head_dim + 15) / 16 * 16 : D, kBf16, false, true);
+          const uint32_t v_lo = (smem_u32(smem + L::kV) >> 4) | ((kHalfBytes >> 4) << 16);
+          const uint32_t tp = tmem + T::p(t), to = tmem + T::o(t);
+          int cnt = 0, items = 0;  // products, items of this tile so far
+          while (code == 0) {
+            int j, j_end, jlo, jhi, n_base, klen;
+            const int idx = pop_item(seq, [&](const Item& d) {
+              j = d.j_begin, j_end = d.j_end, n_base = d.n_base, klen = d.klen;
+              jlo = d.jlo[t], jhi = d.jhi[t];
+            });
+            if (idx < 0) {
+              if (idx == -2) code = 20;
+              break;
+            }
+#pragma unroll 1
+            for (; j < j_end; ++j) {
+              if (!mbar_wait(&bar->v_full[st], ph, abort_flag, budget)) {
+                code = 22;
+                break;
+              }
+              XFB_PROF_LAP(1)  // wait for V
+              if (j >= jlo && j < jhi) {
+                const int n0 = n_base + j * kBN;
+                if (n0 + kBN > klen) {
+                  // V rows past the end of the sequence may hold anything; P is 0 there.
+                  // Both PV warps write the same zeros: no ordering between them is needed.
+                  const int first = max(klen - n0, 0);
+                  uint8_t* vt = smem + L::kV + st * L::kKV;
+#pragma unroll 1
+                  for (int hf = 0; hf < kHalves; ++hf)
+#pragma unroll 1
+                    for (int i = first * 8 + lane; i < kBN * 8; i += 32) *reinterpret_cast<uint4*>(vt + hf * kHalfBytes + i * 16) = make_uint4(0, 0, 0, 0);
+                  fence_proxy_async_smem();
+                  __syncwarp();
+                }
+                // the first product of an item overwrites O_t: the output warps must have read the previous one
+                if (j == jlo && !mbar_wait(&bar->o_empty[t], (items++ & 1) ^ 1, abort_flag, budget)) {
+                  code = 25 + t;
+                  break;
+                }
+                // The first half of the product runs while the softmax is still busy with the second half of P.
+                uint32_t vl = v_lo + st * (L::kKV >> 4), pt = tp;
+#pragma unroll 1
+                for (int half = 0; half < 2; ++half) {
+                  if (!mbar_wait(half == 0 ? &bar->p_half[t] : &bar->p_full[t], cnt & 1, abort_flag, budget)) {
+                    code = 27 + t;
+                    break;
+                  }
+                  tc_fence_after();
+                  XFB_PROF_LAP(2 + 2 * half)  // wait for a half of P
+                  if (elect_one()) {
+#pragma unroll
+                    for (int kk = 0; kk < kBN / 32; ++kk)  // A = P_t: packed 16-bit pairs, 8 columns of tensor memory per 16 keys
+                      umma_ts(to, pt + kk * 8, desc(vl + ((kk * 16 * 128) >> 4)), idesc_pv, kk > 0 ? 1u : uint32_t(j > jlo || half > 0));
+                    if (half > 0) {
+                      tc_commit(&bar->pv_done[t]);
+                      if (j == jhi - 1) tc_commit(&bar->o_full[t]);
+                    }
+                  }
+                  __syncwarp();
+                  XFB_PROF_LAP(3 + 2 * half)  // half of PV issued
+                  vl += (64 * 128) >> 4, pt += 32;
+                }
+                if (code != 0) break;
+                ++cnt;
+                XFB_PROF_COUNT(7)
+              }
+              if (elect_one()) tc_commit(&bar->v_empty[st]);
+              if (++st == kStages) st = 0, ph ^= 1;
+            }
+          }
         }
-        if (!ok) *abort_flag = 1;
+        if (warp != kPvWarp0 + 1) XFB_PROF_STORE(128 + (warp == kQkWarp ? 0 : 16), 16)
+        if (code != 0) {
+          if (lane == 0) give_up(a, code);
+          *abort_flag = 1;
+        }
       }
     } else if (warp >= kOutWarp0) {
       asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOut));
       // ================================================================ output
       const int row = (warp & 3) * 32 + lane;  // TMEM lane == row inside the tile
       const uint32_t lane_sel = uint32_t((warp & 3) * 32) << 16;
-      int seq = 0;
-      int ko[kTiles] = {0, 0};  // items in which tile t took part so far
-      bool ok = true;
-      while (ok) {
-        Item it;
-        const int idx = pop_item(seq, [&](const Item& d) { it = d; });
+      int seq = 0, code = 0;
+      uint32_t oph = 0;  // parities of the two tiles
+      while (code == 0) {
+        struct {
+          int b, tb, g, h, q_row0, m0, qlen, jlo0, jhi0, jlo1, jhi1;
+        } it;
+        const int idx = pop_item(seq, [&](const Item& d) {
+          it.b = d.b, it.tb = d.tb, it.g = d.g, it.h = d.h, it.q_row0 = d.q_row0, it.m0 = d.m0, it.qlen = d.qlen;
+          it.jlo0 = d.jlo[0], it.jhi0 = d.jhi[0], it.jlo1 = d.jlo[1], it.jhi1 = d.jhi[1];
+        });
         if (idx < 0) {
-          if (idx == -2) {
-            give_up(a, 40);
-            ok = false;
-          }
+          if (idx == -2) code = 40;
           break;
         }
-#pragma unroll
+#pragma unroll 1
         for (int t = 0; t < kTiles; ++t) {
           const int i_loc = it.m0 + t * kBM + row;
           const bool valid_row = i_loc < it.qlen;
-          const bool active = it.jhi[t] > it.jlo[t];
+          const bool active = t == 0 ? it.jhi0 > it.jlo0 : it.jhi1 > it.jlo1;
           if (!active && it.m0 + t * kBM >= it.qlen) continue;  // no row of this tile exists
           float m_run = -INFINITY, l_run = 0.f;
-          const uint32_t tmem_o = tmem + 256 + t * 128 + lane_sel;
+          const uint32_t tmem_o = tmem + T::o(t) + lane_sel;
           if (active) {
-            const int k = ko[t]++;
-            ok = mbar_wait(&bar->stats_full[t], k & 1, abort_flag, budget);
+            bool ok = mbar_wait(&bar->stats_full[t], (oph >> t) & 1, abort_flag, budget);
             if (ok) {
               const float2 st = stats[t * kBM + row];
               m_run = st.x, l_run = st.y;
               mbar_arrive(&bar->stats_empty[t]);
-              ok = mbar_wait(&bar->o_full[t], k & 1, abort_flag, budget);
+              ok = mbar_wait(&bar->o_full[t], (oph >> t) & 1, abort_flag, budget);
             }
             if (!ok) {
-              give_up(a, 41 + t);
+              code = 41 + t;
               break;
             }
+            oph ^= 1u << t;
             tc_fence_after();
           }
           const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
           const int64_t o_off = int64_t(it.tb) * a.os.b + int64_t(it.q_row0 + i_loc) * a.os.m + int64_t(it.g) * a.os.g + int64_t(it.h) * a.os.h;
-#pragma unroll
-          for (int cblk = 0; cblk < D / 32; ++cblk) {
-            uint32_t orr[32];
+#pragma unroll 1
+          for (int col = 0; col < D; col += 16) {
+            uint32_t orr[16];
             if (active) {
-              XFB_TMEM_LD_32(tmem_o + cblk * 32, orr);
-              XFB_TMEM_WAIT_LD_32(orr);
-              if (cblk == D / 32 - 1) {
+              XFB_TMEM_LD_16(tmem_o + col, orr);
+              XFB_TMEM_WAIT_LD_16(orr);
+              if (col == D - 16) {
                 // O_t is in registers: the next item's first PV may overwrite it
                 tc_fence_before();
                 mbar_arrive(&bar->o_empty[t]);
               }
             } else {
 #pragma unroll
-              for (int i = 0; i < 32; ++i) orr[i] = 0;
+              for (int i = 0; i < 16; ++i) orr[i] = 0;
             }
             if (valid_row) {
               if (a.out_dtype == XFB200_F32) {
-                float* dst = reinterpret_cast<float*>(a.out) + o_off + cblk * 32;
+                float* dst = reinterpret_cast<float*>(a.out) + o_off + col;
 #pragma unroll
-                for (int i = 0; i < 32; i += 4)
-                  if (!kPad || cblk * 32 + i < head_dim)
+                for (int i = 0; i < 16; i += 4)
+                  if (!kPad || col + i < head_dim)
                     *reinterpret_cast<float4*>(dst + i) = make_float4(__uint_as_float(orr[i]) * inv, __uint_as_float(orr[i + 1]) * inv,
                                                                       __uint_as_float(orr[i + 2]) * inv, __uint_as_float(orr[i + 3]) * inv);
               } else {
-                uint16_t* dst = reinterpret_cast<uint16_t*>(a.out) + o_off + cblk * 32;
+                uint16_t* dst = reinterpret_cast<uint16_t*>(a.out) + o_off + col;
 #pragma unroll
-                for (int i = 0; i < 32; i += 8) {
+                for (int i = 0; i < 16; i += 8) {
                   uint32_t w[4];
 #pragma unroll
                   for (int e = 0; e < 4; ++e) {
                     const float x0 = __uint_as_float(orr[i + 2 * e]) * inv, x1 = __uint_as_float(orr[i + 2 * e + 1]) * inv;
                     w[e] = a.out_dtype == XFB200_BF16 ? pack_pair<true>(x0, x1) : pack_pair<false>(x0, x1);
                   }
-                  if (!kPad || cblk * 32 + i < head_dim) *reinterpret_cast<uint4*>(dst + i) = make_uint4(w[0], w[1], w[2], w[3]);
+                  if (!kPad || col + i < head_dim) *reinterpret_cast<uint4*>(dst + i) = make_uint4(w[0], w[1], w[2], w[3]);
                 }
               }
             }
@@ -827,7 +772,10 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           }
         }
       }
-      if (!ok) *abort_flag = 1;
+      if (code != 0) {
+        give_up(a, code);
+        *abort_flag = 1;
+      }
       tc_fence_before();
     } else {
       asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
@@ -835,8 +783,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
       const int t = warp >> 2;                  // query tile of this warpgroup
       const int row = (warp & 3) * 32 + lane;   // TMEM lane == row inside the tile
       const uint32_t lane_sel = uint32_t((warp & 3) * 32) << 16;
-      const uint32_t tmem_s = tmem + t * 128 + lane_sel;
-      const uint32_t tmem_o = tmem + 256 + t * 128 + lane_sel;
+      const uint32_t tmem_s = tmem + T::kS + lane_sel, tmem_p = tmem + T::p(t) + lane_sel, tmem_o = tmem + T::o(t) + lane_sel;
       // what brings the scores to log2 units; with an additive bias they are brought there before it is added, since the bias itself
       // times 1 / scale would overflow where the bias does not, and a large score would lose against its own maximum what the
       // product rounds
@@ -845,7 +792,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
       int seq = 0;
       int cnt = 0;  // steps of this tile so far, over all items
       int ka = 0;   // items in which this tile took part so far
-      bool ok = true;
+      int code = 0;
       XFB_PROF_DECL(16)
 
       // visibility of the 32 columns starting at key `col0` for this thread's row: hidden scores become -inf
@@ -867,7 +814,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
         return fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
       };
       // 32 score columns -> 16 packed probability pairs against the maximum -m (nm2 = (-m, -m)), summed into
-      // sum2 and stored to the 16 columns of S_t that start at `col`
+      // sum2 and stored to the 16 columns of P_t that start at `col`
       auto exp_store = [&](const uint32_t* sr, int col, uint64_t nm2, uint64_t (&sum2)[4]) {
         uint32_t pr[16];
         // (blocks of 16 independent elements: all FMAs, then all exp2, then the sums and packs -- a lone warp per
@@ -889,24 +836,24 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
             pr[(h + i) / 2] = pack_pair<kBf16>(e[i], e[i + 1]);
           }
         }
-        XFB_TMEM_ST_16(tmem_s + col, pr);
+        XFB_TMEM_ST_16(tmem_p + col, pr);
       };
       // O_t *= alpha (per row), through registers
       auto rescale_o = [&](float alpha) {
         const uint64_t al2 = f2_pack(alpha, alpha);
 #pragma unroll
-        for (int cblk = 0; cblk < D / 32; ++cblk) {
-          uint32_t orr[32];
-          XFB_TMEM_LD_32(tmem_o + cblk * 32, orr);
-          XFB_TMEM_WAIT_LD_32(orr);
+        for (int cblk = 0; cblk < D / 16; ++cblk) {
+          uint32_t orr[16];
+          XFB_TMEM_LD_16(tmem_o + cblk * 16, orr);
+          XFB_TMEM_WAIT_LD_16(orr);
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
+          for (int i = 0; i < 16; i += 2) {
             float x0, x1;
             f2_unpack(fmul2(f2_pack(__uint_as_float(orr[i]), __uint_as_float(orr[i + 1])), al2), x0, x1);
             orr[i] = __float_as_uint(x0);
             orr[i + 1] = __float_as_uint(x1);
           }
-          XFB_TMEM_ST_32(tmem_o + cblk * 32, orr);
+          XFB_TMEM_ST_16(tmem_o + cblk * 16, orr);
         }
         tc_wait_st();
       };
@@ -1014,22 +961,18 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           add2(k * 8, mine[k].x), add2(k * 8 + 2, mine[k].y), add2(k * 8 + 4, mine[k].z), add2(k * 8 + 6, mine[k].w);
       };
 
-      while (ok) {
+      while (code == 0) {
         struct {
           int jlo, jhi, m0, shift, shift2, n_base, klen, qlen;
           int64_t bias_off;  // of the item's (batch, head) in the additive bias, in elements
         } it;
         const int idx = pop_item(seq, [&](const Item& d) {
-          it.jlo = t == 0 ? d.jlo[0] : d.jlo[1];
-          it.jhi = t == 0 ? d.jhi[0] : d.jhi[1];
+          it.jlo = d.jlo[t], it.jhi = d.jhi[t];
           it.m0 = d.m0, it.shift = d.shift, it.shift2 = d.shift2, it.n_base = d.n_base, it.klen = d.klen, it.qlen = d.qlen;
           it.bias_off = kBias ? int64_t(d.b) * a.bias_b + int64_t(d.g) * a.bias_g + int64_t(d.h) * a.bias_h : 0;
         });
         if (idx < 0) {
-          if (idx == -2) {
-            give_up(a, 30);
-            ok = false;
-          }
+          if (idx == -2) code = 30;
           break;
         }
         const int jlo = it.jlo, jhi = it.jhi;
@@ -1069,12 +1012,11 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
             bias_load(bw, it.bias_off, mt0, it.qlen, n0, klen, rel_lo, rel_hi, whole);
             bias_prefetch(it.bias_off, mt0, it.qlen, n0 + kBN, j + 1 < jhi ? klen : 0);
           }
-          ok = mbar_wait(&bar->s_full[t], cnt & 1, abort_flag, budget);
-          XFB_PROF_LAP(1)  // wait for the scores
-          if (!ok) {
-            give_up(a, 31 + t);
+          if (!mbar_wait(&bar->s_full[t], cnt & 1, abort_flag, budget)) {
+            code = 31 + t;
             break;
           }
+          XFB_PROF_LAP(1)  // wait for the scores
           tc_fence_after();
           if (need_mask) {
             // Diagonal and ragged tiles: hidden scores are turned into -inf where they lie, in tensor memory, by this
@@ -1104,62 +1046,66 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
               }
             }
             tc_wait_st();
-            XFB_PROF_COUNT(5)
             XFB_PROF_LAP(3)  // the visibility test
           }
           {
-            uint32_t sa[32], sb[32];
-            // ---- first pass: the maximum of the scores
-            XFB_TMEM_LD_32(tmem_s, sa);
-            XFB_TMEM_LD_32(tmem_s + 32, sb);
-            XFB_TMEM_WAIT_LD_32(sa);
-            XFB_TMEM_WAIT_LD_32(sb);
+            // ---- the row's 128 scores come into registers, and the buffer is free for the next QK^T
+            uint32_t s0[32], s1[32], s2[32], s3[32];
+            XFB_TMEM_LD_32(tmem_s, s0);
+            XFB_TMEM_LD_32(tmem_s + 32, s1);
             if constexpr (kBias) {
-              // the biased scores of keys 0-63 are read again in the second pass: they go back to where they came from
-              bias_add(sa, bw, 0);
-              XFB_TMEM_ST_32(tmem_s, sa);
-              bias_add(sb, bw, 1);
-              XFB_TMEM_ST_32(tmem_s + 32, sb);
+              XFB_TMEM_WAIT_LD_32(s0);
+              XFB_TMEM_WAIT_LD_32(s1);
+              bias_add(s0, bw, 0);
+              bias_add(s1, bw, 1);
               if (bias_f32) bias_load(bw, it.bias_off, mt0, it.qlen, n0 + 64, klen, rel_lo, rel_hi, whole);
             }
-            float mx = fmaxf(chunk_max(reinterpret_cast<float*>(sa)), chunk_max(reinterpret_cast<float*>(sb)));
-            if constexpr (kBias) tc_wait_st();
-            XFB_TMEM_LD_32(tmem_s + 64, sa);
-            XFB_TMEM_LD_32(tmem_s + 96, sb);
-            XFB_TMEM_WAIT_LD_32(sa);
-            XFB_TMEM_WAIT_LD_32(sb);
+            XFB_TMEM_LD_32(tmem_s + 64, s2);
+            XFB_TMEM_LD_32(tmem_s + 96, s3);
+            XFB_TMEM_WAIT_LD_32(s0);
+            XFB_TMEM_WAIT_LD_32(s1);
+            XFB_TMEM_WAIT_LD_32(s2);
+            XFB_TMEM_WAIT_LD_32(s3);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar->s_empty);
             if constexpr (kBias) {
-              bias_add(sa, bw, 2);
-              bias_add(sb, bw, 3);
+              bias_add(s2, bw, 2);
+              bias_add(s3, bw, 3);
             }
-            mx = fmaxf(mx, fmaxf(chunk_max(reinterpret_cast<float*>(sa)), chunk_max(reinterpret_cast<float*>(sb))));
+            XFB_PROF_LAP(5)  // scores read
+            float mx = fmaxf(chunk_max(reinterpret_cast<float*>(s0)), chunk_max(reinterpret_cast<float*>(s1)));
+            mx = fmaxf(mx, fmaxf(chunk_max(reinterpret_cast<float*>(s2)), chunk_max(reinterpret_cast<float*>(s3))));
             const float ms = mx * sl2;  // scale > 0 (host guarantees)
-            // ---- the reference follows the maximum only when it has to (a fresh row: from -inf).  QK(t,j) completing
-            // implies PV(t,j-1) completed: O_t is quiescent here.
+            XFB_PROF_LAP(8)  // their maximum
+            // ---- the previous product of the tile has to be through: P_t is free again, O_t quiescent
+            if (!mbar_wait(&bar->pv_done[t], (cnt & 1) ^ 1, abort_flag, budget)) {
+              code = 35 + t;
+              break;
+            }
+            tc_fence_after();
+            XFB_PROF_LAP(7)  // wait for the previous product
+            // ---- the reference follows the maximum only when it has to (a fresh row: from -inf)
             if (__any_sync(0xffffffffu, ms > m_run + kRescaleThreshold)) {
-              XFB_PROF_COUNT(7)
               const float m_new = ms > m_run + kRescaleThreshold ? ms : m_run;
               const float alpha = m_new == m_run ? 1.f : (m_run == -INFINITY ? 0.f : fast_exp2(m_run - m_new));
               if (j > jlo) rescale_o(alpha);
               l_run *= alpha;
               m_run = m_new;
             }
-            // ---- second pass: probabilities.  Keys 64-127 are in registers; keys 0-63 come back behind them.
+            // ---- probabilities
             const float m_use = m_run == -INFINITY ? 0.f : m_run;
             const uint64_t nm2 = f2_pack(-m_use, -m_use);
             uint64_t sum2[4] = {f2_pack(0.f, 0.f), f2_pack(0.f, 0.f), f2_pack(0.f, 0.f), f2_pack(0.f, 0.f)};
-            exp_store(sa, 64, nm2, sum2);
-            XFB_TMEM_LD_32(tmem_s, sa);
-            exp_store(sb, 80, nm2, sum2);
-            XFB_TMEM_LD_32(tmem_s + 32, sb);
+            exp_store(s0, 0, nm2, sum2);
+            exp_store(s1, 16, nm2, sum2);
             tc_wait_st();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&bar->p_half[t]);
-            XFB_TMEM_WAIT_LD_32(sa);
-            XFB_TMEM_WAIT_LD_32(sb);
-            exp_store(sa, 96, nm2, sum2);
-            exp_store(sb, 112, nm2, sum2);
+            XFB_PROF_LAP(2)  // first half of the probabilities
+            exp_store(s2, 32, nm2, sum2);
+            exp_store(s3, 48, nm2, sum2);
             {
               float x0, x1, y0, y1;
               f2_unpack(fadd2(sum2[0], sum2[1]), x0, x1);
@@ -1167,32 +1113,32 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
               l_run += (x0 + x1) + (y0 + y1);
             }
           }
-          XFB_PROF_LAP(2)  // the step proper
           XFB_PROF_COUNT(6)
           tc_wait_st();
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&bar->p_full[t]);
-          XFB_PROF_LAP(4)  // storing P
+          XFB_PROF_LAP(4)  // second half
         }
-        if (!ok) break;
+        if (code != 0) break;
         // hand the row's statistics to the output warps
-        if (ka > 0 && !mbar_wait(&bar->stats_empty[t], (ka - 1) & 1, abort_flag, budget)) {
-          give_up(a, 33 + t);
-          ok = false;
+        if (!mbar_wait(&bar->stats_empty[t], (ka++ & 1) ^ 1, abort_flag, budget)) {
+          code = 33 + t;
           break;
         }
-        ++ka;
         stats[t * kBM + row] = make_float2(m_run, l_run);
         mbar_arrive(&bar->stats_full[t]);
       }
-      if (!ok) *abort_flag = 1;
+      if (code != 0) {
+        give_up(a, code);
+        *abort_flag = 1;
+      }
       tc_fence_before();
-      XFB_PROF_STORE(warp * 8, 8)
+      XFB_PROF_STORE(warp * 16, 16)
     }
 
     __syncthreads();
-    if (warp == kMmaWarp0) {
+    if (warp == kQkWarp) {
       tc_fence_after();
       tmem_dealloc(tmem, 512);
     }
@@ -1237,9 +1183,9 @@ static int launch_t(const Sm100Args& a, cudaStream_t stream) {
 #ifdef XFB_PST_PROFILE
 extern "C" __attribute__((visibility("default"))) int xfb200_debug_read_prefill_profile(long long* out, int clear) {
   cudaDeviceSynchronize();
-  cudaError_t e = cudaMemcpyFromSymbol(out, pst::g_prof, sizeof(long long) * 160 * 96);
+  cudaError_t e = cudaMemcpyFromSymbol(out, pst::g_prof, sizeof(long long) * 160 * 160);
   if (e == cudaSuccess && clear) {
-    static long long zeros[160 * 96] = {0};
+    static long long zeros[160 * 160] = {0};
     e = cudaMemcpyToSymbol(pst::g_prof, zeros, sizeof(zeros));
   }
   return e == cudaSuccess ? 0 : -3;
