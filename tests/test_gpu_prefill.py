@@ -568,6 +568,30 @@ def test_padded_head_dims_on_the_tcgen05_kernel(D, layout):
 
 
 @gpu
+@pytest.mark.parametrize("kind", ["none", "bottom_right", "varlen_local", "heads_outermost"])
+@pytest.mark.parametrize("H,D", [(2, 128), (3, 128), (4, 80), (8, 64), (16, 128), (128, 64)])
+def test_heads_of_a_group_share_a_tile(H, D, kind):
+    """GQA groups of a power of two up to 128 are packed into the rows of a tile (3 is not): odd numbers of tokens, items without
+    a key (bottom right, more queries than keys), windows, several sequences, heads that lie further apart than tokens."""
+    require_cuda()
+    dtype, G = torch.float16, 2
+    Mq, Mkv = (333, 77) if kind == "bottom_right" else (131, 300)
+    if kind == "varlen_local":
+        q_lens, k_lens = [1, 70, 33, 40], [40, 133, 33, 200]
+        q, k, v = rand_qkv(1, sum(q_lens), sum(k_lens), G, H, D, dtype, seed=H + D)
+        bias = ab.BlockDiagonalMask.from_seqlens(q_lens, k_lens, device="cuda").make_local_attention_from_bottomright(45)
+    else:
+        q, k, v = rand_qkv(2, Mq, Mkv, G, H, D, dtype, seed=H * D)
+        bias = {"none": None, "bottom_right": ab.LowerTriangularFromBottomRightMask(), "heads_outermost": ab.LowerTriangularMask()}[kind]
+    if kind == "heads_outermost":
+        q = q.permute(0, 2, 3, 1, 4).contiguous().permute(0, 3, 1, 2, 4)
+    out, lse = fmha.memory_efficient_attention_forward_requires_grad(q, k, v, bias, op=P.FwOp_Tcgen05_Persistent)
+    ro, rl = ref(q, k, v, bias)
+    assert_o_lse(out, lse, ro, rl, dtype, f"packed {kind} H={H} D={D}")
+    _status_ok()
+
+
+@gpu
 @pytest.mark.parametrize("causal", [False, True])
 @pytest.mark.parametrize("bias_dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("Mkv,wide,D", [(520, 520, 128), (517, 520, 64), (517, 517, 80), (3, 8, 128), (131, 136, 40)])

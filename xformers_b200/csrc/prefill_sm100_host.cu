@@ -8,16 +8,16 @@ namespace xfb {
 
 constexpr long long kDefaultWaitBudgetCycles = 400000000LL;  // ~0.2 s of SM clock
 
-// Tensor map over [D, heads, rows, batch] (innermost first); box = 64 x 1 x box_rows x 1, 128B swizzle.
+// Tensor map over [D, heads, rows, batch] (innermost first); box = 64 x box_heads x box_rows x 1, 128B swizzle.
 static int make_map(CUtensorMap* tm, const void* base, int dtype, int D, int64_t heads, int64_t head_stride, int64_t rows,
-                    int64_t row_stride, int64_t batch, int64_t batch_stride, const char* what, int box_rows = 128) {
+                    int64_t row_stride, int64_t batch, int64_t batch_stride, const char* what, int box_heads = 1) {
   EncodeTiledFn enc = encode_tiled_fn();
   if (enc == nullptr) return set_error(XFB200_E_CUDA, "prefill: cuTensorMapEncodeTiled is not available from this driver");
   const cuuint64_t dims[4] = {cuuint64_t(D), cuuint64_t(heads), cuuint64_t(rows), cuuint64_t(batch)};
   // a dimension of extent 1 never contributes to an address; give it a legal stride
   auto st = [&](int64_t s, int64_t extent) { return cuuint64_t((extent > 1 ? s : int64_t(D)) * 2); };
   const cuuint64_t strides[3] = {st(head_stride, heads), st(row_stride, rows), st(batch_stride, batch)};
-  const cuuint32_t box[4] = {64, 1, cuuint32_t(box_rows), 1};
+  const cuuint32_t box[4] = {64, cuuint32_t(box_heads), cuuint32_t(128 / box_heads), 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = enc(tm, dtype == XFB200_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
                    const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -71,9 +71,15 @@ int prefill_sm100_launch(const xfb200_prefill_params* p, cudaStream_t stream) {
   const int64_t q_rows = varlen ? p->total_q : p->mq;
   const int64_t k_rows = p->mkv;
   const int64_t nb = varlen ? 1 : p->batch;
-  int rc = make_map(&a.tm_q, p->q, p->dtype, D, hc, hs, q_rows, p->q_strides.m, nb, p->q_strides.b, "q");
-  if (rc) return rc;
   const bool kbc = H > 1 && p->k_strides.h == 0;
+  // Heads that read the same keys fill a tile together (its rows are (token, head) pairs): a block of few tokens is not padded to
+  // 128 rows per head, and the two tiles of an item end at the same key step of a causal mask.  (An additive bias belongs to a head.)
+  if (kbc && p->bias == nullptr && p->kernel_path != XFB200_PREFILL_TCGEN05_CTA && H <= 128 && (H & (H - 1)) == 0 &&
+      int64_t(p->mq) * H <= 0x3fffffff)
+    while ((1 << a.pack_shift) < H) ++a.pack_shift;
+  const int pack = 1 << a.pack_shift;
+  int rc = make_map(&a.tm_q, p->q, p->dtype, D, hc, hs, q_rows, p->q_strides.m, nb, p->q_strides.b, "q", pack);
+  if (rc) return rc;
   int64_t khs = p->k_strides.g, khc = G, vhs = p->v_strides.g;
   if (!kbc) {
     heads_flatten(p->k_strides, G, H, &khs, &khc);
@@ -107,21 +113,22 @@ int prefill_sm100_launch(const xfb200_prefill_params* p, cudaStream_t stream) {
     // 900 with 128, 830-840 with 8..32).  Causal launches take larger groups: their items differ in weight, and the
     // more of them run side by side the shorter the tail of a group.
     const double keys = varlen ? double(p->mkv) / double(p->batch > 0 ? p->batch : 1) : double(p->mkv);
-    const double per_head = 2.0 * keys * D * 2.0 / (kbc ? H : 1);  // K and V, 2 bytes per element; a GQA group shares them
+    const double per_head = 2.0 * keys * D * 2.0 / (kbc ? H / pack : 1);  // K and V, 2 bytes per element; a GQA group shares them
     const double budget = (p->mask_type == XFB200_MASK_NONE ? 16.0 : 64.0) * 1024.0 * 1024.0;
     int hpw = 1;
     while (hpw < 256 && 2.0 * hpw * per_head <= budget) hpw *= 2;
-    if (kbc && hpw < H) hpw = H;  // the heads of a GQA group read the same keys: keep them together
+    if (kbc && hpw < H / pack) hpw = H / pack;  // the heads of a GQA group read the same keys: keep them together
     a.heads_per_wave = hpw;
   }
   a.scale_log2 = p->scale * 1.4426950408889634f;
-  a.q_tiles = (p->mq + 255) / 256, a.item_rows = 256;
+  const int64_t rows = int64_t(p->mq) * pack;  // of all tiles of a (sequence, head or group of packed heads)
+  a.q_tiles = int32_t((rows + 255) / 256), a.item_rows = 256;
   if (p->kernel_path != XFB200_PREFILL_TCGEN05_CTA) {
     // Where even items of a single tile leave no SM two of them, tiles get an SM each: alone on it, a tile's step does not wait
     // for the other's softmax and products (causal, 4 heads x 4096
     // rows 68.5 -> 61.8 us, 4 x 1024 25.1 -> 23.0; 8 heads x 700, no mask, 23.0 -> 21.0).
-    const int64_t tiles = (int64_t(p->mq) + 127) / 128;
-    if (int64_t(G) * H * p->batch * tiles <= sm_count() - a.sm_margin) a.q_tiles = int32_t(tiles), a.item_rows = 128;
+    const int64_t tiles = (rows + 127) / 128;
+    if (int64_t(G) * H / pack * p->batch * tiles <= sm_count() - a.sm_margin) a.q_tiles = int32_t(tiles), a.item_rows = 128;
   }
   a.debug_flags = p->debug_flags;
   a.wait_budget = p->wait_budget_kcycles > 0 ? 1000LL * p->wait_budget_kcycles : kDefaultWaitBudgetCycles;

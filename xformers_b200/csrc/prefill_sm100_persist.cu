@@ -2,7 +2,9 @@
 //
 // A work item is a block of 256 query rows of one (sequence, query head): two
 // 128-row query tiles that share every K/V tile TMA brings in.  (One tile, where
-// the tiles of the whole launch are no more than the SMs.)  Items are
+// the tiles of the whole launch are no more than the SMs.)  Where the heads of a
+// GQA group read the same keys, the rows of a tile are (token, head of the group)
+// pairs, which the box of the Q copies lays out that way.  Items are
 // handed out by one atomic counter, heaviest first (the last row block of every
 // head, then the one before, ...) inside groups of heads whose keys and values
 // fit the L2 together, so the SMs stay evenly loaded whatever the sequence
@@ -246,8 +248,9 @@ __device__ __forceinline__ int sequence_order(const Sm100Args& a, int lane) {
 // Returns false when the item has no query row at all (a row block past the end of its sequence).  Called by a whole warp.
 __device__ __forceinline__ bool decode_item(const Sm100Args& a, int order, int idx, Item& it) {
   it.idx = idx;
-  const int n_heads = a.groups * a.heads_per_group;
+  const int n_heads = (a.groups * a.heads_per_group) >> a.pack_shift;  // (or groups of packed heads)
   const int n_bh = n_heads * a.batch;
+  const int tile_rows = kBM >> a.pack_shift;  // query rows (tokens) of a tile
   // Heaviest (latest) row blocks first, but not over all heads at once: the CTAs of a launch run side by side, and
   // the keys and values they read should fit the L2 (a K/V tile is read once per row block of its head: from DRAM
   // the first time only, if it is still there).  Heads are taken in groups of heads_per_wave; inside a group the
@@ -261,7 +264,7 @@ __device__ __forceinline__ bool decode_item(const Sm100Args& a, int order, int i
   const int bh = first_bh + rr % in_grp;
   it.b = bh / n_heads;
   if (a.seqstart_q != nullptr && a.batch <= 32) it.b = __shfl_sync(0xffffffffu, order, it.b);
-  it.head = bh % n_heads;
+  it.head = (bh % n_heads) << a.pack_shift;
   it.g = it.head / a.heads_per_group, it.h = it.head % a.heads_per_group;
   it.kv_head = it.g * (a.kv_h_is_broadcast ? 1 : a.heads_per_group) + (a.kv_h_is_broadcast ? 0 : it.h);
   it.q_row0 = 0, it.k_row0 = 0, it.qlen = a.mq, it.klen = a.mkv, it.tb = it.b;
@@ -272,24 +275,25 @@ __device__ __forceinline__ bool decode_item(const Sm100Args& a, int order, int i
     it.klen = a.seqlen_k != nullptr ? a.seqlen_k[it.b] : a.seqstart_k[it.b + 1] - it.k_row0;
     it.tb = 0;
   }
-  it.m0 = qt * a.item_rows;
+  const int item_rows = a.item_rows >> a.pack_shift;
+  it.m0 = qt * item_rows;
   if (it.m0 >= it.qlen) return false;
   it.shift = (a.bottom_right ? it.klen - it.qlen : 0) - a.kv_offset;
-  it.qlen = min(it.qlen, it.m0 + a.item_rows);  // (an item of one tile has no row of the other)
+  it.qlen = min(it.qlen, it.m0 + item_rows);  // (an item of one tile has no row of the other)
   it.shift2 = -a.kv_offset2;
   it.n_base = 0;
   if (a.window_left >= 0) it.n_base = max(0, it.m0 + it.shift - a.window_left) / kBN * kBN;
   it.j_begin = 0x7fffffff, it.j_end = 0;
 #pragma unroll
   for (int t = 0; t < kTiles; ++t) {
-    const int mt0 = it.m0 + t * kBM;
+    const int mt0 = it.m0 + t * tile_rows;
     int hi = it.klen, lo = it.n_base;
-    if (a.window_right >= 0) hi = min(hi, mt0 + kBM + it.shift + a.window_right);
+    if (a.window_right >= 0) hi = min(hi, mt0 + tile_rows + it.shift + a.window_right);
     if (a.kv_split > 0) {
       // Two key ranges back to back (causal, the second one later in the sequence): rows that see any key of the
       // second range see all of the first, so the visible keys are still one run of rows of the tensor.
-      const int hi1 = min(it.klen - a.kv_split, mt0 + kBM + it.shift2);
-      hi = hi1 > 0 ? a.kv_split + hi1 : min(a.kv_split, mt0 + kBM + it.shift);
+      const int hi1 = min(it.klen - a.kv_split, mt0 + tile_rows + it.shift2);
+      hi = hi1 > 0 ? a.kv_split + hi1 : min(a.kv_split, mt0 + tile_rows + it.shift);
     }
     if (a.window_left >= 0) lo = max(it.n_base, max(0, mt0 + it.shift - a.window_left) / kBN * kBN);
     if (mt0 >= it.qlen) hi = lo;  // no valid row in this tile
@@ -325,7 +329,9 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
   float2* stats = reinterpret_cast<float2*>(smem + L::kStats);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const int n_items = a.q_tiles * a.groups * a.heads_per_group * a.batch;
+  const int n_items = ((a.q_tiles * a.groups * a.heads_per_group) >> a.pack_shift) * a.batch;
+  const int pack_shift = kBias ? 0 : a.pack_shift;
+  const int tile_rows = kBM >> pack_shift;  // query rows (tokens) of a tile
   const long long budget = a.wait_budget;
   const int head_dim = kPad ? a.head_dim : D;
 
@@ -420,7 +426,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
             }
             if (!decode_item(a, order, idx, it)) continue;
             if (it.j_end > it.j_begin) return;
-            const int nrows = min(kBM * kTiles, it.qlen - it.m0);
+            const int nrows = (it.qlen - it.m0) << pack_shift, head_mask = (1 << pack_shift) - 1;
             const int osz = a.out_dtype == XFB200_F32 ? 4 : 2;
             const int chunks = head_dim * osz / 16;
             uint8_t* ob = reinterpret_cast<uint8_t*>(a.out);
@@ -428,13 +434,13 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
 #pragma unroll 1
             for (int i = lane; i < nrows * chunks; i += 32) {
               const int r = i / chunks, c = i % chunks;
-              *reinterpret_cast<uint4*>(ob + (base + int64_t(r) * a.os.m) * osz + c * 16) = make_uint4(0, 0, 0, 0);
+              *reinterpret_cast<uint4*>(ob + (base + int64_t(r >> pack_shift) * a.os.m + int64_t(r & head_mask) * a.os.h) * osz + c * 16) = make_uint4(0, 0, 0, 0);
             }
             if (a.lse != nullptr) {
               const int64_t lo = a.seqstart_q != nullptr ? int64_t(it.g) * a.lse_g + int64_t(it.h) * a.lse_h + it.q_row0 + it.m0
                                                          : int64_t(it.b) * a.lse_b + int64_t(it.g) * a.lse_g + int64_t(it.h) * a.lse_h + it.m0;
 #pragma unroll 1
-              for (int r = lane; r < nrows; r += 32) a.lse[lo + r] = -INFINITY;
+              for (int r = lane; r < nrows; r += 32) a.lse[lo + (r >> pack_shift) + int64_t(r & head_mask) * a.lse_h] = -INFINITY;
             }
           }
         };
@@ -501,7 +507,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
                   break;
                 }
                 qph ^= 1u << t;
-                load_tile(L::kQ + t * L::kQTile, &a.tm_q, &bar->q_full[t], cur.head, cur.q_row0 + cur.m0 + t * kBM, cur.tb);
+                load_tile(L::kQ + t * L::kQTile, &a.tm_q, &bar->q_full[t], cur.head, cur.q_row0 + cur.m0 + t * tile_rows, cur.tb);
               }
               if (code != 0) break;
             }
@@ -703,10 +709,10 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
         }
 #pragma unroll 1
         for (int t = 0; t < kTiles; ++t) {
-          const int i_loc = it.m0 + t * kBM + row;
+          const int i_loc = it.m0 + t * tile_rows + (row >> pack_shift), h_loc = row & ((1 << pack_shift) - 1);
           const bool valid_row = i_loc < it.qlen;
           const bool active = t == 0 ? it.jhi0 > it.jlo0 : it.jhi1 > it.jlo1;
-          if (!active && it.m0 + t * kBM >= it.qlen) continue;  // no row of this tile exists
+          if (!active && it.m0 + t * tile_rows >= it.qlen) continue;  // no row of this tile exists
           float m_run = -INFINITY, l_run = 0.f;
           const uint32_t tmem_o = tmem + T::o(t) + lane_sel;
           if (active) {
@@ -725,7 +731,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
             tc_fence_after();
           }
           const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-          const int64_t o_off = int64_t(it.tb) * a.os.b + int64_t(it.q_row0 + i_loc) * a.os.m + int64_t(it.g) * a.os.g + int64_t(it.h) * a.os.h;
+          const int64_t o_off = int64_t(it.tb) * a.os.b + int64_t(it.q_row0 + i_loc) * a.os.m + int64_t(it.g) * a.os.g + int64_t(it.h + h_loc) * a.os.h;
 #pragma unroll 1
           for (int col = 0; col < D; col += 16) {
             uint32_t orr[16];
@@ -766,8 +772,8 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           }
           if (valid_row && a.lse != nullptr) {
             const float lse = l_run > 0.f ? (m_run + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
-            const int64_t lo = a.seqstart_q != nullptr ? int64_t(it.g) * a.lse_g + int64_t(it.h) * a.lse_h + it.q_row0 + i_loc
-                                                       : int64_t(it.b) * a.lse_b + int64_t(it.g) * a.lse_g + int64_t(it.h) * a.lse_h + i_loc;
+            const int64_t lo = a.seqstart_q != nullptr ? int64_t(it.g) * a.lse_g + int64_t(it.h + h_loc) * a.lse_h + it.q_row0 + i_loc
+                                                       : int64_t(it.b) * a.lse_b + int64_t(it.g) * a.lse_g + int64_t(it.h + h_loc) * a.lse_h + i_loc;
             a.lse[lo] = lse;
           }
         }
@@ -977,8 +983,8 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
         }
         const int jlo = it.jlo, jhi = it.jhi;
         if (jhi <= jlo) continue;  // this tile sees no key in this item
-        const int mt0 = it.m0 + t * kBM;
-        const int i_loc = mt0 + row;
+        const int mt0 = it.m0 + t * tile_rows;
+        const int i_loc = mt0 + (row >> pack_shift);
         const bool causal = a.window_right >= 0;
         col_hi = causal ? min(it.klen, i_loc + it.shift + a.window_right + 1) : it.klen;
         col_lo = a.window_left >= 0 ? i_loc + it.shift - a.window_left : 0;
@@ -999,7 +1005,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
             col_hi = min(klen, i_loc + shift + 1);
           }
           const bool need_mask = (n0 + kBN > klen) || (causal && n0 + kBN - 1 > mt0 + shift + a.window_right) ||
-                                 (a.window_left >= 0 && n0 < mt0 + kBM - 1 + shift - a.window_left);
+                                 (a.window_left >= 0 && n0 < mt0 + tile_rows - 1 + shift - a.window_left);
           uint4 bw[kBias ? 16 : 1];
           bool whole = false;
           int rel_lo = 0, rel_hi = 0;  // visible keys of row r: from r + rel_lo, below r + rel_hi
@@ -1165,7 +1171,7 @@ static int launch_t(const Sm100Args& a, cudaStream_t stream) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return cuda_fail("prefill(sm100, persistent): cudaFuncSetAttribute", e);
   }
-  const int64_t items = int64_t(a.groups) * a.heads_per_group * a.batch * a.q_tiles;
+  const int64_t items = ((int64_t(a.groups) * a.heads_per_group) >> a.pack_shift) * a.batch * a.q_tiles;
   if (items > 0x3fffffff) return set_error(XFB200_E_UNSUPPORTED, "prefill: too many blocks of query rows");
   int sms = sm_count() - a.sm_margin;
   if (sms < 1) sms = 1;
