@@ -149,6 +149,9 @@ struct DecStage {
   __host__ __device__ static int ss_bytes(int hb) { return kFmt == kFmtFp8 ? tokens(hb) * hb * 4 : 0; }
 };
 
+// Floats of a row in the area where the warps of a CTA meet: the un-normalised output, maximum, sum; rows on 16-byte boundaries.
+__host__ __device__ constexpr int cmb_pitch(int D) { return D + 4; }
+
 constexpr int kDecMaxStages = 12;
 // Bytes of cache in flight per SM are what hide the HBM latency.  The 16-bit
 // kernel runs one CTA per SM with a ~212 KB ring.  The int4 kernel does 4x the
@@ -170,7 +173,7 @@ struct DecWarp {
   uint64_t* full_bar;
   uint64_t* empty_bar;
   uint64_t* q_done_bar;
-  float* mine;  // this warp's slot of the combine area: [ROWS][D + 2]
+  float* mine;  // this warp's slot of the combine area: [ROWS][cmb_pitch(D)]
   int lane, hw, sub, wph, row0;
   int b, head;  // sequence and kv head of this warp
   int chunk_lo, chunk_hi, kv_len, n_tiles;
@@ -192,7 +195,7 @@ template <int D, int MT, bool kBf16, bool kExtras>
 __device__ __forceinline__ void consume_plain(const DecodeArgs& a, const DecWarp& w) {
   constexpr int KS = D / 16;  // k-steps of the QK^T product
   constexpr int NT = D / 8;   // n-tiles of the PV product
-  constexpr int kCmbRow = D + 2;
+  constexpr int kCmbRow = cmb_pitch(D);
   constexpr int kSps = DecStage<D, kFmtPlain>::kSubTiles;
   const int lane = w.lane, r = lane >> 2, c = lane & 3;
   const int R = a.rows, hw = w.hw, row_bytes = w.row_bytes;
@@ -642,7 +645,7 @@ __device__ __forceinline__ void quant_rows_finish(QuantRows<NTQ>& q, const DecWa
     for (int nt = 0; nt < NTQ; ++nt)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        float* row = w.mine + (nt * 8 + 2 * c + e) * (D + 2);
+        float* row = w.mine + (nt * 8 + 2 * c + e) * cmb_pitch(D);
         row[D] = q.slack[nt][e] == -INFINITY ? -INFINITY : q.ref[nt][e];
         row[D + 1] = q.l[nt][e];
       }
@@ -689,7 +692,7 @@ __device__ __forceinline__ void consume_int4(const DecodeArgs& a, const DecWarp&
   constexpr int MTV = D / 16;   // m-tiles of V^T P^T
   constexpr int WPT = D / 64;   // V words per thread and token
   constexpr int kQRowBytes = D * 2;
-  constexpr int kCmbRow = D + 2;
+  constexpr int kCmbRow = cmb_pitch(D);
   constexpr int U = DecStage<D, kFmtInt4>::kSubTiles;  // all of a stage in one step
   const int lane = w.lane, r = lane >> 2, c = lane & 3;
   const int hw = w.hw;
@@ -845,7 +848,7 @@ __device__ __forceinline__ void consume_int4_groups(const DecodeArgs& a, const D
   constexpr int GW = (D / 8) / NG;   // nibble words per group
   static_assert(GW >= WPT && GW >= 1 && (D / 8) % NG == 0, "groups of at least 16 elements");
   constexpr int kQRowBytes = D * 2;
-  constexpr int kCmbRow = D + 2;
+  constexpr int kCmbRow = cmb_pitch(D);
   constexpr int kSps = DecStage<D, kFmtInt4, NG>::kSubTiles;
   constexpr float kLazy = 4.f;
   const int lane = w.lane, r = lane >> 2, c = lane & 3;
@@ -1224,7 +1227,7 @@ __device__ __forceinline__ void consume_fp8(const DecodeArgs& a, const DecWarp& 
   constexpr int MTV = D / 16;  // m-tiles of V^T P^T
   constexpr int WJ = D / 32;   // V words per thread and token
   constexpr int kQRowBytes = D * 2;
-  constexpr int kCmbRow = D + 2;
+  constexpr int kCmbRow = cmb_pitch(D);
   constexpr int kSps = DecStage<D, kFmtFp8>::kSubTiles;
   const int lane = w.lane, r = lane >> 2, c = lane & 3;
   const int hw = w.hw, hb = a.hb;
@@ -1627,8 +1630,8 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt, MT>::kCtasPerS
     __syncwarp();
   }
   // Partial results of the warps meet in shared memory once the ring is drained.
-  float* cmb = reinterpret_cast<float*>(smem_raw);  // [warp][ROWS][D + 2]  (acc, m, l)
-  constexpr int kCmbRow = D + 2;
+  float* cmb = reinterpret_cast<float*>(smem_raw);  // [warp][ROWS][pitch]  (acc, m, l)
+  constexpr int kCmbRow = cmb_pitch(D);
   DecWarp w;
   w.qs = q_smem + warp * ROWS * kQRowBytes;
   w.stage_base = stage_base;
@@ -1647,72 +1650,93 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt, MT>::kCtasPerS
   else
     consume_plain<D, MT, kBf16, kFmt == kFmtPlainX>(a, w);
   asm volatile("bar.sync 1, %0;" ::"n"(kDecConsumerWarps * 32) : "memory");
-  // warps of head hw share the rows: warp `sub` finalises rows sub, sub+wph, ...
+  // The wph partials of a row are added up, four columns to a thread, without a branch between the loads.  (A warp per row that
+  // went through them one by one took 1.4 us for 16 rows of 8 partials: two sequences of 16384 keys, f16, 11.7 -> 10.8 us; 64
+  // sequences of up to 32768 keys over the int4 cache 285.7 -> 281.)
   const bool direct = a.split_k == 1;
-  for (int rr = sub; rr < ROWS; rr += wph) {
-    const int row = row0 + rr;
-    if (row >= R) break;
+  const int hb_shift = __ffs(hb) - 1;
+  const int n_rows = min(ROWS, R - row0) << hb_shift;  // (row, head) pairs
+  constexpr int kCols = D / 4;                          // threads to a row
+  for (int i = threadIdx.x; i < n_rows * kCols; i += kDecConsumerWarps * 32) {
+    const int col = (i % kCols) * 4, hh = (i / kCols) & (hb - 1), rr = (i / kCols) >> hb_shift;
+    const float* src = cmb + (hh * ROWS + rr) * kCmbRow;
+    const int pitch = (ROWS * kCmbRow) << hb_shift;  // from a warp to the next one of the same head
     float mx = -INFINITY;
-    for (int w2 = 0; w2 < wph; ++w2) mx = fmaxf(mx, cmb[size_t(w2 * hb + hw) * ROWS * kCmbRow + rr * kCmbRow + D]);
+#pragma unroll
+    for (int w2 = 0; w2 < kDecConsumerWarps; ++w2)
+      if (w2 < wph) mx = fmaxf(mx, src[w2 * pitch + D]);
     const float m_use = mx == -INFINITY ? 0.f : mx;
     float den = 0.f;
-    float o[D / 32];
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto add = [&](float2 ml, float4 x) {
+      const bool any = ml.x != -INFINITY;  // (a warp without a visible token may hold anything)
+      const float wgt = any ? fast_exp2(ml.x - m_use) : 0.f;
+      den += any ? wgt * ml.y : 0.f;
+      o.x += any ? wgt * x.x : 0.f, o.y += any ? wgt * x.y : 0.f;
+      o.z += any ? wgt * x.z : 0.f, o.w += any ? wgt * x.w : 0.f;
+    };
+    auto m_l = [&](int w2) { return *reinterpret_cast<const float2*>(src + w2 * pitch + D); };
+    auto part = [&](int w2) { return *reinterpret_cast<const float4*>(src + w2 * pitch + col); };
+    if constexpr (kQuant) {
+      // (partials held in registers at once would be registers that the main loop has to do without: 4 % of the fp8 case)
+#pragma unroll 8
+      for (int w2 = 0; w2 < wph; ++w2) add(m_l(w2), part(w2));
+    } else {
+      float2 ml[kDecConsumerWarps];
+      float4 x[kDecConsumerWarps];
 #pragma unroll
-    for (int i = 0; i < D / 32; ++i) o[i] = 0.f;
-    for (int w2 = 0; w2 < wph; ++w2) {
-      const float* src = cmb + size_t(w2 * hb + hw) * ROWS * kCmbRow + rr * kCmbRow;
-      const float mw = src[D];
-      if (mw == -INFINITY) continue;
-      const float wgt = fast_exp2(mw - m_use);
-      den += wgt * src[D + 1];
+      for (int w2 = 0; w2 < kDecConsumerWarps; ++w2) {
+        ml[w2] = make_float2(-INFINITY, 0.f);
+        x[w2] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (w2 < wph) ml[w2] = m_l(w2), x[w2] = part(w2);
+      }
 #pragma unroll
-      for (int i = 0; i < D / 32; ++i) o[i] += wgt * src[i * 32 + lane];
+      for (int w2 = 0; w2 < kDecConsumerWarps; ++w2) add(ml[w2], x[w2]);
     }
     const float inv = den > 0.f ? 1.f / den : 0.f;
     const float lse = den > 0.f ? (m_use + log2f(den)) * 0.6931471805599453f : -INFINITY;
-    const int qi = row / a.q_per_kv, h = row % a.q_per_kv;
+    o = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+    const int row = row0 + rr, oh = hblk * hb + hh;
     if (direct) {
-      const int64_t off = (int64_t(b) * a.mq + qi) * a.o_sm + int64_t(head) * a.o_sg + int64_t(h) * a.o_sh;
+      const int qi = row / a.q_per_kv, h = row % a.q_per_kv;
+      const int64_t off = (int64_t(b) * a.mq + qi) * a.o_sm + int64_t(oh) * a.o_sg + int64_t(h) * a.o_sh + col;
+      const float val[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
-      for (int i = 0; i < D / 32; ++i) {
-        const float val = o[i] * inv;
-        const int d = i * 32 + lane;
+      for (int e = 0; e < 4; ++e) {  // (rows of the output need not start on a boundary)
         if (a.out_dtype == XFB200_F32)
-          reinterpret_cast<float*>(a.out)[off + d] = val;
+          reinterpret_cast<float*>(a.out)[off + e] = val[e];
         else if (a.out_dtype == XFB200_BF16)
-          reinterpret_cast<__nv_bfloat16*>(a.out)[off + d] = __float2bfloat16_rn(val);
+          reinterpret_cast<__nv_bfloat16*>(a.out)[off + e] = __float2bfloat16_rn(val[e]);
         else
-          reinterpret_cast<__half*>(a.out)[off + d] = __float2half_rn(val);
+          reinterpret_cast<__half*>(a.out)[off + e] = __float2half_rn(val[e]);
       }
-      if (a.lse != nullptr && lane == 0) a.lse[int64_t(head) * a.lse_sg + int64_t(h) * a.lse_sh + int64_t(b) * a.mq + qi] = lse;
+      if (a.lse != nullptr && col == 0) a.lse[int64_t(oh) * a.lse_sg + int64_t(h) * a.lse_sh + int64_t(b) * a.mq + qi] = lse;
     } else {
-      const int64_t prow = ((int64_t(b) * a.split_k + split) * a.kv_heads + head) * R + row;
-      float* po = a.part_o + prow * D;
-#pragma unroll
-      for (int i = 0; i < D / 32; ++i) po[i * 32 + lane] = o[i] * inv;
-      if (lane == 0) a.part_lse[prow] = lse;
+      const int64_t prow = ((int64_t(b) * a.split_k + split) * a.kv_heads + oh) * R + row;
+      *reinterpret_cast<float4*>(a.part_o + prow * D + col) = o;
+      if (col == 0) a.part_lse[prow] = lse;
     }
   }
 }
 
 // ---------------------------------------------------------------------------
-// Merge of the per-chunk partials of each sequence.  Four warps per output row
-// (b, kv head, query row), which take its chunks in turn with four loads in
-// flight each and meet in shared memory: with one warp per row, walking the
-// chunks one after the other, 64 rows of 128 chunks took 28 us -- latency, not
-// bytes.  Every chunk goes to a fixed warp and the warps are added up in order,
+// Merge of the per-chunk partials of each sequence.  Latency bounds it, not bytes: what a row needs is asked for in one round
+// of loads -- the log-sum-exps of all chunks for the maximum, and for each of the row's kWarpsPerRow warps eight
+// (or four) of its chunks with their log-sum-exps -- where the partials used to wait for the maximum.  Few rows get eight warps each
+// and cover 64 chunks in that round (4 sequences of 1000 keys, 9.4 -> 8.5 us for both kernels); many rows hide one another's latency,
+// and registers for eight chunks would cost them CTAs (4096 rows, 26 chunks: 5 us).  Lengths are read before the split kernel
+// has ended: it began only when whatever wrote them had.
+// Every chunk goes to a fixed warp and the warps are added up in order,
 // whatever the number of chunks, so the result is deterministic and does not
 // depend on a bound.  Only the chunks that exist for sequence b are read.
 // ---------------------------------------------------------------------------
-constexpr int kMergeWarpsPerCta = 8, kMergeWarpsPerRow = 4;
-template <int D>
+constexpr int kMergeWarpsPerCta = 8;
+template <int D, int kWarpsPerRow, int U>
 __global__ void __launch_bounds__(kMergeWarpsPerCta * 32) decode_merge_kernel(const __grid_constant__ DecodeArgs a) {
   constexpr int V = D / 32;
   __shared__ float red[kMergeWarpsPerCta][D + 4];
-  grid_dep_wait();
-  grid_dep_launch();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int step = kMergeWarpsPerRow;
+  constexpr int step = kWarpsPerRow;
   const int part = warp % step;
   const int64_t gw = int64_t(blockIdx.x) * (kMergeWarpsPerCta / step) + warp / step;
   const int R = a.rows;
@@ -1724,7 +1748,31 @@ __global__ void __launch_bounds__(kMergeWarpsPerCta * 32) decode_merge_kernel(co
   if (a.window_size > 0) kv_len = min(kv_len, a.window_span);
   const int nsplit = live ? min(a.split_k, (kv_len + a.chunk_tokens - 1) / a.chunk_tokens) : 0;
   const int64_t prow0 = (int64_t(b) * a.split_k * a.kv_heads + head) * R + row, pstep = int64_t(a.kv_heads) * R;
+  grid_dep_wait();
+  grid_dep_launch();
 
+  float l[U], x[U][V];
+  auto load = [&](int s0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int s = s0 + u * step;
+      l[u] = -INFINITY;
+#pragma unroll
+      for (int i = 0; i < V; ++i) x[u][i] = 0.f;
+      if (s < nsplit) {
+        l[u] = a.part_lse[prow0 + s * pstep];
+        const float* po = a.part_o + (prow0 + s * pstep) * D + lane * V;
+        if constexpr (V == 4) {
+          const float4 y = *reinterpret_cast<const float4*>(po);
+          x[u][0] = y.x, x[u][1] = y.y, x[u][2] = y.z, x[u][3] = y.w;
+        } else {
+          const float2 y = *reinterpret_cast<const float2*>(po);
+          x[u][0] = y.x, x[u][1] = y.y;
+        }
+      }
+    }
+  };
+  load(part);
   float mx = -INFINITY;
   for (int s = lane; s < nsplit; s += 32) mx = fmaxf(mx, a.part_lse[prow0 + s * pstep]);
 #pragma unroll
@@ -1734,33 +1782,17 @@ __global__ void __launch_bounds__(kMergeWarpsPerCta * 32) decode_merge_kernel(co
   for (int i = 0; i < V; ++i) acc[i] = 0.f;
   float den = 0.f;
   if (mx > -INFINITY) {
-    for (int s0 = part; s0 < nsplit; s0 += 4 * step) {
-      float l[4], x[4][V];
+    for (int s0 = part;;) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int s = s0 + u * step;
-        l[u] = -INFINITY;
-#pragma unroll
-        for (int i = 0; i < V; ++i) x[u][i] = 0.f;
-        if (s < nsplit) {
-          l[u] = a.part_lse[prow0 + s * pstep];
-          const float* po = a.part_o + (prow0 + s * pstep) * D + lane * V;
-          if constexpr (V == 4) {
-            const float4 y = *reinterpret_cast<const float4*>(po);
-            x[u][0] = y.x, x[u][1] = y.y, x[u][2] = y.z, x[u][3] = y.w;
-          } else {
-            const float2 y = *reinterpret_cast<const float2*>(po);
-            x[u][0] = y.x, x[u][1] = y.y;
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < U; ++u) {
         const float w = l[u] > -INFINITY ? __expf(l[u] - mx) : 0.f;
         den += w;
 #pragma unroll
         for (int i = 0; i < V; ++i) acc[i] += l[u] > -INFINITY ? w * x[u][i] : 0.f;  // (0 x NaN stays NaN)
       }
+      s0 += U * step;
+      if (s0 >= nsplit) break;
+      load(s0);
     }
   }
 #pragma unroll
@@ -1835,7 +1867,7 @@ static int launch_decode_t(const DecodeArgs& a_in, int head_blocks, cudaStream_t
   const int ss_bytes = Stage::ss_bytes(a_in.hb) * (a_in.ss_tma == 1 ? 4 : 1);  // 16 bytes per entry when the replicas come along
   const size_t stage_bytes = 2 * size_t(kv_bytes) + 2 * size_t(ss_bytes);
   const size_t qbytes = size_t(kDecConsumerWarps) * ROWS * (D * 2);
-  const size_t cmb = size_t(kDecConsumerWarps) * ROWS * (D + 2) * 4;
+  const size_t cmb = size_t(kDecConsumerWarps) * ROWS * cmb_pitch(D) * 4;
   int stages = int(DecOccupancy<kFmt, MT>::kRingBudget / stage_bytes);
   stages = stages > kDecMaxStages ? kDecMaxStages : stages;
   const int q_stages = kQuant ? int((qbytes + stage_bytes - 1) / stage_bytes) : 0;  // only the quantised paths stage Q
@@ -1864,8 +1896,10 @@ static int launch_decode_t(const DecodeArgs& a_in, int head_blocks, cudaStream_t
   if (e != cudaSuccess) return cuda_fail("decode_splitk_kernel launch", e);
   if (a.split_k > 1) {
     const int64_t rows = int64_t(a.batch) * a.kv_heads * a.rows;
-    constexpr int per_cta = kMergeWarpsPerCta / kMergeWarpsPerRow;
-    e = launch_early(decode_merge_kernel<D>, unsigned((rows + per_cta - 1) / per_cta), kMergeWarpsPerCta * 32, 0, stream, a);
+    if (rows <= 2 * sm_count())
+      e = launch_early(decode_merge_kernel<D, 8, 8>, unsigned(rows), kMergeWarpsPerCta * 32, 0, stream, a);
+    else
+      e = launch_early(decode_merge_kernel<D, 4, 4>, unsigned((rows + 1) / 2), kMergeWarpsPerCta * 32, 0, stream, a);
     if (e != cudaSuccess) return cuda_fail("decode_merge_kernel launch", e);
   }
   return XFB200_OK;
@@ -1902,9 +1936,11 @@ extern "C" size_t xfb200_decode_scratch_bytes(int32_t batch, int32_t mq, int32_t
 //   Where chunks of 1280 tokens fill the machine four times over: those (measured optimum for every cache format at 8 kv heads per
 // CTA: 24-32 chunks of a 32k context).
 //   Below: what a small model of the launch says is fastest.  A CTA costs about 3 us before and after its tokens; these come at
-// its share of the memory bandwidth, at most 90 GB/s; the CTAs run in waves of one per SM (two where that many fit); partials
-// are written and read once at 5 TB/s (516 bytes a row, head dim 128; 64, with half of that, keeps the same rule), and the merge costs 2 us.  Two sequences of 16384 keys, 2 kv heads, went from 128
-// chunks (256 CTAs, two waves, 128 partials per row) to 64: 16.4 + 28.7 us to the figures at decode_merge_kernel.
+// its share of the memory bandwidth, at most 60 GB/s for a CTA of a 16-bit cache and 45 for one of the two an SM takes of a quantised
+// one; the CTAs run in waves; partials (516 bytes a row, head dim 128; 64, with half of that, keeps the same rule) are written and
+// read once, at 2 TB/s for a 16-bit cache -- latency of the rounds that combine and merge them more than bytes -- and the merge costs
+// 2 us.  Two sequences of 16384 keys, 2 kv heads, 16 rows, f16, in chunks of 1024 / 768 / 512 keys, one head to a CTA: 13.8 / 12.1 /
+// 10.8 us; 384 / 256 keys, two heads to a CTA: 13.1 / 12.8.
 extern "C" int32_t xfb200_decode_split_k(int32_t batch, int64_t kv_bound, int32_t kv_heads, int32_t rows, int32_t row_bytes,
                                          int32_t quantised) {
   using namespace xfb;
@@ -1924,9 +1960,9 @@ extern "C" int32_t xfb200_decode_split_k(int32_t batch, int64_t kv_bound, int32_
     if (n > kDecMaxSplits) continue;
     const int hb = heads_per_cta(batch, kv_heads, row_blocks, n, quant, sms);
     const int64_t ctas = batch * (kv_heads / hb) * row_blocks * n, waves = (ctas + slots - 1) / slots;
-    const double gbs = std::min(90.0 / per_sm, 6400.0 / double(std::min(ctas, slots)));
+    const double gbs = std::min(quant ? 90.0 / per_sm : 60.0, 6400.0 / double(std::min(ctas, slots)));
     const double us = double(waves) * (3.0 + double(c * hb * 2 * row_bytes) / (gbs * 1e3)) +
-                      (n > 1 ? 2.0 + 2.0 * double(batch * kv_heads * n * rows) * 516.0 / 5e6 : 0.0);
+                      (n > 1 ? 2.0 + 2.0 * double(batch * kv_heads * n * rows) * 516.0 / (quant ? 5e6 : 2e6) : 0.0);
     if (us < best_us * 0.98) best_us = us, best = c;
   }
   return int32_t(chunks(best));
