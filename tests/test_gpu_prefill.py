@@ -592,6 +592,32 @@ def test_heads_of_a_group_share_a_tile(H, D, kind):
 
 
 @gpu
+@pytest.mark.parametrize("layout", ["dense", "causal", "bottom_right_gqa", "varlen"])
+@pytest.mark.parametrize("D", [136, 160, 184, 192, 200, 256])
+def test_head_dims_above_128(D, layout):
+    """One-tile items of the tcgen05 kernel: widths that are no multiple of 16 or 64, keys that end inside a step, more items than
+    SMs, queries without a key."""
+    require_cuda()
+    dtype = torch.bfloat16
+    if layout == "varlen":
+        lens = [1, 127, 300, 64, 129, 33]
+        q, k, v = rand_qkv(1, sum(lens), sum(lens), 1, 3, D, dtype, seed=D, gqa=False)
+        q, k, v = q[:, :, 0], k[:, :, 0], v[:, :, 0]
+        bias = ab.BlockDiagonalCausalMask.from_seqlens(lens, device="cuda")
+    elif layout == "bottom_right_gqa":
+        q, k, v = rand_qkv(1, 200, 131, 2, 4, D, dtype, seed=D)
+        bias = ab.LowerTriangularFromBottomRightMask()
+    else:
+        q, k, v = rand_qkv(3, 333, 333, 1, 17, D, dtype, seed=D, gqa=False)
+        q, k, v = q[:, :, 0], k[:, :, 0], v[:, :, 0]
+        bias = ab.LowerTriangularMask() if layout == "causal" else None
+    out, lse = fmha.memory_efficient_attention_forward_requires_grad(q, k, v, bias)
+    ro, rl = ref(q, k, v, bias)
+    assert_o_lse(out, lse, ro, rl, dtype, f"D={D} {layout}")
+    _status_ok()
+
+
+@gpu
 @pytest.mark.parametrize("causal", [False, True])
 @pytest.mark.parametrize("bias_dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("Mkv,wide,D", [(520, 520, 128), (517, 520, 64), (517, 517, 80), (3, 8, 128), (131, 136, 40)])

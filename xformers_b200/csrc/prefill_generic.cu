@@ -1,7 +1,7 @@
 // Generic attention-forward kernel on warp-level mma.sync (m16n8k16).
 //
 // Covers every shape the tcgen05 kernels do not take:
-// head dims above 128 (multiples of 8 up to 256), and inputs that a tensor map
+// an additive bias at head dims above 128 (multiples of 8 up to 256), the smallest calls there, and inputs that a tensor map
 // cannot describe; different value head dim is not supported.  Same mask model, same outputs.
 //
 // One CTA = 4 warps = one 64-row query tile of one (sequence, head); key tiles

@@ -37,9 +37,15 @@ static bool heads_flatten(const xfb200_strides& s, int G, int H, int64_t* stride
 int prefill_sm100_supported(const xfb200_prefill_params* p) {
   // The persistent kernel takes every head dim up to 128 that its tensor maps can describe (a multiple of 8), as tiles of 64 or
   // 128 columns: 64 x 197 rows x 16 heads of 80 columns, no mask, 75 us against 259 us on the mma.sync kernel (whole calls).
-  // Above 128 two output tiles do not fit the tensor memory.
+  // Above 128, without a bias, it takes items of one tile.
   const bool exact = p->head_dim == 64 || p->head_dim == 128;
-  if (p->head_dim > 128 || p->head_dim % 8 != 0) return 0;
+  if (p->head_dim > 256 || p->head_dim % 8 != 0) return 0;
+  if (p->head_dim > 128) {
+    if (p->kernel_path != XFB200_PREFILL_AUTO || p->bias != nullptr || p->kv_split != 0) return 0;
+    // One step of an mma.sync CTA (64 rows, 64 keys) and no more of them than SMs: nothing to pipeline (50 rows, 16 to 128 heads
+    // in all, D = 160 and 256: 9.3-10.5 us against 10.5-11; from 65 keys or rows on 13.5-18 against 10-10.8).
+    if (p->seqstart_q == nullptr && p->mq <= 64 && p->mkv <= 64 && int64_t(p->batch) * p->groups * p->heads_per_group <= sm_count()) return 0;
+  }
   if (!exact && p->kernel_path == XFB200_PREFILL_TCGEN05_CTA) return 0;
   if (!(p->scale > 0.f)) return 0;
   if (p->mq < 1 || p->batch < 1) return 0;
@@ -128,7 +134,7 @@ int prefill_sm100_launch(const xfb200_prefill_params* p, cudaStream_t stream) {
     // for the other's softmax and products (causal, 4 heads x 4096
     // rows 68.5 -> 61.8 us, 4 x 1024 25.1 -> 23.0; 8 heads x 700, no mask, 23.0 -> 21.0).
     const int64_t tiles = (rows + 127) / 128;
-    if (int64_t(G) * H / pack * p->batch * tiles <= sm_count() - a.sm_margin) a.q_tiles = int32_t(tiles), a.item_rows = 128;
+    if (D > 128 || int64_t(G) * H / pack * p->batch * tiles <= sm_count() - a.sm_margin) a.q_tiles = int32_t(tiles), a.item_rows = 128;
   }
   a.debug_flags = p->debug_flags;
   a.wait_budget = p->wait_budget_kcycles > 0 ? 1000LL * p->wait_budget_kcycles : kDefaultWaitBudgetCycles;

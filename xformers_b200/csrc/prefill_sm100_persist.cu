@@ -79,7 +79,7 @@ namespace pst {
 constexpr int kBM = 128;    // rows per query tile
 constexpr int kTiles = 2;   // query tiles per item
 constexpr int kBN = 128;    // keys per step
-constexpr int kStages = 2;  // depth of the K and of the V ring
+constexpr int kMaxStages = 2;  // depth of the K and of the V ring
 constexpr int kSched = 4;   // depth of the ring that announces work items
 constexpr int kThreads = 512;
 constexpr int kOutWarp0 = 8, kPvWarp0 = 12, kTmaWarp = 14, kQkWarp = 15;
@@ -114,7 +114,7 @@ struct Item {
 struct __align__(8) Barriers {
   uint64_t sched_full[kSched], sched_empty[kSched];
   uint64_t q_full[kTiles], q_empty[kTiles];
-  uint64_t k_full[kStages], v_full[kStages], k_empty[kStages], v_empty[kStages];
+  uint64_t k_full[kMaxStages], v_full[kMaxStages], k_empty[kMaxStages], v_empty[kMaxStages];
   uint64_t s_full[kTiles], s_empty;          // s_empty: the scores are in registers (the two tiles share one buffer)
   uint64_t p_half[kTiles], p_full[kTiles];   // p_half: the probabilities of keys 0-63 are stored
   uint64_t pv_done[kTiles];                  // P_t has been read, O_t is quiescent
@@ -127,10 +127,12 @@ struct __align__(8) Barriers {
 
 template <int D>
 struct Smem {
+  // above 128 columns an item is one tile (two outputs do not fit the tensor memory), and the rings hold one step
+  static constexpr int kQTiles = D > 128 ? 1 : kTiles, kStages = D > 128 ? 1 : kMaxStages;
   static constexpr int kQTile = kBM * D * 2;
   static constexpr int kKV = kBN * D * 2;
   static constexpr int kQ = 0;
-  static constexpr int kK = kQ + kTiles * kQTile;
+  static constexpr int kK = kQ + kQTiles * kQTile;
   static constexpr int kV = kK + kStages * kKV;
   static constexpr int kStats = kV + kStages * kKV;          // float2 [kTiles][kBM]: running maximum (log2 units), row sum
   static constexpr int kBar = kStats + kTiles * kBM * 8;
@@ -142,7 +144,7 @@ struct Smem {
 static_assert(sizeof(Barriers) <= 1024, "barrier block");
 
 // Columns of the tensor memory: scores (fp32, one buffer in which the two tiles take turns), probabilities (16-bit pairs), output
-// (fp32).  At D = 128 these are all 512 columns; at D = 64 a buffer of scores per tile would fit, but then nothing keeps the
+// (fp32).  At D = 128 these are all 512 columns, as at D = 256, where there is one tile; at D = 64 a buffer of scores per tile would fit, but then nothing keeps the
 // tiles half a step apart (4 x 4096 rows, 32 heads, no mask: 778 us with two buffers, 664 with one).
 template <int D>
 struct Tmem {
@@ -308,7 +310,7 @@ __device__ __forceinline__ bool decode_item(const Sm100Args& a, int order, int i
   return true;
 }
 
-// D: columns of the tiles (64 or 128).  kVariant:
+// D: columns of the tiles (64, 128 or 256).  kVariant:
 //   kExact   the head dim is D
 //   kPadded  the head dim a.head_dim is smaller than D; the copies fill the columns behind it with zeros, the products
 //            leave out what lies wholly behind it, the output is written up to it
@@ -344,7 +346,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
         mbar_init(&bar->sched_full[i], 1);
         mbar_init(&bar->sched_empty[i], kItemReaders);
       }
-      for (int i = 0; i < kStages; ++i) {
+      for (int i = 0; i < kMaxStages; ++i) {
         mbar_init(&bar->k_full[i], 1);
         mbar_init(&bar->k_empty[i], 1);
         mbar_init(&bar->v_full[i], 1);
@@ -445,11 +447,13 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           }
         };
         // one tile of 128 rows (Q, K or V), as blocks of 64 columns
+        const int blocks = D > 128 && kPad ? (head_dim + 63) / 64 : kHalves;
         auto load_tile = [&](int at, const CUtensorMap* tm, uint64_t* full, int head, int row, int tb) {
           if (elect_one()) {
-            mbar_expect_tx(full, L::kKV);
+            mbar_expect_tx(full, blocks * kHalfBytes);
 #pragma unroll
-            for (int hf = 0; hf < kHalves; ++hf) tma_load_4d(smem + at + hf * kHalfBytes, tm, full, hf * 64, head, row, tb);
+            for (int hf = 0; hf < kHalves; ++hf)
+              if (hf < blocks) tma_load_4d(smem + at + hf * kHalfBytes, tm, full, hf * 64, head, row, tb);
           }
         };
         // The V tile of a step is loaded behind the K tile of the step after it: its stage comes free a softmax later
@@ -462,7 +466,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
             return false;
           }
           load_tile(L::kV + vs * L::kKV, &a.tm_v, &bar->v_full[vs], pend_head, pend_row, pend_tb);
-          if (++vs == kStages) vs = 0, vph ^= 1;
+          if (++vs == L::kStages) vs = 0, vph ^= 1;
           pend_row = -1;
           return true;
         };
@@ -495,7 +499,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
             // (testing aid: the CTA that got the first item leaves out its last key tile, so that the wait for it runs out)
             if (!((a.debug_flags & 1) && cur.idx == 0 && j == cur.j_end - 1))
               load_tile(L::kK + ks * L::kKV, &a.tm_k, &bar->k_full[ks], cur.kv_head, row, cur.tb);
-            if (++ks == kStages) ks = 0, kph ^= 1;
+            if (++ks == L::kStages) ks = 0, kph ^= 1;
             if (!load_pending_v()) break;
             if (j == cur.j_begin) {
               // Q behind what does not wait for it: its buffers come free with the very last QK^T of the previous item
@@ -604,7 +608,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
               }
               if (code != 0) break;
               if (elect_one()) tc_commit(&bar->k_empty[st]);
-              if (++st == kStages) st = 0, ph ^= 1;
+              if (++st == L::kStages) st = 0, ph ^= 1;
             }
           }
         } else {
@@ -633,8 +637,9 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
               XFB_PROF_LAP(1)  // wait for V
               if (j >= jlo && j < jhi) {
                 const int n0 = n_base + j * kBN;
-                if (n0 + kBN > klen) {
-                  // V rows past the end of the sequence may hold anything; P is 0 there.
+                if (a.seqstart_k != nullptr && n0 + kBN > klen) {
+                  // V rows past the end of the sequence may hold anything; P is 0 there.  (Behind the end of the tensor, where
+                  // every sequence of a dense batch ends, the copy fills in zeros.)
                   // Both PV warps write the same zeros: no ordering between them is needed.
                   const int first = max(klen - n0, 0);
                   uint8_t* vt = smem + L::kV + st * L::kKV;
@@ -678,7 +683,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
                 XFB_PROF_COUNT(7)
               }
               if (elect_one()) tc_commit(&bar->v_empty[st]);
-              if (++st == kStages) st = 0, ph ^= 1;
+              if (++st == L::kStages) st = 0, ph ^= 1;
             }
           }
         }
@@ -1207,6 +1212,7 @@ int prefill_sm100_persist_launch(Sm100Args a, int head_dim, bool bf16, cudaStrea
   if (a.bias != nullptr && a.bias_dtype == (bf16 ? XFB200_BF16 : XFB200_F16))
     return head_dim > 64 ? persist_launch_d<128, pst::kBiasedSame>(a, bf16, stream) : persist_launch_d<64, pst::kBiasedSame>(a, bf16, stream);
   if (a.bias != nullptr) return head_dim > 64 ? persist_launch_d<128, pst::kBiased>(a, bf16, stream) : persist_launch_d<64, pst::kBiased>(a, bf16, stream);
+  if (head_dim > 128) return head_dim == 256 ? persist_launch_d<256, pst::kExact>(a, bf16, stream) : persist_launch_d<256, pst::kPadded>(a, bf16, stream);
   if (head_dim == 128) return persist_launch_d<128, pst::kExact>(a, bf16, stream);
   if (head_dim == 64) return persist_launch_d<64, pst::kExact>(a, bf16, stream);
   return head_dim > 64 ? persist_launch_d<128, pst::kPadded>(a, bf16, stream) : persist_launch_d<64, pst::kPadded>(a, bf16, stream);

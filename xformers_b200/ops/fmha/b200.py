@@ -5,7 +5,7 @@ Slots into the dispatcher next to the reference's forward operators
 tests/test_mem_eff_attention.py:104-111 reads it).  The arithmetic is done by
 ``xfb200_prefill_forward`` of libxfb200.so: a persistent TMA + tcgen05/TMEM
 kernel for head dims up to 128 (every mask, additive tensor biases included),
-an mma.sync kernel for the head dims above.
+and for those up to 256 without a bias; an mma.sync kernel for the rest.
 """
 
 from __future__ import annotations
