@@ -483,12 +483,38 @@ struct QuantRows {  // rows 2c and 2c + 1 of each n-tile
   int lim_min;          // below it nothing is masked for any row of this warp
 };
 
-// Q^T fragments' source: the row's largest magnitude and the power of two 2^k that brings it to [2^14, 2^15).  The f16 values
+// A query row as one of the consumers wants it, a quarter of it to each of the four lanes that share it: in 16-byte chunks 4 i + c
+// (kWords = 4) or 8-byte ones 4 i + c (kWords = 2), straight from global memory.  (Through shared memory, element by element, with
+// eight rows in the same banks, it took several us of every CTA: one sequence of 512 keys, 8 kv heads, 64 query heads, int4 / fp8 cache
+// 14.4 / 17.7 -> 10.9 / 15.0 us; 16 of up to 16384 keys, one kv head, 39.0 / 42.8 -> 24.4 / 35.8.)
+template <int D, int kWords, typename T>
+__device__ __forceinline__ void quant_load_q(const DecodeArgs& a, const DecWarp& w, int row, uint32_t (&x)[D / 8]) {
+  const bool live = row < a.rows;
+  const int qi = live ? row / a.q_per_kv : 0, h = live ? row % a.q_per_kv : 0;
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(reinterpret_cast<const T*>(a.q) + (int64_t(w.b) * a.mq + qi) * a.q_sm + int64_t(w.head) * a.q_sg + int64_t(h) * a.q_sh) +
+                        (w.lane & 3) * kWords;
+#pragma unroll
+  for (int i = 0; i < D / 8 / kWords; ++i) {
+    if constexpr (kWords == 4) {
+      const uint4 y = live ? __ldg(reinterpret_cast<const uint4*>(src + i * 16)) : make_uint4(0, 0, 0, 0);
+      x[4 * i] = y.x, x[4 * i + 1] = y.y, x[4 * i + 2] = y.z, x[4 * i + 3] = y.w;
+    } else {
+      const uint2 y = live ? __ldg(reinterpret_cast<const uint2*>(src + i * 8)) : make_uint2(0, 0);
+      x[2 * i] = y.x, x[2 * i + 1] = y.y;
+    }
+  }
+}
+
+// The power of two 2^k that brings the row's largest magnitude to [2^14, 2^15).  The f16 values
 // keep 11 bits down to 2^-28 of the row's maximum.
-template <int D, typename T>
-__device__ __forceinline__ int quant_q_exponent(const T* qrow, int c) {
+template <bool kBf16, int N>
+__device__ __forceinline__ int quant_q_exponent(const uint32_t (&x)[N]) {
   float amax = 0.f;
-  for (int d = c; d < D; d += 4) amax = fmaxf(amax, fabsf(float(qrow[d])));
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const float2 f = unpack2<kBf16>(x[i]);
+    amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
+  }
   amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
   amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
   const int e = int(__float_as_uint(amax) >> 23) - 127;
@@ -496,13 +522,21 @@ __device__ __forceinline__ int quant_q_exponent(const T* qrow, int c) {
 }
 __device__ __forceinline__ float exp2_int(int k) { return __uint_as_float(uint32_t(127 + k) << 23); }
 
-// Row sums and factors of n-tile `nt` (thread (r, c) has row r at hand), limits, and the empty state.
-template <int D, int NTQ, typename T>
-__device__ __forceinline__ void quant_rows_init(QuantRows<NTQ>& q, int nt, const T* qrow, int kexp, const DecodeArgs& a, const DecWarp& w) {
+// The words become f16 pairs of q * 2^kexp; row sums and factors of n-tile `nt` (thread (r, c) has a quarter of row r at hand),
+// limits, and the empty state.
+template <bool kBf16, int NTQ, int N>
+__device__ __forceinline__ void quant_rows_init(QuantRows<NTQ>& q, int nt, uint32_t (&x)[N], int kexp, const DecodeArgs& a, const DecWarp& w) {
   const int c = w.lane & 3;
   const float qmul = exp2_int(kexp);
   float sr = 0.f;  // the quad of row r adds up that row, then rows 2c, 2c+1 are fetched
-  for (int d = c; d < D; d += 4) sr += __half2float(__float2half_rn(float(qrow[d]) * qmul));
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const float2 f = unpack2<kBf16>(x[i]);
+    const __half2 h = __floats2half2_rn(f.x * qmul, f.y * qmul);
+    const float2 g = __half22float2(h);
+    sr += g.x + g.y;
+    x[i] = *reinterpret_cast<const uint32_t*>(&h);
+  }
   sr += __shfl_xor_sync(0xffffffffu, sr, 1);
   sr += __shfl_xor_sync(0xffffffffu, sr, 2);
   const float fac = exp2_int(-kexp) * a.scale_log2;
@@ -680,7 +714,7 @@ __device__ __forceinline__ void quant_rows_finish(QuantRows<NTQ>& q, const DecWa
 //    overhead is paid once for 32 tokens.
 // 64 sequences of 1024 to 32768 keys, 8 kv heads, 64 query heads, pages of 256:
 // 388 -> 290 us (2.84 -> 3.80 TB/s; 280 with V's even elements left where they
-// are).  314 instructions per sub-tile were 437; neither the issue slots (2.3 of 4)
+// are); 262 with Q read as registers want it.  314 instructions per sub-tile were 437; neither the issue slots (2.3 of 4)
 // nor the integer pipe (56 %) are full, so what is left is their dependent latency with
 // four warps per scheduler.
 // ---------------------------------------------------------------------------
@@ -691,7 +725,6 @@ __device__ __forceinline__ void consume_int4(const DecodeArgs& a, const DecWarp&
   constexpr int KS = D / 16;    // k-steps of K Q^T
   constexpr int MTV = D / 16;   // m-tiles of V^T P^T
   constexpr int WPT = D / 64;   // V words per thread and token
-  constexpr int kQRowBytes = D * 2;
   constexpr int kCmbRow = cmb_pitch(D);
   constexpr int U = DecStage<D, kFmtInt4>::kSubTiles;  // all of a stage in one step
   const int lane = w.lane, r = lane >> 2, c = lane & 3;
@@ -711,26 +744,19 @@ __device__ __forceinline__ void consume_int4(const DecodeArgs& a, const DecWarp&
   QuantRows<NTQ> rows;
 #pragma unroll
   for (int nt = 0; nt < NTQ; ++nt) {
-    const T* qrow = reinterpret_cast<const T*>(w.qs + (nt * 8 + r) * kQRowBytes);
-    const int kexp = quant_q_exponent<D>(qrow, c);
-    quant_rows_init<D>(rows, nt, qrow, kexp, a, w);
-    const float qmul = exp2_int(kexp);
+    // (chunk 4 i + c holds what k-steps 2 i and 2 i + 1 take: element pairs (e, e + 4))
+    uint32_t x[D / 8];
+    quant_load_q<D, 4, T>(a, w, w.row0 + nt * 8 + r, x);
+    const int kexp = quant_q_exponent<kBf16>(x);
+    quant_rows_init<kBf16>(rows, nt, x, kexp, a, w);
 #pragma unroll
     for (int ks = 0; ks < KS; ++ks) {
-      const T* q0 = qrow + (4 * (ks >> 1) + c) * 8;
-      const int e0 = (ks & 1) * 2;
-      auto pk = [qmul](const T* p, int i0, int i1) {
-        const __half2 h = __floats2half2_rn(float(p[i0]) * qmul, float(p[i1]) * qmul);
-        return *reinterpret_cast<const uint32_t*>(&h);
-      };
-      qf[nt][ks][0] = pk(q0, e0, e0 + 4);
-      qf[nt][ks][1] = pk(q0, e0 + 1, e0 + 5);
+      const int lo = 4 * (ks >> 1) + (ks & 1);
+      qf[nt][ks][0] = __byte_perm(x[lo], x[lo + 2], 0x5410);
+      qf[nt][ks][1] = __byte_perm(x[lo], x[lo + 2], 0x7632);
     }
   }
   quant_rows_limit(rows, w.chunk_hi);
-  // Q now lives in registers: release the staging area to the producer
-  __syncwarp();
-  if (lane == 0) mbar_arrive(w.q_done_bar);
 
   float acc[MTV][NTQ][4];
 #pragma unroll
@@ -1226,7 +1252,6 @@ __device__ __forceinline__ void consume_fp8(const DecodeArgs& a, const DecWarp& 
   constexpr int KS = D / 16;   // k-steps of K Q^T
   constexpr int MTV = D / 16;  // m-tiles of V^T P^T
   constexpr int WJ = D / 32;   // V words per thread and token
-  constexpr int kQRowBytes = D * 2;
   constexpr int kCmbRow = cmb_pitch(D);
   constexpr int kSps = DecStage<D, kFmtFp8>::kSubTiles;
   const int lane = w.lane, r = lane >> 2, c = lane & 3;
@@ -1240,23 +1265,14 @@ __device__ __forceinline__ void consume_fp8(const DecodeArgs& a, const DecWarp& 
   QuantRows<NTQ> rows;
 #pragma unroll
   for (int nt = 0; nt < NTQ; ++nt) {
-    const T* qrow = reinterpret_cast<const T*>(w.qs + (nt * 8 + r) * kQRowBytes);
-    const int kexp = min(quant_q_exponent<D>(qrow, c), 0);  // only downwards: f16 values of ordinary queries are exact
-    quant_rows_init<D>(rows, nt, qrow, kexp, a, w);
-    const float qmul = exp2_int(kexp);
+    uint32_t x[D / 8];
+    quant_load_q<D, 2, T>(a, w, w.row0 + nt * 8 + r, x);
+    const int kexp = min(quant_q_exponent<kBf16>(x), 0);  // only downwards: f16 values of ordinary queries are exact
+    quant_rows_init<kBf16>(rows, nt, x, kexp, a, w);
 #pragma unroll
-    for (int ks = 0; ks < KS; ++ks) {
-      const T* q0 = qrow + 16 * ks + 4 * c;
-      const __half2 h01 = __floats2half2_rn(float(q0[0]) * qmul, float(q0[1]) * qmul);
-      const __half2 h23 = __floats2half2_rn(float(q0[2]) * qmul, float(q0[3]) * qmul);
-      qf[nt][ks][0] = *reinterpret_cast<const uint32_t*>(&h01);
-      qf[nt][ks][1] = *reinterpret_cast<const uint32_t*>(&h23);
-    }
+    for (int ks = 0; ks < KS; ++ks) qf[nt][ks][0] = x[2 * ks], qf[nt][ks][1] = x[2 * ks + 1];
   }
   quant_rows_limit(rows, w.chunk_hi);
-  // Q now lives in registers: release the staging area to the producer
-  __syncwarp();
-  if (lane == 0) mbar_arrive(w.q_done_bar);
 
   float acc[MTV][NTQ][4];
 #pragma unroll
@@ -1374,6 +1390,7 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt, MT>::kCtasPerS
   // query rows of one kv head per CTA: MT m-tiles of 16 (16-bit cache) or MT
   // n-tiles of 8 (int4 and fp8 caches, transposed products)
   constexpr int ROWS = kQuant ? 8 * MT : 16 * MT;
+  constexpr bool kStageQ = kInt4 && NG > 1;
 
   // bytes in flight per SM are what hide HBM latency: the ring takes ~200 KB,
   // i.e. 3 stages of 64 KB (bf16, D = 128) up to 12 stages of 17 KB (int4)
@@ -1506,7 +1523,7 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt, MT>::kCtasPerS
           if (lane == 0) atomicCAS(a.status, 0, 1);
           return;
         }
-      } else if (kQuant && tile == a.q_first_stage) {
+      } else if (kStageQ && tile == a.q_first_stage) {
         if (!mbar_wait(&q_done_bar, 0)) {
           if (lane == 0) atomicCAS(a.status, 0, 3);
           return;
@@ -1608,12 +1625,12 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt, MT>::kCtasPerS
   const int row0 = rblk * ROWS;  // first query row (of this kv head) handled here
   const int R = a.rows;
 
-  // ---- int4 path: stage Q (this warp's head) in shared memory, zero rows beyond R.
-  // (The 16-bit path reads its fragments from global memory: a fragment load that
+  // ---- int4 with several groups: stage Q (this warp's head) in shared memory, zero rows beyond R.
+  // (The other paths read it from global memory: a fragment load that
   // nothing consumes yet could still be in flight when the staging area is handed
-  // back to the copy engine.  The int4 path converts what it loads before it
+  // back to the copy engine.  This one converts what it loads before it
   // arrives on q_done, so its loads have returned by then.)
-  if constexpr (kQuant) {
+  if constexpr (kStageQ) {
     uint8_t* qs = q_smem + warp * ROWS * kQRowBytes;
     const T* qg = reinterpret_cast<const T*>(a.q);
     for (int i = lane; i < ROWS * (D / 8); i += 32) {
@@ -1870,7 +1887,7 @@ static int launch_decode_t(const DecodeArgs& a_in, int head_blocks, cudaStream_t
   const size_t cmb = size_t(kDecConsumerWarps) * ROWS * cmb_pitch(D) * 4;
   int stages = int(DecOccupancy<kFmt, MT>::kRingBudget / stage_bytes);
   stages = stages > kDecMaxStages ? kDecMaxStages : stages;
-  const int q_stages = kQuant ? int((qbytes + stage_bytes - 1) / stage_bytes) : 0;  // only the quantised paths stage Q
+  const int q_stages = kFmt == kFmtInt4 && NG > 1 ? int((qbytes + stage_bytes - 1) / stage_bytes) : 0;  // the only path that stages Q
   if (stages < 2 || q_stages > stages) return set_error(XFB200_E_UNSUPPORTED, "decode: shared-memory ring too small for this shape");
   DecodeArgs a = a_in;
   a.stages = stages;
