@@ -1913,10 +1913,19 @@ static int launch_decode_t(const DecodeArgs& a_in, int head_blocks, cudaStream_t
   if (e != cudaSuccess) return cuda_fail("decode_splitk_kernel launch", e);
   if (a.split_k > 1) {
     const int64_t rows = int64_t(a.batch) * a.kv_heads * a.rows;
-    if (rows <= 2 * sm_count())
-      e = launch_early(decode_merge_kernel<D, 8, 8>, unsigned(rows), kMergeWarpsPerCta * 32, 0, stream, a);
+    auto merge = [&](void (*kern)(DecodeArgs), int warps_per_row) {
+      const int per_cta = kMergeWarpsPerCta / warps_per_row;
+      return launch_early(kern, unsigned((rows + per_cta - 1) / per_cta), kMergeWarpsPerCta * 32, 0, stream, a);
+    };
+    const int sms = sm_count();
+    if (rows <= 2 * sms)
+      e = merge(decode_merge_kernel<D, 8, 8>, 8);
+    else if (rows <= 4 * sms)
+      e = merge(decode_merge_kernel<D, 4, 4>, 4);
+    else if (rows <= 8 * sms)
+      e = merge(decode_merge_kernel<D, 2, 4>, 2);
     else
-      e = launch_early(decode_merge_kernel<D, 4, 4>, unsigned((rows + 1) / 2), kMergeWarpsPerCta * 32, 0, stream, a);
+      e = merge(decode_merge_kernel<D, 1, 4>, 1);
     if (e != cudaSuccess) return cuda_fail("decode_merge_kernel launch", e);
   }
   return XFB200_OK;
@@ -1977,7 +1986,7 @@ extern "C" int32_t xfb200_decode_split_k(int32_t batch, int64_t kv_bound, int32_
     if (n > kDecMaxSplits) continue;
     const int hb = heads_per_cta(batch, kv_heads, row_blocks, n, quant, sms);
     const int64_t ctas = batch * (kv_heads / hb) * row_blocks * n, waves = (ctas + slots - 1) / slots;
-    const double gbs = std::min(quant ? 90.0 / per_sm : 60.0, 6400.0 / double(std::min(ctas, slots)));
+    const double gbs = std::min(quant ? 40.0 / per_sm : 60.0, 6400.0 / double(std::min(ctas, slots)));
     const double us = double(waves) * (3.0 + double(c * hb * 2 * row_bytes) / (gbs * 1e3)) +
                       (n > 1 ? 2.0 + 2.0 * double(batch * kv_heads * n * rows) * 516.0 / (quant ? 5e6 : 2e6) : 0.0);
     if (us < best_us * 0.98) best_us = us, best = c;
