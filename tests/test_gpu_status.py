@@ -46,6 +46,32 @@ def test_a_wait_that_runs_out_is_reported_cleared_and_harmless(base):
 
 
 @gpu
+@pytest.mark.parametrize("form", ["one_stage_rings", "packed_heads", "bias", "more_items_than_sms"])
+def test_every_form_of_the_persistent_kernel_leaves_a_wait_that_runs_out(form):
+    """Rings of one step (head dim 256), tiles of (token, head) rows, the variants with a bias, launches whose other items go on:
+    all warps leave their loops together, the launch ends, the next one is right."""
+    require_cuda()
+    dtype, bias = torch.float16, None
+    if form == "one_stage_rings":
+        q, k, v = rand_qkv(1, 300, 300, 1, 2, 256, dtype, seed=4, gqa=False)
+    elif form == "packed_heads":
+        q, k, v = rand_qkv(1, 150, 300, 2, 8, 128, dtype, seed=5)
+    elif form == "bias":
+        q, k, v = rand_qkv(1, 300, 300, 1, 2, 64, dtype, seed=6, gqa=False)
+        bias = torch.randn(1, 1, 2, 300, 300, device="cuda")
+    else:
+        q, k, v = rand_qkv(2, 300, 300, 1, 100, 64, dtype, seed=7, gqa=False)
+    assert P.prefill_device_status() == 0
+    fmha.memory_efficient_attention_forward(q, k, v, bias, op=_withheld(P.FwOp))
+    with pytest.raises(RuntimeError, match="gave up a bounded wait"):
+        P.check_device_status()
+    out, lse = fmha.memory_efficient_attention_forward_requires_grad(q, k, v, bias, op=P.FwOp)
+    ro, rl = ref(q, k, v, bias.cpu() if bias is not None else None)
+    assert_o_lse(out, lse, ro, rl, dtype, f"{form}: launch after a reported time-out")
+    assert P.prefill_device_status() == 0
+
+
+@gpu
 def test_status_calls_through_the_c_abi():
     require_cuda()
     lib = _lib.load()

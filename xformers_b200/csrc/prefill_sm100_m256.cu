@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_m256_kernel(const _
         const int it = j - j_begin, st = it % kStagesK, use = it / kStagesK;
         const int sv = it % kStagesV, use_v = it / kStagesV;
         const int row = k_row0 + n_base + j * kBN;
-        if (use > 0 && !mbar_wait(&bar->k_empty[st], (use - 1) & 1, abort_flag, a.wait_budget)) {
+        if (use > 0 && !mbar_wait_lane(&bar->k_empty[st], (use - 1) & 1, abort_flag, a.wait_budget)) {
           give_up(a, 11);
           *abort_flag = 1;
           break;
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_m256_kernel(const _
           for (int hf = 0; hf < kHalves; ++hf)
             tma_load_4d(smem + L::kK + st * L::kKV + hf * kHalfBytes, &a.tm_k, &bar->k_full[st], hf * 64, kv_head, row, tb);
         }
-        if (use_v > 0 && !mbar_wait(&bar->v_empty[sv], (use_v - 1) & 1, abort_flag, a.wait_budget)) {
+        if (use_v > 0 && !mbar_wait_lane(&bar->v_empty[sv], (use_v - 1) & 1, abort_flag, a.wait_budget)) {
           give_up(a, 12);
           *abort_flag = 1;
           break;

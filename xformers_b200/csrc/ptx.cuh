@@ -52,17 +52,26 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // Bounded wait: gives up after ~0.2 s of SM clock (far beyond any legitimate
 // wait inside these kernels) or as soon as `abort_flag` (shared memory, set by
 // a sibling warp that already gave up) becomes non-zero.
+//   Made by a whole warp, whose lanes all get the same answer: what follows a wait (elect.sync, shuffles, tensor-memory loads,
+// mma) takes the warp as a whole, and a lane that left the loop on the flag or the clock while others saw the phase would leave
+// them waiting for it there without a bound.
 constexpr long long kWaitBudgetCycles = 400000000LL;
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const volatile uint32_t* abort_flag = nullptr,
                                           long long budget_cycles = kWaitBudgetCycles) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   // (units of 1024 clocks in 32 bits: every wait of a kernel has a copy of this loop in its instruction stream)
   const uint32_t t0 = uint32_t(clock64() >> 10), budget = uint32_t(budget_cycles >> 10);
   for (;;) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (abort_flag != nullptr && *abort_flag != 0) return false;
-    if (uint32_t(clock64() >> 10) - t0 > budget) return false;
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if (__any_sync(0xffffffffu, (abort_flag != nullptr && *abort_flag != 0) || uint32_t(clock64() >> 10) - t0 > budget)) return false;
   }
+}
+// The same for a single lane.
+__device__ __forceinline__ bool mbar_wait_lane(uint64_t* bar, uint32_t parity, const volatile uint32_t* abort_flag, long long budget_cycles) {
+  const uint32_t t0 = uint32_t(clock64() >> 10), budget = uint32_t(budget_cycles >> 10);
+  while (!mbar_try_wait(bar, parity))
+    if (*abort_flag != 0 || uint32_t(clock64() >> 10) - t0 > budget) return mbar_try_wait(bar, parity);
+  return true;
 }
 
 // ----------------------------------------------------------------------- TMA
