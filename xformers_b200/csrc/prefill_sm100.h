@@ -33,6 +33,7 @@ struct Sm100Args {
   int32_t q_tiles;  // blocks of query rows per sequence (static bound): 256 rows, or item_rows in the persistent kernel
   int32_t item_rows;  // persistent kernel: rows of a work item, 256 (two tiles) or 128 (one)
   int32_t pack_shift; // persistent kernel: log2 of the heads of a GQA group that share a tile (row = token << pack_shift | head)
+  int32_t n_items;    // persistent kernel: work items of the launch
   uint32_t epoch;   // differs from launch to launch, never 0
   int32_t debug_flags;
   long long wait_budget;  // SM clocks after which a wait gives up

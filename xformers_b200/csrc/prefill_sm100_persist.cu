@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
   float2* stats = reinterpret_cast<float2*>(smem + L::kStats);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const int n_items = ((a.q_tiles * a.groups * a.heads_per_group) >> a.pack_shift) * a.batch;
+  const int n_items = a.n_items;
   const int pack_shift = kBias ? 0 : a.pack_shift;
   const int tile_rows = kBM >> pack_shift;  // query rows (tokens) of a tile
   const long long budget = a.wait_budget;
@@ -1175,7 +1175,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
 }
 
 template <int D, bool kBf16, int kVariant>
-static int launch_t(const Sm100Args& a, cudaStream_t stream) {
+static int launch_t(Sm100Args a, cudaStream_t stream) {
   auto kern = prefill_sm100_persist_kernel<D, kBf16, kVariant>;
   constexpr int smem = kVariant == kBiased || kVariant == kBiasedSame ? Smem<D>::kTotalBiased : Smem<D>::kTotal;
   static_assert(smem <= 227 * 1024, "shared memory of one CTA");
@@ -1186,6 +1186,7 @@ static int launch_t(const Sm100Args& a, cudaStream_t stream) {
   }
   const int64_t items = ((int64_t(a.groups) * a.heads_per_group) >> a.pack_shift) * a.batch * a.q_tiles;
   if (items > 0x3fffffff) return set_error(XFB200_E_UNSUPPORTED, "prefill: too many blocks of query rows");
+  a.n_items = int32_t(items);
   int sms = sm_count() - a.sm_margin;
   if (sms < 1) sms = 1;
   const unsigned grid = unsigned(items < sms ? items : sms);
