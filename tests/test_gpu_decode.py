@@ -495,3 +495,25 @@ def test_mqa_decoding(op, dtype, B, Mkv, H, K):
     out, lse = fmha.memory_efficient_attention_forward_requires_grad(q, k, v, op=op)
     ro, rl = oracle.ref_attention_with_lse(q.float().cpu(), k.float().cpu(), v.float().cpu(), None)
     assert_o_lse(out, lse, ro, rl, dtype, f"mqa decoding K={K}", o_scale=3.0)
+
+
+@gpu
+@pytest.mark.parametrize("D,dtype", [(128, torch.float16), (64, torch.bfloat16)])
+@pytest.mark.parametrize("rows_per_sm,split_k", [(0.1, 17), (0.1, 72), (1.9, 5), (3, 40), (6, 20), (9, 10), (9, 36)])
+def test_merge_of_the_chunks_in_every_form(rows_per_sm, split_k, D, dtype):
+    """Eight, four, two and one warp per row, each with more chunks than one round of its loads takes and with fewer: the number of
+    warps depends on the rows per SM and on the chunks.  Sequences without keys, with one key, with fewer chunks than the bound."""
+    require_cuda()
+    kv_heads, group, padding = 4, 4, split_k * 64
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    bsz = max(1, int(rows_per_sm * sms) // (kv_heads * group))
+    g = torch.Generator().manual_seed(split_k)
+    q = torch.randn(1, bsz, kv_heads, group, D, generator=g).to(dtype).cuda()
+    k, v = (torch.randn(1, bsz * padding, kv_heads, 1, D, generator=g).to(dtype).cuda().expand(-1, -1, -1, group, -1) for _ in range(2))
+    lens = [padding, 0, 1, padding - 63][:bsz] + torch.randint(0, padding + 1, (max(0, bsz - 4),), generator=g).tolist()
+    bias = ab.BlockDiagonalPaddedKeysMask.from_seqlens([1] * bsz, padding, lens, device="cuda")
+    op = S.FwOp_Map[split_k]
+    out, lse = fmha.memory_efficient_attention_forward_requires_grad(q, k, v, bias, op=op)
+    ro, rl = ref(q, k, v, bias)
+    assert_o_lse(out, lse, ro, rl, dtype, f"{bsz * kv_heads * group} rows, {split_k} chunks")
+    assert torch.equal(out, fmha.memory_efficient_attention_forward(q, k, v, bias, op=op))

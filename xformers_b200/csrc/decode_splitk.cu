@@ -1737,12 +1737,11 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt, MT>::kCtasPerS
 }
 
 // ---------------------------------------------------------------------------
-// Merge of the per-chunk partials of each sequence.  Latency bounds it, not bytes: what a row needs is asked for in one round
-// of loads -- the log-sum-exps of all chunks for the maximum, and for each of the row's kWarpsPerRow warps eight
-// (or four) of its chunks with their log-sum-exps -- where the partials used to wait for the maximum.  Few rows get eight warps each
-// and cover 64 chunks in that round (4 sequences of 1000 keys, 9.4 -> 8.5 us for both kernels); many rows hide one another's latency,
-// and registers for eight chunks would cost them CTAs (4096 rows, 26 chunks: 5 us).  Lengths are read before the split kernel
-// has ended: it began only when whatever wrote them had.
+// Merge of the per-chunk partials of each sequence.  Latency bounds it, not bytes: what a row needs is asked for in rounds
+// of loads -- the log-sum-exps of all chunks for the maximum, and for each of the row's kWarpsPerRow warps U of its chunks with their
+// log-sum-exps, which do not wait for the maximum (4 sequences of 1000 keys: 9.4 -> 8.5 us for both kernels).  How many warps a row
+// gets is chosen at the launch.  Lengths are read before the split kernel has ended, which is right only because that kernel lets this
+// one begin behind its own wait: whatever wrote the lengths has ended then.
 // Every chunk goes to a fixed warp and the warps are added up in order,
 // whatever the number of chunks, so the result is deterministic and does not
 // depend on a bound.  Only the chunks that exist for sequence b are read.
@@ -1917,12 +1916,17 @@ static int launch_decode_t(const DecodeArgs& a_in, int head_blocks, cudaStream_t
       const int per_cta = kMergeWarpsPerCta / warps_per_row;
       return launch_early(kern, unsigned((rows + per_cta - 1) / per_cta), kMergeWarpsPerCta * 32, 0, stream, a);
     };
+    // Warps per row.  Few rows have many SMs to themselves and are as long as their rounds of loads; many rows hide one another's
+    // latency, and more warps each are more CTAs to get through.  us of both kernels with 8 / 4 / 2 / 1 warps per row, kv heads of
+    // 8 query heads, the chosen form first: 256 rows in 4 chunks (bf16) 27.2 (4), 28.0 / 27.3 / 27.4; in 64 chunks 40.1 (8), 42.0 /
+    // 43.8 / 46.9; 1024 rows in 16 chunks (int4) 43.9 (2), 49.9 / 45.0 / 45.2; 4096 rows in 16 chunks 138.1 (1), 161.2 / 140.6 /
+    // 138.4; in 64 chunks 209.7 (2), 225.6 / 209.4 / 214.5.
     const int sms = sm_count();
-    if (rows <= 2 * sms)
+    if (rows <= 2 * sms && a.split_k > 16)
       e = merge(decode_merge_kernel<D, 8, 8>, 8);
     else if (rows <= 4 * sms)
       e = merge(decode_merge_kernel<D, 4, 4>, 4);
-    else if (rows <= 8 * sms)
+    else if (rows <= 8 * sms || a.split_k > 32)
       e = merge(decode_merge_kernel<D, 2, 4>, 2);
     else
       e = merge(decode_merge_kernel<D, 1, 4>, 1);
