@@ -504,7 +504,8 @@ def test_merge_of_the_chunks_in_every_form(rows_per_sm, split_k, D, dtype):
     """Eight, four, two and one warp per row, each with more chunks than one round of its loads takes and with fewer: the number of
     warps depends on the rows per SM and on the chunks.  Sequences without keys, with one key, with fewer chunks than the bound."""
     require_cuda()
-    kv_heads, group, padding = 4, 4, split_k * 64
+    kv_heads, group = (8, 2) if rows_per_sm >= 6 else (4, 4)  # (eight heads in a CTA: one warp to a head)
+    padding = split_k * 64
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     bsz = max(1, int(rows_per_sm * sms) // (kv_heads * group))
     g = torch.Generator().manual_seed(split_k)

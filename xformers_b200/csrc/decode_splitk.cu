@@ -18,6 +18,7 @@
 // Lengths and page tables are read from device memory at run time; the grid
 // depends on static bounds only.
 #include <algorithm>
+#include <type_traits>
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -1678,12 +1679,7 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt, MT>::kCtasPerS
     const int col = (i % kCols) * 4, hh = (i / kCols) & (hb - 1), rr = (i / kCols) >> hb_shift;
     const float* src = cmb + (hh * ROWS + rr) * kCmbRow;
     const int pitch = (ROWS * kCmbRow) << hb_shift;  // from a warp to the next one of the same head
-    float mx = -INFINITY;
-#pragma unroll
-    for (int w2 = 0; w2 < kDecConsumerWarps; ++w2)
-      if (w2 < wph) mx = fmaxf(mx, src[w2 * pitch + D]);
-    const float m_use = mx == -INFINITY ? 0.f : mx;
-    float den = 0.f;
+    float m_use = 0.f, den = 0.f;
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
     auto add = [&](float2 ml, float4 x) {
       const bool any = ml.x != -INFINITY;  // (a warp without a visible token may hold anything)
@@ -1694,21 +1690,39 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt, MT>::kCtasPerS
     };
     auto m_l = [&](int w2) { return *reinterpret_cast<const float2*>(src + w2 * pitch + D); };
     auto part = [&](int w2) { return *reinterpret_cast<const float4*>(src + w2 * pitch + col); };
+    auto maximum = [&](auto n) {
+      float mx = -INFINITY;
+#pragma unroll
+      for (int w2 = 0; w2 < decltype(n)::value; ++w2)
+        if (w2 < wph) mx = fmaxf(mx, src[w2 * pitch + D]);
+      m_use = mx == -INFINITY ? 0.f : mx;
+    };
     if constexpr (kQuant) {
+      maximum(std::integral_constant<int, kDecConsumerWarps>{});
       // (partials held in registers at once would be registers that the main loop has to do without: 4 % of the fp8 case)
 #pragma unroll 8
       for (int w2 = 0; w2 < wph; ++w2) add(m_l(w2), part(w2));
     } else {
-      float2 ml[kDecConsumerWarps];
-      float4 x[kDecConsumerWarps];
+      auto combine = [&](auto n) {
+        constexpr int N = decltype(n)::value;
+        float2 ml[N];
+        float4 x[N];
+        maximum(n);
 #pragma unroll
-      for (int w2 = 0; w2 < kDecConsumerWarps; ++w2) {
-        ml[w2] = make_float2(-INFINITY, 0.f);
-        x[w2] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (w2 < wph) ml[w2] = m_l(w2), x[w2] = part(w2);
-      }
+        for (int w2 = 0; w2 < N; ++w2) {
+          ml[w2] = make_float2(-INFINITY, 0.f);
+          x[w2] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (w2 < wph) ml[w2] = m_l(w2), x[w2] = part(w2);
+        }
 #pragma unroll
-      for (int w2 = 0; w2 < kDecConsumerWarps; ++w2) add(ml[w2], x[w2]);
+        for (int w2 = 0; w2 < N; ++w2) add(ml[w2], x[w2]);
+      };
+      // (Eight heads in a CTA are a warp each: one partial per row, and as many rows as there are.  Through the eight-fold form 64 sequences
+      // of 8192 keys, 64 query heads, in 64 chunks took 463 us, 16 in 32 chunks 115 -- with a warp per row 454 and 113 -- now 402 and 105.)
+      if (wph == 1)
+        combine(std::integral_constant<int, 1>{});
+      else
+        combine(std::integral_constant<int, kDecConsumerWarps>{});
     }
     const float inv = den > 0.f ? 1.f / den : 0.f;
     const float lse = den > 0.f ? (m_use + log2f(den)) * 0.6931471805599453f : -INFINITY;
