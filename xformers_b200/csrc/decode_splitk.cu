@@ -1421,6 +1421,7 @@ __global__ void __launch_bounds__(kDecThreads, DecOccupancy<kFmt, MT>::kCtasPerS
     mbar_fence_init();
     if (a.copy_mode == 3) prefetch_tensormap(&a.tm_k), prefetch_tensormap(&a.tm_v);
   }
+  // (In this order: the merge reads the lengths before its own wait, so it must not begin before whatever wrote them has ended.)
   grid_dep_wait();
   grid_dep_launch();
 

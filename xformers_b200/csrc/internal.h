@@ -72,7 +72,8 @@ int prefill_sm100_launch(const xfb200_prefill_params* p, cudaStream_t stream);
 int prefill_generic_launch(const xfb200_prefill_params* p, cudaStream_t stream);
 
 // Launch that may begin while the kernel ahead of it in the stream still runs.  Only for kernels whose every CTA calls
-// grid_dep_wait() before it touches memory: what is saved is the launch itself and what the kernel does before that call, 1-2 us
+// grid_dep_wait() before it touches memory (a kernel launched behind one of the library's own, which lets it begin after its own wait, may
+// read before that what neither writes: decode_merge_kernel the lengths): what is saved is the launch itself and what the kernel does before that call, 1-2 us
 // of a decoding step's 3-6 us kernels.  In a captured stream it becomes an edge of the same kind.
 //   A kernel that leaves SMs free for other streams (sm_margin) neither is launched this way nor lets the next one begin: CTAs that
 // only wait would fill those SMs.
