@@ -1981,11 +1981,13 @@ extern "C" size_t xfb200_decode_scratch_bytes(int32_t batch, int32_t mq, int32_t
 //   Where chunks of 1280 tokens fill the machine four times over: those (measured optimum for every cache format at 8 kv heads per
 // CTA: 24-32 chunks of a 32k context).
 //   Below: what a small model of the launch says is fastest.  A CTA costs about 3 us before and after its tokens; these come at
-// its share of the memory bandwidth, at most 60 GB/s for a CTA of a 16-bit cache and 45 for one of the two an SM takes of a quantised
-// one; the CTAs run in waves; partials (516 bytes a row, head dim 128; 64, with half of that, keeps the same rule) are written and
+// its share of the memory bandwidth, at most 60 GB/s for a CTA of a 16-bit cache and 40 for an SM with a quantised one, 20 for each of
+// the two CTAs it takes where these have one tile of rows (the consumer's rate, not the memory's); the CTAs run in waves; partials (516 bytes a row, head dim 128; 64, with half of that, keeps the same rule) are written and
 // read once, at 2 TB/s for a 16-bit cache -- latency of the rounds that combine and merge them more than bytes -- and the merge costs
 // 2 us.  Two sequences of 16384 keys, 2 kv heads, 16 rows, f16, in chunks of 1024 / 768 / 512 keys, one head to a CTA: 13.8 / 12.1 /
-// 10.8 us; 384 / 256 keys, two heads to a CTA: 13.1 / 12.8.
+// 10.8 us; 384 / 256 keys, two heads to a CTA: 13.1 / 12.8.  Quantised, with 90 GB/s to an SM instead of 40, 1 to 64 sequences of 512 to 32768 keys:
+// slower or as fast throughout.  int4, 8 kv heads of 8 query heads: 4 of 32768 keys in 43 chunks 60.4 us, in 64 48.1; 8 of 8192 in 22 / 32
+// chunks 37.9 / 31.7; 2 of 32768 in 86 / 128 37.9 / 33.8; fp8, one kv head of 16: 8 of 512 keys in 1 / 4 chunks 16.4 / 13.3.
 extern "C" int32_t xfb200_decode_split_k(int32_t batch, int64_t kv_bound, int32_t kv_heads, int32_t rows, int32_t row_bytes,
                                          int32_t quantised) {
   using namespace xfb;
