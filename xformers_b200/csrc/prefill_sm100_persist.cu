@@ -69,6 +69,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "internal.h"
 #include "prefill_sm100.h"
 #include "ptx.cuh"
@@ -136,7 +138,7 @@ struct Smem {
   static constexpr int kV = kK + kStages * kKV;
   static constexpr int kStats = kV + kStages * kKV;          // float2 [kTiles][kBM]: running maximum (log2 units), row sum
   static constexpr int kBar = kStats + kTiles * kBM * 8;
-  static constexpr int kBias = kBar + 1024;  // kBiased only: one unit of 32 rows x 64 bytes for each softmax warp
+  static constexpr int kBias = kBar + 1024;  // with a bias only: one unit of 32 rows x 64 bytes for each softmax warp
   static constexpr int kBiasUnit = 32 * 64;
   static constexpr int kTotal = kBar + 1024 + 1024;
   static constexpr int kTotalBiased = kTotal + 8 * kBiasUnit;
@@ -314,16 +316,14 @@ __device__ __forceinline__ bool decode_item(const Sm100Args& a, int order, int i
 //   kExact   the head dim is D
 //   kPadded  the head dim a.head_dim is smaller than D; the copies fill the columns behind it with zeros, the products
 //            leave out what lies wholly behind it, the output is written up to it
-//   kBiased  an additive bias of any type; the head dim may be D or smaller
-//   kBiasedSame  the same for a bias of the type of q, which the step then knows at compile time (with the type asked for at
-//                every pair of scores, a step of 128 keys took 6000 clocks, without a bias 2100: 2 x 2048 x 2048, 8 heads,
-//                bf16: 96 -> 82 us)
-constexpr int kExact = 0, kPadded = 1, kBiased = 2, kBiasedSame = 3;
+//   kBiasedSame, kBiasedOther, kBiasedF32  an additive bias of the type of q, of the other 16-bit type, of 32 bits, which the step
+//            knows at compile time; the head dim may be D or smaller
+constexpr int kExact = 0, kPadded = 1, kBiasedSame = 2, kBiasedOther = 3, kBiasedF32 = 4;
 template <int D, bool kBf16, int kVariant>
 __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(const __grid_constant__ Sm100Args a) {
   using L = Smem<D>;
   using T = Tmem<D>;
-  constexpr bool kPad = kVariant != kExact, kBias = kVariant == kBiased || kVariant == kBiasedSame, kBiasSame = kVariant == kBiasedSame;
+  constexpr bool kPad = kVariant != kExact, kBias = kVariant >= kBiasedSame, kBiasF32 = kVariant == kBiasedF32;
   constexpr int kHalves = D / 64;
   extern __shared__ uint8_t smem_dyn[];
   uint8_t* smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);  // an offset, so that the compiler keeps seeing shared memory
@@ -877,15 +877,18 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
         tc_wait_st();
       };
 
-      // ---- additive bias (kBiased).  Bound by how its bytes reach the registers: a row per thread is the layout of the
+      // ---- additive bias.  Bound by how its bytes reach the registers: a row per thread is the layout of the
       // scores, and reading memory that way costs one sector request per element (2048 x 2048 x 16 heads, bf16: 600 us).
       // A warp therefore reads its 32 rows in units of 64 bytes per row, four lanes to a row and 16 bytes to a lane, holds
       // the units of a step in registers from before the wait for the scores on, and turns one after the other into
       // rows through 2 KB of shared memory (16-byte chunks XOR-ed with row / 2, no bank conflict either way): 69 us for the
       // same call (34 GFLOP, 134 MB of bias).  A unit is
-      // 32 columns of a 16-bit bias (four units: a step) or 16 of an f32 one (four: half a step).
-      const bool bias_f32 = !kBiasSame && a.bias_dtype == XFB200_F32;
-      const bool bias_bf16 = kBiasSame ? kBf16 : a.bias_dtype == XFB200_BF16;
+      // 32 columns of a 16-bit bias (four units: a step) or 16 of an f32 one (eight).
+      //   An f32 bias takes 128 registers a step, as do the scores.  So its scores come 32 at a time, get their bias and go back to tensor
+      // memory, from where the step reads them as it does without a bias; six units are asked for before the wait, the last two when
+      // the first two are through.  With row and half a step of bias in registers together, the second half asked for when the first was
+      // used up, the step spilled, and the type asked for at run time made it worse: 3 x 3000 x 3000, 12 heads of 64, bf16, f32 bias 457
+      // -> 369 us (413 before the row was kept in registers), 8 heads x 700, causal, 39.8 -> 35.6; f16 with a bf16 bias 329 -> 271 and 31.7 -> 27.6.
       constexpr float kLog2e = 1.4426950408889634f;
       const uint64_t scale2 = f2_pack(a.scale_log2, a.scale_log2), log2e2 = f2_pack(kLog2e, kLog2e);
       uint8_t* const bias_smem = smem + L::kBias + warp * L::kBiasUnit;
@@ -893,8 +896,8 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
       // already, and what the bias holds there, a NaN perhaps, must not meet that.  (Masking behind the addition instead costs the
       // step registers: 75.5 -> 86.7 us for 2 x 2048 x 2048, 8 heads, no mask at all.)  `whole`: a step of which every row and key
       // counts, and rows on 16-byte boundaries; its loads need no test (the tests cost that call 3.4 us).
-      auto bias_load = [&](uint4* w, int64_t off, int mt0, int qlen, int col_first, int n_keys, int rel_lo, int rel_hi, bool whole) {
-        const int esz = bias_f32 ? 4 : 2, per16 = 16 / esz;
+      auto bias_load = [&](uint4* w, auto n_units, int64_t off, int mt0, int qlen, int col_first, int n_keys, int rel_lo, int rel_hi, bool whole) {
+        constexpr int kUnits = decltype(n_units)::value, esz = kBiasF32 ? 4 : 2, per16 = 16 / esz;
         if (whole) {
           const int r = mt0 + (warp & 3) * 32 + (lane >> 2);
           const uint8_t* src = reinterpret_cast<const uint8_t*>(a.bias) + (off + int64_t(r) * a.bias_m + col_first + (lane & 3) * per16) * esz;
@@ -902,7 +905,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
 #pragma unroll
           for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int u = 0; u < 4; ++u) w[u * 4 + i] = __ldg(reinterpret_cast<const uint4*>(src + i * step + u * 64));
+            for (int u = 0; u < kUnits; ++u) w[u * 4 + i] = __ldg(reinterpret_cast<const uint4*>(src + i * step + u * 64));
           return;
         }
 #pragma unroll
@@ -911,7 +914,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           const int lo = r + rel_lo, hi = min(r + rel_hi, n_keys);
           const uint8_t* src = reinterpret_cast<const uint8_t*>(a.bias) + (off + int64_t(r) * a.bias_m) * esz;
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
+          for (int u = 0; u < kUnits; ++u) {
             const int col = col_first + (u * 4 + (lane & 3)) * per16;
             uint4 x = make_uint4(0, 0, 0, 0);
             if (r < qlen && col < hi) {
@@ -935,14 +938,14 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
         }
       };
       auto bias_prefetch = [&](int64_t off, int mt0, int qlen, int col_first, int n_keys) {
-        const int esz = bias_f32 ? 4 : 2;
+        constexpr int esz = kBiasF32 ? 4 : 2;
         const int r = mt0 + row;
         const uint8_t* src = reinterpret_cast<const uint8_t*>(a.bias) + (off + int64_t(r) * a.bias_m) * esz;
         for (int col = col_first; col < col_first + kBN; col += 128 / esz)
           if (r < qlen && col < n_keys) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + int64_t(col) * esz));
       };
-      // the scores of columns [32 chunk, 32 chunk + 32) of this thread's row become (score * scale + bias) * log2 e
-      auto bias_add = [&](uint32_t* sc, const uint4* w, int chunk) {
+      // 32 scores of this thread's row become (score * scale + bias) * log2 e; w: the unit (two, f32) of their columns
+      auto bias_add = [&](uint32_t* sc, const uint4* w) {
         auto to_rows = [&](int u, uint4 (&mine)[4]) {
 #pragma unroll
           for (int i = 0; i < 4; ++i)
@@ -953,11 +956,11 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           __syncwarp();
         };
         auto add = [&](int c, float x) { sc[c] = __float_as_uint(fmaf(__uint_as_float(sc[c]), a.scale_log2, x * kLog2e)); };
-        if (bias_f32) {
+        if constexpr (kBiasF32) {
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             uint4 mine[4];
-            to_rows((chunk & 1) * 2 + h, mine);
+            to_rows(h, mine);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               add(h * 16 + k * 4, __uint_as_float(mine[k].x)), add(h * 16 + k * 4 + 1, __uint_as_float(mine[k].y));
@@ -967,11 +970,10 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           return;
         }
         uint4 mine[4];
-        to_rows(chunk, mine);
+        to_rows(0, mine);
         auto add2 = [&](int c, uint32_t x) {
           float lo, hi;
-          if (bias_bf16) unpack_pair<true>(x, lo, hi);
-          else unpack_pair<false>(x, lo, hi);
+          unpack_pair<kBf16 == (kVariant == kBiasedSame)>(x, lo, hi);
           f2_unpack(ffma2(f2_pack(__uint_as_float(sc[c]), __uint_as_float(sc[c + 1])), scale2, fmul2(f2_pack(lo, hi), log2e2)), lo, hi);
           sc[c] = __float_as_uint(lo), sc[c + 1] = __float_as_uint(hi);
         };
@@ -1019,7 +1021,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           }
           const bool need_mask = (n0 + kBN > klen) || (causal && n0 + kBN - 1 > mt0 + shift + a.window_right) ||
                                  (a.window_left >= 0 && n0 < mt0 + tile_rows - 1 + shift - a.window_left);
-          uint4 bw[kBias ? 16 : 1];
+          uint4 bw[kBiasF32 ? 24 : kBias ? 16 : 1];
           bool whole = false;
           int rel_lo = 0, rel_hi = 0;  // visible keys of row r: from r + rel_lo, below r + rel_hi
           if constexpr (kBias) {
@@ -1028,7 +1030,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
             rel_lo = a.window_left >= 0 ? shift - a.window_left : -0x3fffffff;
             rel_hi = causal ? shift + a.window_right + 1 : 0x3fffffff;
             whole = a.bias_vec && !need_mask && mt0 + kBM <= it.qlen;
-            bias_load(bw, it.bias_off, mt0, it.qlen, n0, klen, rel_lo, rel_hi, whole);
+            bias_load(bw, std::integral_constant<int, kBiasF32 ? 6 : 4>{}, it.bias_off, mt0, it.qlen, n0, klen, rel_lo, rel_hi, whole);
             bias_prefetch(it.bias_off, mt0, it.qlen, n0 + kBN, j + 1 < jhi ? klen : 0);
           }
           if (!mbar_wait(&bar->s_full[t], cnt & 1, abort_flag, budget)) {
@@ -1069,15 +1071,27 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
           }
           {
             // ---- the row's 128 scores come into registers, and the buffer is free for the next QK^T
+            if constexpr (kBiasF32) {
+              uint32_t sc[32];
+#pragma unroll
+              for (int c = 0; c < kBN / 32; ++c) {
+                if (c > 0) tc_wait_st();  // (the store may still be reading the registers)
+                XFB_TMEM_LD_32(tmem_s + c * 32, sc);
+                XFB_TMEM_WAIT_LD_32(sc);
+                bias_add(sc, bw + c % 3 * 8);
+                XFB_TMEM_ST_32(tmem_s + c * 32, sc);
+                if (c == 0) bias_load(bw, std::integral_constant<int, 2>{}, it.bias_off, mt0, it.qlen, n0 + 96, klen, rel_lo, rel_hi, whole);
+              }
+              tc_wait_st();
+            }
             uint32_t s0[32], s1[32], s2[32], s3[32];
             XFB_TMEM_LD_32(tmem_s, s0);
             XFB_TMEM_LD_32(tmem_s + 32, s1);
-            if constexpr (kBias) {
+            if constexpr (kBias && !kBiasF32) {
               XFB_TMEM_WAIT_LD_32(s0);
               XFB_TMEM_WAIT_LD_32(s1);
-              bias_add(s0, bw, 0);
-              bias_add(s1, bw, 1);
-              if (bias_f32) bias_load(bw, it.bias_off, mt0, it.qlen, n0 + 64, klen, rel_lo, rel_hi, whole);
+              bias_add(s0, bw);
+              bias_add(s1, bw + 4);
             }
             XFB_TMEM_LD_32(tmem_s + 64, s2);
             XFB_TMEM_LD_32(tmem_s + 96, s3);
@@ -1088,9 +1102,9 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&bar->s_empty);
-            if constexpr (kBias) {
-              bias_add(s2, bw, 2);
-              bias_add(s3, bw, 3);
+            if constexpr (kBias && !kBiasF32) {
+              bias_add(s2, bw + 8);
+              bias_add(s3, bw + 12);
             }
             XFB_PROF_LAP(5)  // scores read
             float mx = fmaxf(chunk_max(reinterpret_cast<float*>(s0)), chunk_max(reinterpret_cast<float*>(s1)));
@@ -1177,7 +1191,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
 template <int D, bool kBf16, int kVariant>
 static int launch_t(Sm100Args a, cudaStream_t stream) {
   auto kern = prefill_sm100_persist_kernel<D, kBf16, kVariant>;
-  constexpr int smem = kVariant == kBiased || kVariant == kBiasedSame ? Smem<D>::kTotalBiased : Smem<D>::kTotal;
+  constexpr int smem = kVariant >= kBiasedSame ? Smem<D>::kTotalBiased : Smem<D>::kTotal;
   static_assert(smem <= 227 * 1024, "shared memory of one CTA");
   static bool configured[kMaxDevices] = {false};  // the attribute belongs to the device's context
   if (first_use_on_device(configured)) {
@@ -1218,9 +1232,11 @@ static int persist_launch_d(const Sm100Args& a, bool bf16, cudaStream_t stream) 
 }
 
 int prefill_sm100_persist_launch(Sm100Args a, int head_dim, bool bf16, cudaStream_t stream) {
-  if (a.bias != nullptr && a.bias_dtype == (bf16 ? XFB200_BF16 : XFB200_F16))
-    return head_dim > 64 ? persist_launch_d<128, pst::kBiasedSame>(a, bf16, stream) : persist_launch_d<64, pst::kBiasedSame>(a, bf16, stream);
-  if (a.bias != nullptr) return head_dim > 64 ? persist_launch_d<128, pst::kBiased>(a, bf16, stream) : persist_launch_d<64, pst::kBiased>(a, bf16, stream);
+  if (a.bias != nullptr && a.bias_dtype == XFB200_F32)
+    return head_dim > 64 ? persist_launch_d<128, pst::kBiasedF32>(a, bf16, stream) : persist_launch_d<64, pst::kBiasedF32>(a, bf16, stream);
+  if (a.bias != nullptr && a.bias_dtype == (bf16 ? XFB200_F16 : XFB200_BF16))
+    return head_dim > 64 ? persist_launch_d<128, pst::kBiasedOther>(a, bf16, stream) : persist_launch_d<64, pst::kBiasedOther>(a, bf16, stream);
+  if (a.bias != nullptr) return head_dim > 64 ? persist_launch_d<128, pst::kBiasedSame>(a, bf16, stream) : persist_launch_d<64, pst::kBiasedSame>(a, bf16, stream);
   if (head_dim > 128) return head_dim == 256 ? persist_launch_d<256, pst::kExact>(a, bf16, stream) : persist_launch_d<256, pst::kPadded>(a, bf16, stream);
   if (head_dim == 128) return persist_launch_d<128, pst::kExact>(a, bf16, stream);
   if (head_dim == 64) return persist_launch_d<64, pst::kExact>(a, bf16, stream);
