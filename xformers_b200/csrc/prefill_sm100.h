@@ -36,7 +36,7 @@ struct Sm100Args {
   int32_t n_items;    // persistent kernel: work items of the launch
   uint32_t epoch;   // differs from launch to launch, never 0
   int32_t debug_flags;
-  long long wait_budget;  // SM clocks after which a wait gives up
+  uint32_t wait_budget;  // after which a wait gives up, in wait_units()
   // additive bias (persistent kernel, dense batches): element strides of [batch, G, H, mq, mkv], unit stride on mkv;
   // the softmax sees (q k^T * scale + bias) * log2 e
   const void* bias;

@@ -3,10 +3,9 @@
 
 #include "internal.h"
 #include "prefill_sm100.h"
+#include "ptx.cuh"
 
 namespace xfb {
-
-constexpr long long kDefaultWaitBudgetCycles = 400000000LL;  // ~0.2 s of SM clock
 
 // Tensor map over [D, heads, rows, batch] (innermost first); box = 64 x box_heads x box_rows x 1, 128B swizzle.
 static int make_map(CUtensorMap* tm, const void* base, int dtype, int D, int64_t heads, int64_t head_stride, int64_t rows,
@@ -137,7 +136,7 @@ int prefill_sm100_launch(const xfb200_prefill_params* p, cudaStream_t stream) {
     if (D > 128 || int64_t(G) * H / pack * p->batch * tiles <= sm_count() - a.sm_margin) a.q_tiles = int32_t(tiles), a.item_rows = 128;
   }
   a.debug_flags = p->debug_flags;
-  a.wait_budget = p->wait_budget_kcycles > 0 ? 1000LL * p->wait_budget_kcycles : kDefaultWaitBudgetCycles;
+  a.wait_budget = wait_units(p->wait_budget_kcycles > 0 ? 1000LL * p->wait_budget_kcycles : kWaitBudgetCycles);
   a.bias = p->bias, a.bias_dtype = p->bias_dtype;
   a.bias_b = p->bias_stride_b, a.bias_g = p->bias_stride_g, a.bias_h = p->bias_stride_h, a.bias_m = p->bias_stride_m;
   {

@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_sm100_persist_kernel(cons
   const int n_items = a.n_items;
   const int pack_shift = kBias ? 0 : a.pack_shift;
   const int tile_rows = kBM >> pack_shift;  // query rows (tokens) of a tile
-  const long long budget = a.wait_budget;
+  const uint32_t budget = a.wait_budget;
   const int head_dim = kPad ? a.head_dim : D;
 
   // a CTA of this launch already gave up: take no work (the counters are still settled below)
