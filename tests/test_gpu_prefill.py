@@ -65,15 +65,31 @@ def test_dense_bmhk(op, dtype, D, causal, B, Mq, Mkv, H):
 @gpu
 @pytest.mark.parametrize("D", [8, 16, 32, 40, 72, 96, 120, 160, 256])
 @pytest.mark.parametrize("causal", [False, True])
-def test_other_head_dims_use_the_mma_kernel(D, causal):
+@pytest.mark.parametrize("op", [None, P.FwOp_Generic])
+def test_other_head_dims(op, D, causal):
+    """What the dispatch takes for them, and the mma.sync kernel."""
     require_cuda()
     dtype = torch.bfloat16
     q, k, v = rand_qkv(2, 68, 132, 1, 3, D, dtype, seed=D, gqa=False)
     q, k, v = q[:, :, 0], k[:, :, 0], v[:, :, 0]
     bias = ab.LowerTriangularMask() if causal else None
-    out, lse = fmha.memory_efficient_attention_forward_requires_grad(q, k, v, bias)
+    out, lse = fmha.memory_efficient_attention_forward_requires_grad(q, k, v, bias, op=op)
     ro, rl = ref(q, k, v, bias)
     assert_o_lse(out, lse, ro, rl, dtype, f"D={D}")
+
+
+@gpu
+@pytest.mark.parametrize("D", [160, 256])
+@pytest.mark.parametrize("M,Mkv,scale", [(1, 1, None), (50, 64, None), (64, 33, None), (200, 130, -0.05)])
+def test_calls_above_head_dim_128_that_stay_on_mma_sync(M, Mkv, scale, D):
+    """At most 64 rows and keys, or a scale that is not positive."""
+    require_cuda()
+    dtype = torch.float16
+    q, k, v = rand_qkv(2, M, Mkv, 1, 3, D, dtype, seed=D + M, gqa=False)
+    q, k, v = q[:, :, 0], k[:, :, 0], v[:, :, 0]
+    out, lse = fmha.memory_efficient_attention_forward_requires_grad(q, k, v, scale=scale)
+    ro, rl = ref(q, k, v, None, scale)
+    assert_o_lse(out, lse, ro, rl, dtype, f"D={D} {M} x {Mkv}")
 
 
 @gpu
@@ -592,13 +608,13 @@ def test_heads_of_a_group_share_a_tile(H, D, kind):
 
 
 @gpu
-@pytest.mark.parametrize("layout", ["dense", "causal", "bottom_right_gqa", "varlen"])
-@pytest.mark.parametrize("D", [136, 160, 184, 192, 200, 256])
-def test_head_dims_above_128(D, layout):
-    """One-tile items of the tcgen05 kernel: widths that are no multiple of 16 or 64, keys that end inside a step, more items than
-    SMs, queries without a key."""
+@pytest.mark.parametrize("layout", ["dense", "causal", "bottom_right_gqa", "varlen", "window"])
+@pytest.mark.parametrize("D,dtype,out_dtype", [(D, torch.bfloat16, None) for D in (136, 160, 184, 192, 200, 256)] +
+                         [(136, torch.float16, torch.float32), (200, torch.float16, None), (256, torch.float16, None), (256, torch.float16, torch.float32)])
+def test_head_dims_above_128(D, dtype, out_dtype, layout):
+    """One-tile items of the tcgen05 kernel (which of the calls it gets: test_route_above_head_dim_128): widths that are no multiple
+    of 16 or 64, keys that end inside a step, more items than SMs, queries without a key, windows."""
     require_cuda()
-    dtype = torch.bfloat16
     if layout == "varlen":
         lens = [1, 127, 300, 64, 129, 33]
         q, k, v = rand_qkv(1, sum(lens), sum(lens), 1, 3, D, dtype, seed=D, gqa=False)
@@ -607,11 +623,15 @@ def test_head_dims_above_128(D, layout):
     elif layout == "bottom_right_gqa":
         q, k, v = rand_qkv(1, 200, 131, 2, 4, D, dtype, seed=D)
         bias = ab.LowerTriangularFromBottomRightMask()
+    elif layout == "window":
+        q, k, v = rand_qkv(1, 300, 421, 2, 4, D, dtype, seed=D)
+        bias = ab.LocalAttentionFromBottomRightMask(window_left=150, window_right=20)
     else:
         q, k, v = rand_qkv(3, 333, 333, 1, 17, D, dtype, seed=D, gqa=False)
         q, k, v = q[:, :, 0], k[:, :, 0], v[:, :, 0]
         bias = ab.LowerTriangularMask() if layout == "causal" else None
-    out, lse = fmha.memory_efficient_attention_forward_requires_grad(q, k, v, bias)
+    out, lse = fmha.memory_efficient_attention_forward_requires_grad(q, k, v, bias, output_dtype=out_dtype)
+    assert out.dtype == (out_dtype or dtype)
     ro, rl = ref(q, k, v, bias)
     assert_o_lse(out, lse, ro, rl, dtype, f"D={D} {layout}")
     _status_ok()

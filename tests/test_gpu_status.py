@@ -72,6 +72,23 @@ def test_every_form_of_the_persistent_kernel_leaves_a_wait_that_runs_out(form):
 
 
 @gpu
+@pytest.mark.parametrize("D,M,Mkv,heads_per_sm,tcgen05", [
+    (160, 64, 64, 0.1, False), (256, 64, 64, 1, False), (256, 1, 1, 0.1, False), (160, 65, 64, 0.1, True), (256, 64, 65, 0.1, True),
+    (136, 64, 64, 1.01, True), (200, 300, 300, 0.1, True), (256, 333, 333, 0.1, True)])
+def test_route_above_head_dim_128(D, M, Mkv, heads_per_sm, tcgen05):
+    """Which kernel the automatic dispatch takes, seen by the testing aid that only the tcgen05 kernel has: dense calls of at most 64
+    rows and keys and no more heads than SMs stay on mma.sync."""
+    require_cuda()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    H = max(1, -int(-heads_per_sm * sms // 1))
+    q, k, v = rand_qkv(1, M, Mkv, 1, H, D, torch.float16, seed=M, gqa=False)
+    q, k, v = q[:, :, 0], k[:, :, 0], v[:, :, 0]
+    assert P.prefill_device_status() == 0
+    fmha.memory_efficient_attention_forward(q, k, v, op=_withheld(P.FwOp))
+    assert (P.prefill_device_status() != 0) == tcgen05
+
+
+@gpu
 def test_status_calls_through_the_c_abi():
     require_cuda()
     lib = _lib.load()
