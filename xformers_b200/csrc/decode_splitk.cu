@@ -715,8 +715,8 @@ __device__ __forceinline__ void quant_rows_finish(QuantRows<NTQ>& q, const DecWa
 //    overhead is paid once for 32 tokens.
 // 64 sequences of 1024 to 32768 keys, 8 kv heads, 64 query heads, pages of 256:
 // 388 -> 290 us (2.84 -> 3.80 TB/s; 280 with V's even elements left where they
-// are); 262 with Q read as registers want it.  314 instructions per sub-tile were 437; neither the issue slots (2.3 of 4)
-// nor the integer pipe (56 %) are full, so what is left is their dependent latency with
+// are); 262 with Q read as registers want it.  284 instructions per sub-tile were 437; neither the issue slots (2.4 of 4)
+// nor the integer pipe (60 %) are full, so what is left is their dependent latency with
 // four warps per scheduler.
 // ---------------------------------------------------------------------------
 template <int D, int NTQ, bool kBf16, int HB>

@@ -49,7 +49,7 @@
 // and long wait loops, the kernel had 110 KB of code, 21 % of the instruction requests missed (the former design: 10 %) and the
 // schedule above took 3900 clocks.  Hence: one copy of the code for both tiles, short loops,
 // elect.sync, a warp index known to be uniform, a wait loop of a few instructions, one place
-// per role that reports an error: 60 KB, 0.6 % misses.
+// per role that reports an error: 60 KB, 1.5 % misses.
 //
 // Softmax: thread = row.  If the maximum of a step exceeds the row's reference maximum by
 // more than 2^8 the row is re-based at once; otherwise the reference stays and nothing is rescaled -- one vote and
